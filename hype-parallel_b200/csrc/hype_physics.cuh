@@ -25,9 +25,11 @@ enum : int { BC_WALL = 0, BC_INLET = 1, BC_PERIODIC = 2, BC_REFLECTIVE = 3, BC_T
 // error bits reported through the device error word
 enum : unsigned { ERR_INADMISSIBLE_FACE = 1u, ERR_NONFINITE = 2u, ERR_TMA_TIMEOUT = 4u, ERR_BAD_LAUNCH = 8u };
 
-struct Eos {
+struct EosBase {
     double g1, g2, pi1, pi2;
     int fix_p2;   // Baer-Nunziato: 0 = flux pressure of phase 2 read from V[8] as baer_nunziato.c:271 does
+};
+struct Eos : EosBase {
     // constants the FP64 performance form (hype_physics_fast.cuh) reads instead of
     // dividing by them; filled by derive() at the start of each of its tiles
     double g1m1, g2m1, inv_g1m1, inv_g2m1, inv_g12, g1pi1, g2pi2, c1, c2;
@@ -143,8 +145,23 @@ template <int N, int Q> struct PhiVol { template <int K> static constexpr double
 template <int N, int Q> struct DPhiVolX { template <int K> static constexpr double at() { return Quad<N>::dphi_vol_x(Q, K); } };
 template <int N, int Q> struct DPhiVolY { template <int K> static constexpr double at() { return Quad<N>::dphi_vol_y(Q, K); } };
 
+// x in [2^LO, 2^HI), by its high word (one integer subtraction and comparison: the
+// FP64 pipe, which bounds the tiles, has no part in it); false for NaN and -x
+template <int LO, int HI>
+__device__ __forceinline__ bool exp_in(double x)
+{
+    return (unsigned)__double2hiint(x) - ((1023u + LO) << 20) < ((unsigned)(HI - LO) << 20);
+}
+// x in [0, 1)
+__device__ __forceinline__ bool frac_in(double x) { return (unsigned)__double2hiint(x) < 0x3ff00000u; }
+
 // ---------------------------------------------------------------------------
 // PDE systems (primitive-variable path)
+//
+// pad_quick<c>(v): value v of variable c lies in a range where, for constants that
+// quick_eos accepts, pad() is true whatever the other variables are within theirs.
+// Almost every cell is accepted by it, without the sound speeds' divisions; the rest
+// takes pad() itself.
 // ---------------------------------------------------------------------------
 template <int SYS> struct System;
 
@@ -156,7 +173,7 @@ template <> struct System<SYS_KAPILA> {
     // kapila_5eqn.c:14-35; dv(a, b) = a / b (cons2prim_dv: the bit-exact tile's row staging
     // passes the branch-free correctly rounded division, so the independent divisions overlap)
     template <class Dv>
-    __device__ __forceinline__ static void cons2prim_dv(const Eos &e, const double *Q, double *V, Dv dv)
+    __device__ __forceinline__ static void cons2prim_dv(const EosBase &e, const double *Q, double *V, Dv dv)
     {
         double alpha_1 = Q[5];
         double alpha_2 = 1.0 - alpha_1;
@@ -175,12 +192,12 @@ template <> struct System<SYS_KAPILA> {
         V[4] = p;
         V[5] = alpha_1;
     }
-    __device__ __forceinline__ static void cons2prim(const Eos &e, const double *Q, double *V)
+    __device__ __forceinline__ static void cons2prim(const EosBase &e, const double *Q, double *V)
     {
         cons2prim_dv(e, Q, V, [](double a, double b) { return a / b; });
     }
     // kapila_5eqn.c:41-61
-    __device__ __forceinline__ static void prim2cons(const Eos &e, const double *V, double *Q)
+    __device__ __forceinline__ static void prim2cons(const EosBase &e, const double *V, double *Q)
     {
         double alpha_1 = V[5];
         double alpha_2 = 1.0 - alpha_1;
@@ -199,7 +216,7 @@ template <> struct System<SYS_KAPILA> {
     }
     // kapila_5eqn.c:326-371
     template <int DIR>
-    __device__ __forceinline__ static double flux(const Eos &e, const double *V, double *F, bool &bad)
+    __device__ __forceinline__ static double flux(const EosBase &e, const double *V, double *F, bool &bad)
     {
         constexpr double nx = DIR == 0 ? 1.0 : 0.0, ny = DIR == 0 ? 0.0 : 1.0;
         double alpha_1 = V[5];
@@ -225,7 +242,7 @@ template <> struct System<SYS_KAPILA> {
         return fabs(un) + sqrt(a_sq);
     }
     // kapila_5eqn.c:417-444
-    __device__ __forceinline__ static void ncp(const Eos &e, const double *V, const double *gx, const double *gy, double *B)
+    __device__ __forceinline__ static void ncp(const EosBase &e, const double *V, const double *gx, const double *gy, double *B)
     {
         double alpha_1 = V[5];
         double alpha_2 = 1.0 - alpha_1;
@@ -239,8 +256,26 @@ template <> struct System<SYS_KAPILA> {
         B[5] = u * phi_x + v * phi_y - K * (u_x + v_y);
     }
     static constexpr bool ncp_nonzero(int c) { return c == 5; }
+    static constexpr int order(int k) { constexpr int o[6] = {5, 2, 3, 4, 0, 1}; return o[k]; }
+    // With rho_k in [2^-30, 2^16), p in [2^-20, 2^100), alpha_1 in [0, 1), 1 <= gamma <= 2^10 and
+    // 0 <= pi <= 2^100: rho >= 2^-32 > RHO_FLOOR; rho_k a_k^2 = gamma_k (p + pi_k) >= 2^-20 and the
+    // mixture's rho a^2 is at least the smaller of the two, so a^2 >= 2^-20 / 2^16 > PRS_FLOOR with
+    // room for rounding; no product of pad() leaves [2^-400, 2^400]
+    __device__ __forceinline__ static bool quick_eos(const EosBase &e)
+    {
+        return e.g1 >= 1.0 && e.g1 <= 1024.0 && e.g2 >= 1.0 && e.g2 <= 1024.0 && e.pi1 >= 0.0 && e.pi1 <= 0x1p100 &&
+               e.pi2 >= 0.0 && e.pi2 <= 0x1p100;
+    }
+    template <int C>
+    __device__ __forceinline__ static bool pad_quick(double v)
+    {
+        if constexpr (C <= 1) return exp_in<-30, 16>(v);
+        else if constexpr (C == 4) return exp_in<-20, 100>(v);
+        else if constexpr (C == 5) return frac_in(v);
+        else return true;
+    }
     // kapila_5eqn.c:450-479
-    __device__ __forceinline__ static bool pad(const Eos &e, const double *V)
+    __device__ __forceinline__ static bool pad(const EosBase &e, const double *V)
     {
         double alpha_1 = V[5];
         double alpha_2 = 1.0 - alpha_1;
@@ -314,7 +349,7 @@ template <> struct System<SYS_KAPILA> {
     // ---- conservative-variable path (RHSFunction, rhs_function.c) ----
     // kapila_5eqn.c:67-113
     template <int DIR>
-    __device__ __forceinline__ static double flux_cons(const Eos &e, const double *Q, double *F, bool &bad)
+    __device__ __forceinline__ static double flux_cons(const EosBase &e, const double *Q, double *F, bool &bad)
     {
         constexpr double nx = DIR == 0 ? 1.0 : 0.0, ny = DIR == 0 ? 0.0 : 1.0;
         double alpha_1 = Q[5];
@@ -343,7 +378,7 @@ template <> struct System<SYS_KAPILA> {
         return fabs(un) + sqrt(a_sq);
     }
     // kapila_5eqn.c:164-198
-    __device__ __forceinline__ static void ncp_cons(const Eos &e, const double *Q, const double *gx, const double *gy, double *B)
+    __device__ __forceinline__ static void ncp_cons(const EosBase &e, const double *Q, const double *gx, const double *gy, double *B)
     {
         double alpha_1 = Q[5];
         double alpha_2 = 1.0 - alpha_1;
@@ -369,9 +404,10 @@ template <> struct System<SYS_KAPILA> {
     }
     static constexpr bool ncp_cons_nonzero(int c) { return c == 5; }
     // kapila_5eqn.c:247-283; its alpha test (line 278) rejects every alpha_1 != 1
-    __device__ __forceinline__ static bool pad_cons(const Eos &e, const double *Q)
+    __device__ __forceinline__ static bool pad_cons(const EosBase &e, const double *Q)
     {
         double alpha_1 = Q[5];
+        if (alpha_1 < 1.0 || alpha_1 > 1.0) return false;   // every test rejects: the cheap one first
         double alpha_2 = 1.0 - alpha_1;
         double rho_1 = Q[0] / alpha_1;
         double rho_2 = Q[1] / alpha_2;
@@ -388,7 +424,6 @@ template <> struct System<SYS_KAPILA> {
         double a_sq = (rho_1 * a1_sq * rho_2 * a2_sq) / (rho * (alpha_2 * rho_1 * a1_sq + alpha_1 * rho_2 * a2_sq));
         if (rho < RHO_FLOOR) return false;
         if (a_sq < PRS_FLOOR) return false;
-        if (alpha_1 < 1.0 || alpha_1 > 1.0) return false;
         return true;
     }
 };
@@ -399,12 +434,12 @@ template <> struct System<SYS_BN> {
     static constexpr int NV = 9;
     static constexpr int RX0 = 1, RX1 = 5, RY0 = 2, RY1 = 6;   // rhs_function_prim.c:115-117, 244-246
     // baer_nunziato.c:14-41; dv(a, b) = a / b (cons2prim_dv as for the Kapila system)
-    __device__ __forceinline__ static void cons2prim(const Eos &e, const double *Q, double *V)
+    __device__ __forceinline__ static void cons2prim(const EosBase &e, const double *Q, double *V)
     {
         cons2prim_dv(e, Q, V, [](double a, double b) { return a / b; });
     }
     template <class Dv>
-    __device__ __forceinline__ static void cons2prim_dv(const Eos &e, const double *Q, double *V, Dv dv)
+    __device__ __forceinline__ static void cons2prim_dv(const EosBase &e, const double *Q, double *V, Dv dv)
     {
         double phi_1 = Q[8];
         double phi_2 = 1.0 - Q[8];
@@ -421,7 +456,7 @@ template <> struct System<SYS_BN> {
         V[8] = phi_1;
     }
     // baer_nunziato.c:47-60
-    __device__ __forceinline__ static void prim2cons(const Eos &e, const double *V, double *Q)
+    __device__ __forceinline__ static void prim2cons(const EosBase &e, const double *V, double *Q)
     {
         Q[0] = V[8] * V[0];
         Q[1] = Q[0] * V[1];
@@ -435,7 +470,7 @@ template <> struct System<SYS_BN> {
     }
     // baer_nunziato.c:256-321 (phase-2 flux pressure from V[8] unless fix_p2)
     template <int DIR>
-    __device__ __forceinline__ static double flux(const Eos &e, const double *V, double *F, bool &bad)
+    __device__ __forceinline__ static double flux(const EosBase &e, const double *V, double *F, bool &bad)
     {
         constexpr double nx = DIR == 0 ? 1.0 : 0.0, ny = DIR == 0 ? 0.0 : 1.0;
         double phi_1 = V[8];
@@ -464,7 +499,7 @@ template <> struct System<SYS_BN> {
         return (s_1 < s_2) ? s_2 : s_1;
     }
     // baer_nunziato.c:327-344
-    __device__ __forceinline__ static void ncp(const Eos &, const double *V, const double *gx, const double *gy, double *B)
+    __device__ __forceinline__ static void ncp(const EosBase &, const double *V, const double *gx, const double *gy, double *B)
     {
         double u_I = V[1], v_I = V[2];
         double p_I = V[7];
@@ -480,8 +515,19 @@ template <> struct System<SYS_BN> {
         B[8] = u_I * phi_x + v_I * phi_y;
     }
     static constexpr bool ncp_nonzero(int c) { return c != 0 && c != 4; }
+    static constexpr int order(int k) { constexpr int o[9] = {8, 1, 2, 7, 0, 3, 4, 5, 6}; return o[k]; }
+    // rho_k >= 2^-30 > RHO_FLOOR, p_k >= 2^-20 and pi_k >= 0: p_k + pi_k > PRS_FLOOR, alpha_1 in [0, 1)
+    __device__ __forceinline__ static bool quick_eos(const EosBase &e) { return e.pi1 >= 0.0 && e.pi2 >= 0.0; }
+    template <int C>
+    __device__ __forceinline__ static bool pad_quick(double v)
+    {
+        if constexpr (C == 0 || C == 4) return exp_in<-30, 1000>(v);
+        else if constexpr (C == 3 || C == 7) return exp_in<-20, 1000>(v);
+        else if constexpr (C == 8) return frac_in(v);
+        else return true;
+    }
     // baer_nunziato.c:350-385
-    __device__ __forceinline__ static bool pad(const Eos &e, const double *V)
+    __device__ __forceinline__ static bool pad(const EosBase &e, const double *V)
     {
         bool ok = true;
         if (V[0] < RHO_FLOOR) ok = false;
@@ -495,7 +541,7 @@ template <> struct System<SYS_BN> {
     // ---- conservative-variable path (RHSFunction, rhs_function.c) ----
     // baer_nunziato.c:66-131
     template <int DIR>
-    __device__ __forceinline__ static double flux_cons(const Eos &e, const double *Q, double *F, bool &bad)
+    __device__ __forceinline__ static double flux_cons(const EosBase &e, const double *Q, double *F, bool &bad)
     {
         constexpr double nx = DIR == 0 ? 1.0 : 0.0, ny = DIR == 0 ? 0.0 : 1.0;
         double phi_1 = Q[8];
@@ -525,7 +571,7 @@ template <> struct System<SYS_BN> {
         return (s_1 < s_2) ? s_2 : s_1;
     }
     // baer_nunziato.c:137-165: u_I = u_1, p_I = p_2 from the phase-2 state
-    __device__ __forceinline__ static void ncp_cons(const Eos &e, const double *Q, const double *gx, const double *gy, double *B)
+    __device__ __forceinline__ static void ncp_cons(const EosBase &e, const double *Q, const double *gx, const double *gy, double *B)
     {
         double phi_2 = 1.0 - Q[8];
         double rho_2 = Q[4] / phi_2;
@@ -546,7 +592,7 @@ template <> struct System<SYS_BN> {
     }
     static constexpr bool ncp_cons_nonzero(int c) { return c != 0 && c != 4; }
     // baer_nunziato.c:207-250
-    __device__ __forceinline__ static bool pad_cons(const Eos &e, const double *Q)
+    __device__ __forceinline__ static bool pad_cons(const EosBase &e, const double *Q)
     {
         bool ok = true;
         double phi_1 = Q[8];
@@ -573,7 +619,7 @@ template <> struct System<SYS_EULER> {
     static constexpr int NV = 4;
     static constexpr int RX0 = 1, RX1 = -1, RY0 = 2, RY1 = -1;   // rhs_function_prim.c:101-102, 230-231
     // euler.c:14-23
-    __device__ __forceinline__ static void cons2prim(const Eos &e, const double *Q, double *V)
+    __device__ __forceinline__ static void cons2prim(const EosBase &e, const double *Q, double *V)
     {
         double irho = 1.0 / Q[0];
         V[0] = Q[0];
@@ -582,7 +628,7 @@ template <> struct System<SYS_EULER> {
         V[3] = (e.g1 - 1.0) * (Q[3] - 0.5 * irho * (Q[1] * Q[1] + Q[2] * Q[2]));
     }
     // euler.c:29-38
-    __device__ __forceinline__ static void prim2cons(const Eos &e, const double *V, double *Q)
+    __device__ __forceinline__ static void prim2cons(const EosBase &e, const double *V, double *Q)
     {
         double ei = (V[3]) / (e.g1 - 1.0);
         double k = 0.5 * V[0] * (V[1] * V[1] + V[2] * V[2]);
@@ -593,7 +639,7 @@ template <> struct System<SYS_EULER> {
     }
     // euler.c:197-236
     template <int DIR>
-    __device__ __forceinline__ static double flux(const Eos &e, const double *V, double *F, bool &bad)
+    __device__ __forceinline__ static double flux(const EosBase &e, const double *V, double *F, bool &bad)
     {
         constexpr double nx = DIR == 0 ? 1.0 : 0.0, ny = DIR == 0 ? 0.0 : 1.0;
         double rho = V[0], u = V[1], v = V[2];
@@ -609,13 +655,22 @@ template <> struct System<SYS_EULER> {
         return fabs(un) + sqrt(e.g1 * p / rho);
     }
     // euler.c:278-286
-    __device__ __forceinline__ static void ncp(const Eos &, const double *, const double *, const double *, double *B)
+    __device__ __forceinline__ static void ncp(const EosBase &, const double *, const double *, const double *, double *B)
     {
         B[0] = 0.0; B[1] = 0.0; B[2] = 0.0; B[3] = 0.0;
     }
     static constexpr bool ncp_nonzero(int) { return false; }
+    static constexpr int order(int k) { constexpr int o[4] = {0, 1, 2, 3}; return o[k]; }
+    // rho >= 2^-30 > RHO_FLOOR, p >= 2^-30 > PRS_FLOOR
+    __device__ __forceinline__ static bool quick_eos(const EosBase &) { return true; }
+    template <int C>
+    __device__ __forceinline__ static bool pad_quick(double v)
+    {
+        if constexpr (C == 0 || C == 3) return exp_in<-30, 1000>(v);
+        else return true;
+    }
     // euler.c:292-310
-    __device__ __forceinline__ static bool pad(const Eos &, const double *V)
+    __device__ __forceinline__ static bool pad(const EosBase &, const double *V)
     {
         bool ok = true;
         if (V[0] < RHO_FLOOR) ok = false;
@@ -626,7 +681,7 @@ template <> struct System<SYS_EULER> {
     // ---- conservative-variable path (RHSFunction, rhs_function.c) ----
     // euler.c:44-84
     template <int DIR>
-    __device__ __forceinline__ static double flux_cons(const Eos &e, const double *Q, double *F, bool &bad)
+    __device__ __forceinline__ static double flux_cons(const EosBase &e, const double *Q, double *F, bool &bad)
     {
         constexpr double nx = DIR == 0 ? 1.0 : 0.0, ny = DIR == 0 ? 0.0 : 1.0;
         double rho = Q[0];
@@ -644,13 +699,13 @@ template <> struct System<SYS_EULER> {
         F[3] = un * (E + p);
         return fabs(un) + sqrt(e.g1 * p * irho);
     }
-    __device__ __forceinline__ static void ncp_cons(const Eos &, const double *, const double *, const double *, double *B)
+    __device__ __forceinline__ static void ncp_cons(const EosBase &, const double *, const double *, const double *, double *B)
     {
         B[0] = 0.0; B[1] = 0.0; B[2] = 0.0; B[3] = 0.0;
     }
     static constexpr bool ncp_cons_nonzero(int) { return false; }
     // euler.c:169-191
-    __device__ __forceinline__ static bool pad_cons(const Eos &e, const double *Q)
+    __device__ __forceinline__ static bool pad_cons(const EosBase &e, const double *Q)
     {
         bool ok = true;
         double rho = Q[0];

@@ -17,8 +17,7 @@ __global__ void __launch_bounds__(2 * CELLS, (StageKernel<SYS, N, CELLS>::MIN_BL
 stage_kernel(const __grid_constant__ CUtensorMap tmap, const StageParams p)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ double red_s[2 * CELLS / 32];
-    stage_tile<SYS, N, CELLS, false>(p, &tmap, blockIdx.x, p.run0 + (int)blockIdx.y, smem_raw, red_s);
+    stage_tile<SYS, N, CELLS, false>(p, &tmap, blockIdx.x, p.run0 + (int)blockIdx.y, smem_raw);
 }
 
 // Persistent form: the block walks a list of (grid, tile) work items; every grid
@@ -29,11 +28,10 @@ stage_batch_kernel(const StageParams *__restrict__ inst, const CUtensorMap *__re
                    const int2 *__restrict__ work, int *__restrict__ sched)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ double red_s[2 * CELLS / 32];
     __shared__ int item_s;
     // the item's parameters live in shared memory: re-read after every barrier
     // of the tile instead of pinning registers for the whole tile
-    __shared__ StageParams p_s;
+    __shared__ BatchParams p_s;
     const int nwork = sched[0];
     const DevScalars *last = nullptr;
     for (;;) {
@@ -41,13 +39,12 @@ stage_batch_kernel(const StageParams *__restrict__ inst, const CUtensorMap *__re
         if (w >= nwork) break;
         const int2 it = work[w];
         if (threadIdx.x == 0) {
-            p_s = inst[it.x];
-            p_s.runs *= item_refine(it.y);
+            p_s.load(inst[it.x], item_refine(it.y));
             fence_tensormap_acquire(&tmaps[it.x]);
         }
         __syncthreads();
         const int tile = item_tile(it.y);
-        stage_tile<SYS, N, CELLS, false>(p_s, &tmaps[it.x], tile % p_s.strips, tile / p_s.strips, smem_raw, red_s);
+        stage_tile<SYS, N, CELLS, false>(p_s, &tmaps[it.x], tile % p_s.strips, tile / p_s.strips, smem_raw);
         last = p_s.sc;
     }
     work_finish(sched);

@@ -29,9 +29,8 @@ path_batch_kernel(const StageParams *__restrict__ inst, const CUtensorMap *__res
                   int *__restrict__ sched)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ double red_s[2 * STAGE_CELLS / 32];
     __shared__ int item_s;
-    __shared__ StageParams p_s;   // the item's parameters, re-read after every barrier of the tile
+    __shared__ BatchParams p_s;   // the item's parameters, re-read after every barrier of the tile
     const int nwork = sched[0];
     const DevScalars *last = nullptr;
     for (;;) {
@@ -39,13 +38,12 @@ path_batch_kernel(const StageParams *__restrict__ inst, const CUtensorMap *__res
         if (w >= nwork) break;
         const int2 it = work[w];
         if (threadIdx.x == 0) {
-            p_s = inst[it.x];
-            p_s.runs *= item_refine(it.y);
+            p_s.load(inst[it.x], item_refine(it.y));
             fence_tensormap_acquire(&tmaps[it.x]);
         }
         __syncthreads();
         const int tile = item_tile(it.y);
-        stage_tile<SYS, N, STAGE_CELLS, CONS, VISC>(p_s, &tmaps[it.x], tile % p_s.strips, tile / p_s.strips, smem_raw, red_s);
+        stage_tile<SYS, N, STAGE_CELLS, CONS, VISC>(p_s, &tmaps[it.x], tile % p_s.strips, tile / p_s.strips, smem_raw);
         last = p_s.sc;
     }
     work_finish(sched);

@@ -24,6 +24,26 @@
 // below.  Row r-1 is completed (y-flux difference, volume non-conservative
 // term, RK combination) while row r is processed.
 //
+// One pass over a cell's coefficients gives every point value the row needs:
+// the values at the four faces' Gauss point q = h, which are also the nodes of
+// the admissibility check, and at the half's volume Gauss points.  The points
+// differ by signs only, so the pass forms each product coefficient x |basis
+// value| once and adds or subtracts it (a product changes only its sign with
+// its factor's: same bits).  The left and right values then replace the
+// coefficients in shared memory, the top values stay for the row above, the
+// bottom and volume values in registers.
+//
+// What bounds the tile is FP64 issue: dependent FP64 chains at 8 or 16 warps per SM.
+// With the point values in one pass, the admissibility divisions left to the few cells
+// that need them and no sums or shuffles of products that are zero, the Kapila N = 2
+// tile executes 9.54e8 warp instructions per 2048^2 right-hand side instead of 1.21e9
+// (3.8 k FP64 instructions a cell instead of 5.0 k) and the call takes 1.76 ms instead of
+// 2.09; Euler 1531x897 0.380 ms instead of 0.417, BN 1024^2 0.896 instead of 0.947.
+//
+// Two block barriers a row: after the first, the neighbours' face values are
+// there, and row r+3 (loaded in the previous iteration) is converted beside
+// the x-face problems; the second makes the x fluxes and that row visible.
+//
 // Compiled with --fmad=false: arithmetic rounds exactly as the reference's C does.
 #pragma once
 #include <cuda.h>
@@ -33,6 +53,35 @@
 #include "hype_tma.cuh"
 
 namespace hype {
+
+// The stage parameters a persistent kernel's tile reads, copied to shared memory for each
+// work item.  What a batch instance never has (slab and block offsets, interleaved output,
+// a run range, the test hook) is a constant: the tile drops its code, and the struct leaves
+// room for two blocks per SM.
+struct BatchParams {
+    int nx, ny, pitch, strips, runs, mode, reduce_smax;
+    int bc[4];
+    long long plane;
+    EosBase eos;
+    double r1_h, ka, kb, kc, mu1, mu2;
+    const double *in, *xn, *inlet;
+    double *out, *out2;
+    DevScalars *sc;
+    static constexpr int out_aos = 0, row_off = 0, col_off = 0, skip_loads = 0, skip_loads_from = 0;
+    static constexpr int push_shift_lo = 0, push_shift_hi = 0;
+    static constexpr long long push_plane_lo = 0, push_plane_hi = 0;
+    static constexpr double *push_lo = nullptr, *push_hi = nullptr;
+    __device__ __forceinline__ void load(const StageParams &p, int refine)
+    {
+        nx = p.nx; ny = p.ny; pitch = p.pitch; strips = p.strips; runs = p.runs * refine;
+        mode = p.mode; reduce_smax = p.reduce_smax;
+        for (int k = 0; k < 4; ++k) bc[k] = p.bc[k];
+        plane = p.plane;
+        eos = p.eos;
+        r1_h = p.r1_h; ka = p.ka; kb = p.kb; kc = p.kc; mu1 = p.mu1; mu2 = p.mu2;
+        in = p.in; xn = p.xn; inlet = p.inlet; out = p.out; out2 = p.out2; sc = p.sc;
+    }
+};
 
 template <int SYS, int N, int CELLS_>
 struct StageKernel {
@@ -48,14 +97,27 @@ struct StageKernel {
     static constexpr int ROW_ELEMS = BW * NV;
     static constexpr int ROW_BYTES = ROW_ELEMS * 8;
     static constexpr int SLOT_STRIDE = ((ROW_BYTES + 127) / 128) * 128 / 8;   // doubles
-    // per-cell arrays, [k][c][cell] so consecutive cells hit consecutive banks
-    static constexpr int COEF_ELEMS = (NC > 2 ? NC : 2) * NV * CELLS;         // also the x-flux exchange (2 NV)
-    static constexpr int YT_ELEMS = 2 * NV * CELLS;                            // top-face values, by Gauss point
-    static constexpr int CARRY_ELEMS = 4 * NV * CELLS;                         // ncp, t1, G below, E below
+    // components with a non-conservative product (the same ones on the conservative path)
+    static constexpr int nz(int c)   // its index among them, -1 where there is none
+    {
+        if (!S::ncp_nonzero(c)) return -1;
+        int z = 0;
+        for (int k = 0; k < c; ++k) z += S::ncp_nonzero(k) ? 1 : 0;
+        return z;
+    }
+    static constexpr int count_nz() { int z = 0; for (int c = 0; c < S::NV; ++c) z += S::ncp_nonzero(c) ? 1 : 0; return z; }
+    static constexpr int NZ = count_nz();
+    // per-cell arrays, [k][c][cell] so consecutive cells hit consecutive banks.  Coefficients
+    // k >= 1; later, by slot, the left and right face values at each Gauss point (2 q, 2 q + 1)
+    // and the x-face fluxes (slot 0) and fluctuations (slot 2)
+    static constexpr int COEF_ELEMS = (NC > 3 ? NC : 3) * NV * CELLS;
+    static constexpr int YT_ELEMS = 2 * QD::NFGP * NV * CELLS;                 // top-face values of rows r-1 and r, by Gauss point
+    static constexpr int CARRY_ELEMS = (2 * NV + 2 * NZ) * CELLS;              // t1, G below; ncp, E below
     // the ring, the per-cell arrays and one more row slot: the conserved input of the row
     // being finished (row r-1), for the RK combination
-    static constexpr size_t SMEM = 128 /* barriers */ + (size_t)(SLOTS + 1) * SLOT_STRIDE * 8 +
-                                   (size_t)(COEF_ELEMS + YT_ELEMS + CARRY_ELEMS) * 8 + 64;
+    static constexpr size_t SMEM = (size_t)(SLOTS + 1) * SLOT_STRIDE * 8 + (size_t)(COEF_ELEMS + YT_ELEMS + CARRY_ELEMS) * 8 +
+                                   64 /* barriers */;
+    static_assert((SLOTS + 1) * 8 <= 64, "the barriers fit their space");
     // blocks the 228 KB of an SM's shared memory holds (1 KB reserved per block); the
     // launch bound asks for no more than that, so no register limit is paid for blocks
     // that could not be resident anyway (Kapila N = 3 at 128-column tiles: 1)
@@ -65,30 +127,81 @@ struct StageKernel {
     static constexpr size_t smem_bytes() { return SMEM; }
 };
 
-// Value of one variable's polynomial cf[0..NDOF) at Gauss point q (0/1, run
-// time) of face F.  Where both Gauss points share a basis value it is folded
-// at compile time (zero terms dropped, exact as in poly_eval); otherwise the
-// product with the selected value is formed exactly as the reference does.
-template <int N, int F>
-__device__ __forceinline__ double face_val(const double *cf, int q)
+__device__ __forceinline__ int hi_word(double x) { return __double2hiint(x); }
+// x with its sign flipped where mask = 0x80000000 (0: unchanged)
+__device__ __forceinline__ double flip_sign(double x, unsigned mask)
 {
-    using QD = Quad<N>;
-    double v = 0.0;
-    static_for<QD::NDOF>([&](auto kk) {
-        constexpr int k = decltype(kk)::value;
-        constexpr double p0 = QD::phi_face(F, 0, k);
-        constexpr double p1 = QD::phi_face(F, QD::NFGP > 1 ? 1 : 0, k);
-        if constexpr (p0 == p1) {
-            if constexpr (p0 != 0.0) {
-                if constexpr (p0 == 1.0) v = v + cf[k];
-                else v = v + cf[k] * p0;
-            }
-        } else {
-            const double p = q ? p1 : p0;
-            v = v + cf[k] * p;
-        }
-    });
+    return __hiloint2double((int)((unsigned)__double2hiint(x) ^ mask), __double2loint(x));
+}
+
+// v + ck * p, where p is P0 for half 0 of the pair and P1 for half 1 and |P0| = |P1|.
+// `mask` flips half 0's sign.  The product is formed with |p| and added or subtracted,
+// so that points whose basis values differ in sign share it; FAST fuses each term instead.
+template <bool FAST, class P>
+__device__ __forceinline__ double add_term(double v, double ck, unsigned mask)
+{
+    constexpr double p0 = P::p0(), p1 = P::p1(), a = p1 < 0.0 ? -p1 : p1;
+    static_assert(p0 == p1 || p0 == -p1, "the halves' points mirror each other");
+    if constexpr (a == 0.0) {
+        return v;   // the reference adds ck * 0 to a sum that is never -0
+    } else if constexpr (p0 == p1) {
+        const double t = a == 1.0 ? ck : ck * a;
+        return p1 > 0.0 ? v + t : v - t;
+    } else if constexpr (FAST) {
+        const double cs = flip_sign(ck, mask);
+        return p1 > 0.0 ? v + cs * a : v - cs * a;
+    } else {
+        const double t = flip_sign(ck * a, mask);
+        return p1 > 0.0 ? v + t : v - t;
+    }
+}
+// the basis values of coefficient K at the points of halves 0 and 1: face F's Gauss point
+// q = half; the half's volume Gauss point A, values and derivatives
+template <int N, int F, int K> struct FacePt {
+    static constexpr double p0() { return Quad<N>::phi_face(F, 0, K); }
+    static constexpr double p1() { return Quad<N>::phi_face(F, Quad<N>::NFGP > 1 ? 1 : 0, K); }
+};
+template <int N, int A, int K> struct VolPt {
+    static constexpr int q1 = Quad<N>::NVGP > 1 ? Quad<N>::NVGP / 2 + A : A;
+    static constexpr double p0() { return Quad<N>::phi_vol(A, K); }
+    static constexpr double p1() { return Quad<N>::phi_vol(q1, K); }
+};
+template <int N, int A, int D, int K> struct VolGrad {
+    static constexpr int q1 = VolPt<N, A, K>::q1;
+    static constexpr double p0() { return D == 0 ? Quad<N>::dphi_vol_x(A, K) : Quad<N>::dphi_vol_y(A, K); }
+    static constexpr double p1() { return D == 0 ? Quad<N>::dphi_vol_x(q1, K) : Quad<N>::dphi_vol_y(q1, K); }
+};
+// One variable's polynomial at face F's Gauss point of the half, terms in ascending k as the
+// reference's loops.  The reference starts from 0.0: 0.0 + c0 differs from c0 for c0 = -0 only,
+// and a zero's sign reaches no result (every flux and product sum starts from +0).
+template <int N, int F, bool FAST>
+__device__ __forceinline__ double face_pt(const double *cf, unsigned mask)
+{
+    double v = cf[0];
+    static_for<Quad<N>::NDOF - 1>([&](auto kk) { constexpr int k = decltype(kk)::value + 1; v = add_term<FAST, FacePt<N, F, k>>(v, cf[k], mask); });
     return v;
+}
+template <int N, int A, bool FAST>
+__device__ __forceinline__ double vol_pt(const double *cf, unsigned mask)
+{
+    double v = cf[0];
+    static_for<Quad<N>::NDOF - 1>([&](auto kk) { constexpr int k = decltype(kk)::value + 1; v = add_term<FAST, VolPt<N, A, k>>(v, cf[k], mask); });
+    return v;
+}
+template <int N, int A, int D, bool FAST>
+__device__ __forceinline__ double vol_grad(const double *cf, unsigned mask)
+{
+    if constexpr (N == 0) {
+        return 0.0;
+    } else {
+        constexpr int first = 1 + D;   // the linear coefficient along D, basis derivative 1
+        double v = cf[first];
+        static_for<Quad<N>::NDOF - 1 - first>([&](auto kk) {
+            constexpr int k = decltype(kk)::value + 1 + first;
+            v = add_term<FAST, VolGrad<N, A, D, k>>(v, cf[k], mask);
+        });
+        return v;
+    }
 }
 
 // Gradient component D (0: x, 1: y) of one variable at Gauss point q of face
@@ -121,8 +234,8 @@ __device__ __forceinline__ double face_grad(const double *uc, int q)
 // (RiemannSolverPrim, VL/VR primitive) or, for the conservative path,
 // riemann.c:52-105 (RiemannSolver, VL/VR conserved); S is the system's physics
 // (System<SYS>, or FastSystem<SYS> for the FP64 performance form)
-template <class S, int DIR, bool CONS>
-__device__ __forceinline__ double riemann_gp(const Eos &eos, const double *VL, const double *VR, double *F, double *D, bool &bad)
+template <class S, int DIR, bool CONS, class E>
+__device__ __forceinline__ double riemann_gp(const E &eos, const double *VL, const double *VR, double *F, double *D, bool &bad)
 {
     constexpr int NV = S::NV;
     constexpr double nx = DIR == 0 ? 1.0 : 0.0, ny = DIR == 0 ? 0.0 : 1.0;
@@ -173,37 +286,39 @@ __device__ __forceinline__ double riemann_gp(const Eos &eos, const double *VL, c
 // FAST: the FP64 performance form (primitive path only): FastSystem / ReconFast
 // of hype_physics_fast.cuh, in a translation unit built with FMA contraction;
 // reads the derived constants of p.eos (Eos::derive, filled by the host).
-template <int SYS, int N, int CELLS_, bool CONS, bool VISC = false, bool FAST = false>
-__device__ __forceinline__ void stage_tile(const StageParams &p, const CUtensorMap *tmap, int strip, int run,
-                                           unsigned char *smem_raw, double *red_s)
+template <int SYS, int N, int CELLS_, bool CONS, bool VISC = false, bool FAST = false, class P>
+__device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, int strip, int run, unsigned char *smem_raw)
 {
     static_assert(!(FAST && (CONS || VISC)), "the FP64 performance form covers the primitive inviscid path");
     using K = StageKernel<SYS, N, CELLS_>;
     using S = std::conditional_t<FAST, FastSystem<SYS>, typename K::S>;
     using QD = typename K::QD;
-    constexpr int NV = K::NV, CELLS = K::CELLS, BW = K::BW, SLOTS = K::SLOTS, NDOF = K::NDOF;
-    constexpr int NFGP = QD::NFGP, NVGP = QD::NVGP, NNODE = QD::NNODE;
+    constexpr int NV = K::NV, CELLS = K::CELLS, BW = K::BW, SLOTS = K::SLOTS, NDOF = K::NDOF, NZ = K::NZ;
+    constexpr int NFGP = QD::NFGP, NVGP = QD::NVGP;
     constexpr int NVH = (NV + 1) / 2;          // variables per half in the reconstruction
     constexpr unsigned FULL = 0xffffffffu;
+    constexpr bool HAS_PAD = CONS ? N >= 1 : N >= 2;   // orders whose coefficients the admissibility check can replace
 
     if (p.sc->idle) return;   // finished or held run (set by begin_step; 0 outside a time loop)
 
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem_raw);
-    double *rows_s = reinterpret_cast<double *>(smem_raw + 128);
-    double *coef_s = rows_s + (size_t)SLOTS * K::SLOT_STRIDE;   // [k-1][c][cell]; later [F|D][c][cell]
-    double *yt_s = coef_s + K::COEF_ELEMS;                      // [q][c][cell]
-    double *carry_s = yt_s + K::YT_ELEMS;                       // [ncp|t1|gb|eb][c][cell]
+    double *rows_s = reinterpret_cast<double *>(smem_raw);
+    // conserved input of row r-1 (the row the RK combination finishes), [c][BW], its own mbarrier
+    double *orow_s = rows_s + (size_t)SLOTS * K::SLOT_STRIDE;
+    double *coef_s = orow_s + K::SLOT_STRIDE;                   // [slot][c][cell]
+    double *yt_s = coef_s + K::COEF_ELEMS;                      // [row parity][q][c][cell]
+    double *carry_s = yt_s + K::YT_ELEMS;                       // t1, G below [c][cell]; ncp, E below [z][cell]
+    uint64_t *bars = reinterpret_cast<uint64_t *>(carry_s + K::CARRY_ELEMS);
     // VISC: gradients of the variables the viscous flux reads (primitive u, v;
     // conserved a1r1, a2r2, ru, rv) at the top face, kept for the row above:
-    // [q][g][d][cell], right behind the carries
+    // [q][g][d][cell], right behind the barriers
     constexpr int NG = CONS ? 4 : 2, G0 = CONS ? 0 : 2;
-    // conserved input of row r-1 (the row the RK combination finishes), [c][BW], its own mbarrier
-    double *orow_s = carry_s + K::CARRY_ELEMS;
-    double *ygt_s = orow_s + K::SLOT_STRIDE;
+    double *ygt_s = carry_s + K::CARRY_ELEMS + 8;
+    double *red_s = carry_s;                                    // block reductions at the tile's end
 
     const int t = threadIdx.x;
     const int m = t >> 1;            // cell of this thread's pair
     const int h = t & 1;             // which half of the pair
+    const unsigned mask0 = h ? 0u : 0x80000000u;   // half 0's sign (add_term)
     // strips split the columns evenly on even boundaries (TMA x origin alignment);
     // row runs split the rows evenly
     const int x0 = 2 * (int)(((long long)strip * p.nx) / (2LL * p.strips));
@@ -220,13 +335,15 @@ __device__ __forceinline__ void stage_tile(const StageParams &p, const CUtensorM
     const bool active = m <= owc + 1;
     const bool owned = m >= 1 && m <= owc;
     const bool xface = m >= 1 && m <= owc + 1;
+    const bool warp_active = ((t & ~31) >> 1) <= owc + 1;   // some cell of this warp is in the strip
     const bool touches_x = (x0 == 0) || (x0 + owc >= p.nx);
     const int bcL = p.bc[0], bcR = p.bc[1], bcB = p.bc[2], bcT = p.bc[3];
     const bool py = (bcB == BC_PERIODIC || bcT == BC_PERIODIC);
     const double dt = (p.mode == OUT_RHS) ? 0.0 : p.sc->dt;
     const double b = dt / p.kb;   // the RK combination's dt/kb, the same for every row
-    const Eos eos = p.eos;
+    const auto &eos = p.eos;
     const double r1_h = p.r1_h;
+    const bool quick_eos = S::quick_eos(eos);   // pad_quick's accept holds for these constants
 
     __syncthreads();   // the previous tile of this block is done with every buffer
     if (t == 0) {
@@ -239,8 +356,49 @@ __device__ __forceinline__ void stage_tile(const StageParams &p, const CUtensorM
     int next_issue = row_lo, next_conv = row_lo;
     auto slot_of = [&](int row) { return (row - row_lo) % SLOTS; };
     auto row_ptr = [&](int row) { return rows_s + (size_t)slot_of(row) * K::SLOT_STRIDE; };   // [c][BW]
-    auto cidx = [&](int k1, int c, int cell) { return (k1 * NV + c) * CELLS + cell; };         // coef_s index, k1 = k-1
-    auto carry = [&](int which, int c) -> double & { return carry_s[(which * NV + c) * CELLS + m]; };
+    auto cidx = [&](int slot, int c, int cell) { return (slot * NV + c) * CELLS + cell; };     // coef_s index
+    auto t1_s = [&](int c) -> double & { return carry_s[c * CELLS + m]; };
+    auto g_s = [&](int c) -> double & { return carry_s[(NV + c) * CELLS + m]; };
+    auto ncp_s = [&](int z) -> double & { return carry_s[(2 * NV + z) * CELLS + m]; };
+    auto e_s = [&](int z) -> double & { return carry_s[(2 * NV + NZ + z) * CELLS + m]; };
+    // Component c = 2 j + h of the half, j compile time: a per-component register array's
+    // element, and whether and where the component has a non-conservative product
+    auto own = [&](auto jj, const double *a) {
+        constexpr int c0 = 2 * decltype(jj)::value, c1 = c0 + 1 < NV ? c0 + 1 : c0;
+        return h ? a[c1] : a[c0];
+    };
+    // the other half's component 2 j + 1 - h of the array, 0 where there is none
+    auto other = [&](auto jj, const double *a) {
+        constexpr int c0 = 2 * decltype(jj)::value, c1 = c0 + 1 < NV ? c0 + 1 : c0;
+        return h ? a[c0] : a[c1];
+    };
+
+    // A face's flux of component 2 j + h from its two Gauss points' weighted values, one per half:
+    // Flux = 0.0; Flux += w F(q0); Flux += w F(q1)   (rhs_function_prim.c:548-577),
+    // VISC: Flux += w Fv(q) after each Gauss point's convective part.  Each half sends the
+    // other the component it needs; two terms add up alike in either order
+    auto face_sum = [&](auto jj, const double *Fq, const double *Vq) {
+        if constexpr (NFGP > 1) {
+            const double f = own(jj, Fq), fo = __shfl_xor_sync(FULL, other(jj, Fq), 1);
+            if constexpr (VISC) {
+                const double v = own(jj, Vq), vo = __shfl_xor_sync(FULL, other(jj, Vq), 1);
+                return (((0.0 + (h ? fo : f)) + (h ? vo : v)) + (h ? f : fo)) + (h ? v : vo);
+            } else {
+                return (0.0 + f) + fo;
+            }
+        } else {
+            if constexpr (VISC) return (0.0 + own(jj, Fq)) + own(jj, Vq);
+            else return 0.0 + own(jj, Fq);
+        }
+    };
+    auto fluct_sum = [&](auto jj, const double *Dq) {
+        if constexpr (NFGP > 1) {
+            const double d = own(jj, Dq), d_o = __shfl_xor_sync(FULL, other(jj, Dq), 1);
+            return (0.0 + d) + d_o;
+        } else {
+            return 0.0 + own(jj, Dq);
+        }
+    };
 
     double smax_loc = 0.0, smaxv_loc = 0.0;
     bool bad = false;
@@ -259,148 +417,110 @@ __device__ __forceinline__ void stage_tile(const StageParams &p, const CUtensorM
         if (drained)
             for (int k = 0; k <= SLOTS; ++k) mbar_inval(&bars[k]);
     };
+    // thread 0: issue the ring rows up to `last`
+    auto issue_rows = [&](int last) {
+        for (; next_issue <= min(last, row_hi) && (!p.skip_loads || next_issue < p.skip_loads_from); ++next_issue) {
+            const int row = next_issue;
+            const int src = map_axis(row, p.ny, bcB, bcT);
+            uint64_t *bar = &bars[slot_of(row)];
+            mbar_expect_tx(bar, K::ROW_BYTES);
+            tma_load_3d(row_ptr(row), tmap, xs + p.col_off, src + p.row_off, 0, bar);   // the map starts col_off columns left of column 0, row_off rows below row 0
+        }
+    };
+    auto wait_row = [&](int row) { return mbar_wait_bounded(&bars[slot_of(row)], (unsigned)(((row - row_lo) / SLOTS) & 1)); };
+    // Ghost columns of a loaded row fetch their conserved source values; needs a block
+    // barrier before convert_row overwrites the sources
+    auto fetch_ghosts = [&](int row) {
+        const int cc = 1 + t, g = xs + cc;
+        if (cc > owc + 6 || (g >= 0 && g < p.nx)) return true;
+        if (!wait_row(row)) return false;
+        double *rp = row_ptr(row);
+        const int gm = map_axis(g, p.nx, bcL, bcR);
+        if (gm == g) return true;   // a block's halo column, loaded in place
+        if (gm - xs >= 0 && gm - xs < BW) {
+#pragma unroll
+            for (int c = 0; c < NV; ++c) rp[c * BW + cc] = rp[c * BW + (gm - xs)];
+        } else {
+            const int src = map_axis(row, p.ny, bcB, bcT);
+#pragma unroll
+            for (int c = 0; c < NV; ++c) rp[c * BW + cc] = p.in[(long long)c * p.plane + (long long)src * p.pitch + gm];
+        }
+        return true;
+    };
+    // Convert a loaded row in place, apply reflections and inlet values.  Columns
+    // cc = 1 .. owc+6 are the ones the stencils read
+    auto convert_row = [&](int row) {
+        const int cc = 1 + t;
+        if (cc > owc + 6) return;
+        double *rp = row_ptr(row);
+        const bool yg = row < 0 || row >= p.ny;
+        const bool yrefl = yg && ((row < 0 ? bcB : bcT) == BC_REFLECTIVE);
+        const int g = xs + cc;
+        const bool isg = g < 0 || g >= p.nx;
+        double Q[NV], V[NV];
+#pragma unroll
+        for (int c = 0; c < NV; ++c) Q[c] = rp[c * BW + cc];
+        if constexpr (CONS) {
+#pragma unroll
+            for (int c = 0; c < NV; ++c) V[c] = Q[c];
+        } else if constexpr (!FAST && ((SYS == SYS_BN && (N == 1 || N == 2)) || (SYS == SYS_KAPILA && N <= 1))) {
+            // branch-free correctly rounded divisions (hype_div.cuh): the cell's
+            // independent divisions overlap instead of each waiting on the last
+            // one's slow-path branch; the compiler's division where an operand is
+            // outside their range.  Only in the tiles where it measured faster
+            // (Kapila N = 2, 3 lose to the extra registers)
+            bool special = false;
+            S::cons2prim_dv(eos, Q, V, [&special](double a, double b) { return cr_div(a, b, special); });
+            if (special) S::cons2prim(eos, Q, V);
+        } else {
+            S::cons2prim(eos, Q, V);
+        }
+        if (isg) {
+            const int side_bc = g < 0 ? bcL : bcR;
+            if (side_bc == BC_INLET && p.inlet) {
+                const int jr = py ? row : map_axis(row, p.ny, bcB, bcT);
+#pragma unroll
+                for (int c = 0; c < NV; ++c) V[c] = p.inlet[((size_t)(g + 3) * (p.ny + 6) + (jr + 3)) * NV + c];
+            } else if (side_bc == BC_REFLECTIVE) {
+                if (S::RX0 >= 0) V[S::RX0] = -V[S::RX0];
+                if (S::RX1 >= 0) V[S::RX1] = -V[S::RX1];
+                if constexpr (VISC) V[S::RXV] = -V[S::RXV];
+            }
+        }
+        if (yrefl) {
+            if (S::RY0 >= 0) V[S::RY0] = -V[S::RY0];
+            if (S::RY1 >= 0) V[S::RY1] = -V[S::RY1];
+            if constexpr (VISC) V[S::RYV] = -V[S::RYV];
+        }
+#pragma unroll
+        for (int c = 0; c < NV; ++c) rp[c * BW + cc] = V[c];
+    };
+
+    // ---------------- prologue: rows y0-3 .. y0+1, row y0+2 in flight --------------
+    if (t == 0) {
+        fence_proxy_async();   // earlier generic accesses to the slots precede the TMA writes
+        issue_rows(y0 + 2);
+    }
+    {
+        bool here = true;
+        for (int row = row_lo; row <= y0 + 1; ++row) here = here && wait_row(row);
+        if (touches_x && here)
+            for (int row = row_lo; row <= y0 + 1; ++row) here = here && fetch_ghosts(row);
+        if (__syncthreads_or(!here)) {
+            give_up(false, 0u);
+            return;   // block-uniform exit; the caller's next barrier is block-uniform too
+        }
+        for (; next_conv <= y0 + 1; ++next_conv) convert_row(next_conv);
+    }
+    __syncthreads();
 
     for (int r = y0 - 1; r <= y0 + H; ++r) {
-        // this iteration finishes an owned row (r-1) with an RK combination that reads its input
-        const bool finish_row = r > y0 && p.mode != OUT_RHS;
-        // ---------------- A. bring rows up to r+2 into the ring --------------
-        if (t == 0) {
-            fence_proxy_async();   // earlier generic accesses to the slots precede the TMA writes
-            for (; next_issue <= min(r + 3, row_hi) && (!p.skip_loads || next_issue < p.skip_loads_from); ++next_issue) {
-                const int row = next_issue;
-                const int src = map_axis(row, p.ny, bcB, bcT);
-                uint64_t *bar = &bars[slot_of(row)];
-                mbar_expect_tx(bar, K::ROW_BYTES);
-                tma_load_3d(row_ptr(row), tmap, xs + p.col_off, src + p.row_off, 0, bar);   // the map starts col_off columns left of column 0, row_off rows below row 0
-            }
-            if (finish_row && (!p.skip_loads || r - 1 < p.skip_loads_from)) {   // row r-1's conserved input for the RK combination in section C
-                mbar_expect_tx(&bars[SLOTS], K::ROW_BYTES);
-                tma_load_3d(orow_s, tmap, xs + p.col_off, (r - 1) + p.row_off, 0, &bars[SLOTS]);
-            }
-        }
-        for (; next_conv <= r + 2; ++next_conv) {
-            const int row = next_conv;
-            const unsigned parity = (unsigned)(((row - row_lo) / SLOTS) & 1);
-            const bool ok = mbar_wait_bounded(&bars[slot_of(row)], parity);
-            if (__syncthreads_or(!ok)) {
-                give_up(finish_row && (!p.skip_loads || r - 1 < p.skip_loads_from), (unsigned)((r - y0 - 1) & 1));
-                return;   // block-uniform exit; the caller's next barrier is block-uniform too
-            }
-            double *rp = row_ptr(row);
-            const int src = map_axis(row, p.ny, bcB, bcT);
-            const bool yg = row < 0 || row >= p.ny;
-            const bool yrefl = yg && ((row < 0 ? bcB : bcT) == BC_REFLECTIVE);
-            // column cc = 1 + t; columns 1 .. owc+6 are the ones the stencils read
-            const int cc = 1 + t;
-            const bool conv = cc <= owc + 6;
-            const int g = xs + cc;
-            const bool isg = conv && (g < 0 || g >= p.nx);
-            double Q[NV];
-            if (touches_x) {
-                // Phase 1: ghost columns fetch their conserved source values before anyone converts
-                if (isg) {
-                    const int gm = map_axis(g, p.nx, bcL, bcR);
-                    if (gm - xs >= 0 && gm - xs < BW) {
-#pragma unroll
-                        for (int c = 0; c < NV; ++c) Q[c] = rp[c * BW + (gm - xs)];
-                    } else {
-#pragma unroll
-                        for (int c = 0; c < NV; ++c) Q[c] = p.in[(long long)c * p.plane + (long long)src * p.pitch + gm];
-                    }
-                }
-                __syncthreads();
-            }
-            // Phase 2: convert in place, apply reflections / inlet values
-            if (conv) {
-                if (!isg) {
-#pragma unroll
-                    for (int c = 0; c < NV; ++c) Q[c] = rp[c * BW + cc];
-                }
-                double V[NV];
-                if constexpr (CONS) {
-#pragma unroll
-                    for (int c = 0; c < NV; ++c) V[c] = Q[c];
-                } else if constexpr (!FAST && ((SYS == SYS_BN && (N == 1 || N == 2)) || (SYS == SYS_KAPILA && N <= 1))) {
-                    // branch-free correctly rounded divisions (hype_div.cuh): the cell's
-                    // independent divisions overlap instead of each waiting on the last
-                    // one's slow-path branch; the compiler's division where an operand is
-                    // outside their range.  Only in the tiles where it measured faster
-                    // (Kapila N = 2, 3 lose to the extra registers)
-                    bool special = false;
-                    S::cons2prim_dv(eos, Q, V, [&special](double a, double b) { return cr_div(a, b, special); });
-                    if (special) S::cons2prim(eos, Q, V);
-                } else {
-                    S::cons2prim(eos, Q, V);
-                }
-                if (isg) {
-                    const int side_bc = g < 0 ? bcL : bcR;
-                    if (side_bc == BC_INLET && p.inlet) {
-                        const int jr = py ? row : map_axis(row, p.ny, bcB, bcT);
-#pragma unroll
-                        for (int c = 0; c < NV; ++c) V[c] = p.inlet[((size_t)(g + 3) * (p.ny + 6) + (jr + 3)) * NV + c];
-                    } else if (side_bc == BC_REFLECTIVE) {
-                        if (S::RX0 >= 0) V[S::RX0] = -V[S::RX0];
-                        if (S::RX1 >= 0) V[S::RX1] = -V[S::RX1];
-                        if constexpr (VISC) V[S::RXV] = -V[S::RXV];
-                    }
-                }
-                if (yrefl) {
-                    if (S::RY0 >= 0) V[S::RY0] = -V[S::RY0];
-                    if (S::RY1 >= 0) V[S::RY1] = -V[S::RY1];
-                    if constexpr (VISC) V[S::RYV] = -V[S::RYV];
-                }
-#pragma unroll
-                for (int c = 0; c < NV; ++c) rp[c * BW + cc] = V[c];
-            }
-        }
-        if (finish_row) {   // the copy of row r-1 issued at the start of this iteration
-            const unsigned parity = (unsigned)((r - y0 - 1) & 1);
-            const bool ok = mbar_wait_bounded(&bars[SLOTS], parity);
-            if (__syncthreads_or(!ok)) {
-                give_up(false, 0u);   // the finish-row load is the one that did not come
-                return;   // block-uniform exit
-            }
-        }
-        __syncthreads();   // S1: prim rows r-2 .. r+2 ready
-
-        // ---------------- B. reconstruction of cell (r, i), split by variable ---
+        const bool in_rows = r >= y0;
+        const bool full_row = r >= y0 && r < y0 + H;
+        const int q = NFGP > 1 ? h : 0;
         const int ccm = m + 3;                                    // column of i in the ring rows
         const double *w_m2 = row_ptr(r - 2), *w_m1 = row_ptr(r - 1), *w_0 = row_ptr(r), *w_p1 = row_ptr(r + 1), *w_p2 = row_ptr(r + 2);
-        if (active) {
-#pragma unroll 1
-            for (int kv = 0; kv < NVH; ++kv) {
-                const int c = h * NVH + kv;
-                if (c >= NV) break;
-                Stencil st;
-                const double *a0 = w_0 + c * BW + ccm;
-                st.c = a0[0];
-                st.xm2 = a0[-2]; st.xm1 = a0[-1]; st.xp1 = a0[1]; st.xp2 = a0[2];
-                st.ym2 = w_m2[c * BW + ccm]; st.ym1 = w_m1[c * BW + ccm]; st.yp1 = w_p1[c * BW + ccm]; st.yp2 = w_p2[c * BW + ccm];
-                st.pp = w_p1[c * BW + ccm + 1]; st.pm = w_m1[c * BW + ccm + 1]; st.mp = w_p1[c * BW + ccm - 1]; st.mm = w_m1[c * BW + ccm - 1];
-                double cf[NDOF];
-                if constexpr (FAST) {
-                    ReconFast<N>::run(st, cf);
-                } else if constexpr (SYS == SYS_BN && N == 2) {
-                    // branch-free correctly rounded divisions let the weights' chains overlap
-                    // (the Baer-Nunziato tile runs 8 warps per SM); the compiler's division
-                    // where an operand is outside their range
-                    bool special = false;
-                    Recon2Cr::run(st, cf, special);
-                    if (special) Recon<N>::run(st, cf);
-                } else {
-                    Recon<N>::run(st, cf);
-                }
-#pragma unroll
-                for (int k = 1; k < NDOF; ++k) coef_s[cidx(k - 1, c, m)] = cf[k];
-            }
-        }
-        __syncwarp();
-        // own coefficients of one variable of cell `cell`, k = 0 from the ring row
-        auto load_cf = [&](int c, int cell, double *cf) {
-            cf[0] = w_0[c * BW + cell + 3];
-#pragma unroll
-            for (int k = 1; k < NDOF; ++k) cf[k] = coef_s[cidx(k - 1, c, cell)];
-        };
+        const bool finish_row = r > y0 && p.mode != OUT_RHS;   // this iteration's RK combination reads row r-1's input
         // VISC: unlimited coefficients of variable c of the cell `cell` of row r, from the ring rows
         auto load_uc = [&](int c, int cell, double *uc) {
             if constexpr (VISC) {
@@ -414,77 +534,156 @@ __device__ __forceinline__ void stage_tile(const StageParams &p, const CUtensorM
                 UCoef<N>::run(st, uc);
             }
         };
-        // admissibility at the nodes (rhs_function_prim.c:382-404), nodes split between the pair
-        bool ok = true;
-        if (active) {
-            static_for<NNODE / 2>([&](auto sq) {
-                constexpr int s0 = decltype(sq)::value, s1 = NNODE / 2 + s0;
-                if (!ok) return;
-                double V[NV];
+        // finish_row: row r-1's conserved input, issued in the previous iteration
+        bool here = !finish_row || mbar_wait_bounded(&bars[SLOTS], (unsigned)((r - y0 - 1) & 1));
+
+        if (warp_active) {
+        // ---------------- A. reconstruction of cell (r, i), split by variable ---
+#pragma unroll 1
+        for (int kv = 0; kv < NVH; ++kv) {
+            const int c = h * NVH + kv;
+            if (c >= NV) break;
+            Stencil st;
+            const double *a0 = w_0 + c * BW + ccm;
+            st.c = a0[0];
+            st.xm2 = a0[-2]; st.xm1 = a0[-1]; st.xp1 = a0[1]; st.xp2 = a0[2];
+            st.ym2 = w_m2[c * BW + ccm]; st.ym1 = w_m1[c * BW + ccm]; st.yp1 = w_p1[c * BW + ccm]; st.yp2 = w_p2[c * BW + ccm];
+            st.pp = w_p1[c * BW + ccm + 1]; st.pm = w_m1[c * BW + ccm + 1]; st.mp = w_p1[c * BW + ccm - 1]; st.mm = w_m1[c * BW + ccm - 1];
+            double cf[NDOF];
+            if constexpr (FAST) {
+                ReconFast<N>::run(st, cf);
+            } else if constexpr (SYS == SYS_BN && N == 2) {
+                // branch-free correctly rounded divisions let the weights' chains overlap
+                // (the Baer-Nunziato tile runs 8 warps per SM); the compiler's division
+                // where an operand is outside their range
+                bool special = false;
+                Recon2Cr::run(st, cf, special);
+                if (special && active) Recon<N>::run(st, cf);
+            } else {
+                Recon<N>::run(st, cf);
+            }
 #pragma unroll
-                for (int c = 0; c < NV; ++c) {
-                    double cf[NDOF];
-                    load_cf(c, m, cf);
-                    double v = 0.0;
-                    static_for<NDOF>([&](auto kk) {
-                        constexpr int k = decltype(kk)::value;
-                        constexpr double p0 = QD::phi_node(s0, k), p1 = QD::phi_node(s1, k);
-                        if constexpr (p0 == p1) {
-                            if constexpr (p0 != 0.0) { if constexpr (p0 == 1.0) v = v + cf[k]; else v = v + cf[k] * p0; }
-                        } else {
-                            v = v + cf[k] * (h ? p1 : p0);
-                        }
-                    });
-                    V[c] = v;
-                }
-                if constexpr (CONS) ok = S::pad_cons(eos, V);
-                else ok = S::pad(eos, V);
-            });
+            for (int k = 1; k < NDOF; ++k) coef_s[cidx(k - 1, c, m)] = cf[k];
         }
-        {
+        __syncwarp();
+
+        // ---------------- B. point values of the cell, all variables ----------------
+        // bottom and (old) top values at the y-face's Gauss point, values and gradients at
+        // the half's volume Gauss points in registers; left, right and (new) top in shared memory
+        constexpr int QH = NVGP > 1 ? NVGP / 2 : 1;
+        double VR[NV];                              // bottom values
+        const double *yt_lo = yt_s + ((((r - y0) & 1) * NFGP + q) * NV) * CELLS + m;     // top values of row r-1,
+        double *yt_up = yt_s + ((((r - y0 + 1) & 1) * NFGP + q) * NV) * CELLS + m;       // and of row r
+        double tq[QH][NV];                          // weighted volume products
+        bool ok = quick_eos;                        // every node in the plainly admissible range
+        // the point values from the coefficients that coef(c, cf) gives
+        auto points = [&](auto coef) {
+            double Vv[QH][NV], gx[QH][NV], gy[QH][NV];
+            static_for<NV>([&](auto sc_) {
+                constexpr int c = S::order(decltype(sc_)::value);   // the product's velocity part first: fewer values wait for it
+                double cf[NDOF];
+                cf[0] = w_0[c * BW + ccm];
+                coef(c, cf);
+                const double vl = face_pt<N, 0, FAST>(cf, mask0), vr = face_pt<N, 1, FAST>(cf, mask0);
+                const double vt = face_pt<N, 3, FAST>(cf, mask0);
+                VR[c] = face_pt<N, 2, FAST>(cf, mask0);
+                coef_s[cidx(2 * q, c, m)] = vl;
+                coef_s[cidx(2 * q + 1, c, m)] = vr;
+                yt_up[c * CELLS] = vt;
+                if constexpr (HAS_PAD && !CONS)
+                    ok = ok && S::template pad_quick<c>(vl) && S::template pad_quick<c>(vr) && S::template pad_quick<c>(VR[c]) &&
+                         S::template pad_quick<c>(vt);
+                if constexpr (NZ > 0) {
+                    static_for<QH>([&](auto sa) {
+                        constexpr int a = decltype(sa)::value;
+                        Vv[a][c] = vol_pt<N, a, FAST>(cf, mask0);
+                        gx[a][c] = r1_h * vol_grad<N, a, 0, FAST>(cf, mask0);
+                        gy[a][c] = r1_h * vol_grad<N, a, 1, FAST>(cf, mask0);
+                    });
+                }
+            });
+            // the volume non-conservative products (rhs_function_prim.c:459-479)
+            if constexpr (NZ > 0) {
+                static_for<QH>([&](auto sa) {
+                    constexpr int a = decltype(sa)::value;
+                    double B[NV];
+                    if constexpr (CONS) S::ncp_cons(eos, Vv[a], gx[a], gy[a], B);
+                    else S::ncp(eos, Vv[a], gx[a], gy[a], B);
+#pragma unroll
+                    for (int c = 0; c < NV; ++c) tq[a][c] = -QD::wv(0) * B[c];
+                });
+            }
+        };
+        points([&](int c, double *cf) {
+#pragma unroll
+            for (int k = 1; k < NDOF; ++k) cf[k] = coef_s[cidx(k - 1, c, m)];
+            __syncwarp();   // both halves have the variable's coefficients: its face values may replace them
+        });
+        if constexpr (HAS_PAD) {
+            // admissibility at the nodes (rhs_function_prim.c:382-404): the four faces' values at
+            // this half's Gauss point
+            if (active && (CONS || !ok)) {
+                ok = true;
+#pragma unroll 1
+                for (int f = 0; f < 4 && ok; ++f) {
+                    double V[NV];
+#pragma unroll
+                    for (int c = 0; c < NV; ++c) V[c] = f == 0 ? VR[c] : f < 3 ? coef_s[cidx(2 * q + f - 1, c, m)] : yt_up[c * CELLS];
+                    ok = CONS ? S::pad_cons(eos, V) : S::pad(eos, V);
+                }
+            }
             // every lane takes part in the shuffle (no short-circuit around it)
             const int ok_pair = __shfl_xor_sync(FULL, (int)ok, 1);
-            ok = ok && (ok_pair != 0);
-        }
-        if (CONS && !ok && N >= 1 && active) {   // rhs_function.c:410-420: the slopes are zeroed from k = 1 on
-#pragma unroll 1
-            for (int kv = 0; kv < NVH; ++kv) {
-                const int c = h * NVH + kv;
-                if (c >= NV) break;
+            if (active && !(ok && ok_pair)) {
+                // the fallback's coefficients: [w, minmod_x, minmod_y, 0 ...] (rhs_function_prim.c:407-421);
+                // conservative path: the mean alone (rhs_function.c:410-420)
+                points([&](int c, double *cf) {
 #pragma unroll
-                for (int k = 1; k < NDOF; ++k) coef_s[cidx(k - 1, c, m)] = 0.0;
-            }
-        }
-        if (!CONS && !ok && N >= 2 && active) {   // rhs_function_prim.c:407-421: [w, minmod_x, minmod_y, 0 ...]
-#pragma unroll 1
-            for (int kv = 0; kv < NVH; ++kv) {
-                const int c = h * NVH + kv;
-                if (c >= NV) break;
-                const double w0 = w_0[c * BW + ccm];
-                coef_s[cidx(0, c, m)] = minmod(w_0[c * BW + ccm + 1] - w0, w0 - w_0[c * BW + ccm - 1]);
-                coef_s[cidx(1, c, m)] = minmod(w_p1[c * BW + ccm] - w0, w0 - w_m1[c * BW + ccm]);
-#pragma unroll
-                for (int k = 3; k < NDOF; ++k) coef_s[cidx(k - 1, c, m)] = 0.0;
+                    for (int k = 1; k < NDOF; ++k) cf[k] = 0.0;
+                    if constexpr (!CONS && N >= 2) {
+                        const double *a0 = w_0 + c * BW + ccm;
+                        cf[1] = minmod(a0[1] - cf[0], cf[0] - a0[-1]);
+                        cf[2] = minmod(w_p1[c * BW + ccm] - cf[0], cf[0] - w_m1[c * BW + ccm]);
+                    }
+                });
             }
         }
         __syncwarp();
 
-        // ---------------- C. y-face below (r, i): Gauss point q = h ----------------
-        const bool in_rows = r >= y0 && r <= y0 + H;
-        const int q = NFGP > 1 ? h : 0;
+        // ---------------- C. volume non-conservative term: the pair's sum
+        double vol[(NV + 1) / 2];   // of components 2 j + h; kept once row r-1 has read its own
+        if constexpr (NZ > 0) {
+            // rhs = 0.0; rhs += -w_q B_q for q = 0..NVGP-1; the pair holds q = 2h, 2h+1
+            static_for<(NV + 1) / 2>([&](auto jj) {
+                constexpr int j = decltype(jj)::value, z0 = K::nz(2 * j), z1 = 2 * j + 1 < NV ? K::nz(2 * j + 1) : -1;
+                if constexpr (z0 >= 0 || z1 >= 0) {
+                    double acc = 0.0;
+                    if constexpr (NVGP > 1) {
+                        double parts[NVGP];
+#pragma unroll
+                        for (int a = 0; a < QH; ++a) {
+                            const double mine = own(jj, tq[a]), got = __shfl_xor_sync(FULL, other(jj, tq[a]), 1);
+                            parts[a] = h ? got : mine;
+                            parts[QH + a] = h ? mine : got;
+                        }
+#pragma unroll
+                        for (int a = 0; a < NVGP; ++a) acc += parts[a];
+                    } else {
+                        acc = 0.0 + own(jj, tq[0]);
+                    }
+                    vol[j] = acc;
+                }
+            });
+        }
+
+        // ---------------- D. y-face below (r, i): Gauss point q = h ----------------
         {
-            double G[NV], E[NV];
             const bool doit = owned && in_rows;
             double Fq[NV], Dq[NV], Vq[NV];
             if (doit) {
-                double VL[NV], VR[NV];
+                double VL[NV];
 #pragma unroll
-                for (int c = 0; c < NV; ++c) {
-                    double cf[NDOF];
-                    load_cf(c, m, cf);
-                    VR[c] = face_val<N, 2>(cf, q);
-                    VL[c] = yt_s[(q * NV + c) * CELLS + m];
-                }
+                for (int c = 0; c < NV; ++c) VL[c] = yt_lo[c * CELLS];
                 const double s = riemann_gp<S, 1, CONS>(eos, VL, VR, Fq, Dq, bad);
                 smax_loc = fmax(smax_loc, s);
 #pragma unroll
@@ -514,53 +713,37 @@ __device__ __forceinline__ void stage_tile(const StageParams &p, const CUtensorM
 #pragma unroll
                     for (int c = 0; c < NV; ++c) Vq[c] = QD::wf(0) * (0.5 * (FvR[c] + FvL[c]));
                 }
+                if (bad && bad_cell == 0xffffffffu) bad_cell = (unsigned)(r * p.nx + i);
             } else {
 #pragma unroll
                 for (int c = 0; c < NV; ++c) { Fq[c] = 0.0; Dq[c] = 0.0; Vq[c] = 0.0; }
             }
-            // Flux = 0.0; Flux += w F(q0); Flux += w F(q1)   (rhs_function_prim.c:548-577),
-            // VISC: Flux += w Fv(q) after each Gauss point's convective part
-#pragma unroll
-            for (int c = 0; c < NV; ++c) {
-                if constexpr (NFGP > 1) {
-                    const double fo = __shfl_xor_sync(FULL, Fq[c], 1), d_o = __shfl_xor_sync(FULL, Dq[c], 1);
-                    const double f0 = h ? fo : Fq[c], f1 = h ? Fq[c] : fo;
-                    const double d0 = h ? d_o : Dq[c], d1 = h ? Dq[c] : d_o;
-                    if constexpr (VISC) {
-                        const double vo = __shfl_xor_sync(FULL, Vq[c], 1);
-                        const double v0 = h ? vo : Vq[c], v1 = h ? Vq[c] : vo;
-                        G[c] = (((0.0 + f0) + v0) + f1) + v1;
-                    } else {
-                        G[c] = (0.0 + f0) + f1;
-                    }
-                    E[c] = (0.0 + d0) + d1;
-                } else {
-                    if constexpr (VISC) G[c] = (0.0 + Fq[c]) + Vq[c];
-                    else G[c] = 0.0 + Fq[c];
-                    E[c] = 0.0 + Dq[c];
-                }
-            }
-            if (doit && bad && bad_cell == 0xffffffffu) bad_cell = (unsigned)(r * p.nx + i);
-            if (doit) {
+            static_for<(NV + 1) / 2>([&](auto jj) {
+                constexpr int j = decltype(jj)::value, z0 = K::nz(2 * j), z1 = 2 * j + 1 < NV ? K::nz(2 * j + 1) : -1;
+                const double Gc = face_sum(jj, Fq, Vq);
+                double Ec = 0.0;
+                if constexpr (z0 >= 0 || z1 >= 0) Ec = fluct_sum(jj, Dq);
+                if (!doit || (2 * j + 1 >= NV && h)) return;   // odd NV: the last variable is half 0's alone
+                const int c = 2 * j + h;
+                const int z = h ? z1 : z0;
                 if (r > y0) {
                     // row r-1: rhs = ncp + ((-1/h) X - (1/h) Y)  (rhs_function_prim.c:589-602), then the RK combination
                     const int jo = r - 1;
                     const size_t gidx = (size_t)jo * p.pitch + i;
-                    // the halves take alternate variables, c = 2 j + h, so every lane works in every pass
-#pragma unroll
-                    for (int j = 0; j < (NV + 1) / 2; ++j) {
-                        if (2 * j + 1 >= NV && h) continue;   // odd NV: the last variable is half 0's alone
-                        const int c = 2 * j + h;
-                        const double Gc = h ? G[2 * j + 1 < NV ? 2 * j + 1 : 2 * j] : G[2 * j];
-                        const double Ec = h ? E[2 * j + 1 < NV ? 2 * j + 1 : 2 * j] : E[2 * j];
-                        const double Y = Gc - carry(2, c) + 0.5 * (Ec + carry(3, c));
-                        const double ty = r1_h * Y;
-                        const double rhs = carry(0, c) + (carry(1, c) - ty);
-                        if (p.mode == OUT_RHS) {
-                            if (p.out_aos) p.out[((size_t)jo * p.nx + i) * NV + c] = rhs;
-                            else p.out[(size_t)c * p.plane + gidx] = rhs;
-                            continue;
+                    double Y = Gc - g_s(c);
+                    double ncp = 0.0;
+                    if constexpr (z0 >= 0 || z1 >= 0) {   // a component without a product adds 0.5 (0 + 0)
+                        if (z >= 0) {
+                            Y = Y + 0.5 * (Ec + e_s(z));
+                            ncp = ncp_s(z);
                         }
+                    }
+                    const double ty = r1_h * Y;
+                    const double rhs = ncp + (t1_s(c) - ty);
+                    if (p.mode == OUT_RHS) {
+                        if (p.out_aos) p.out[((size_t)jo * p.nx + i) * NV + c] = rhs;
+                        else p.out[(size_t)c * p.plane + gidx] = rhs;
+                    } else {
                         const double Sv = orow_s[c * BW + ccm];   // = p.in[c * plane + gidx], staged by TMA
                         const double bF = b * rhs;
                         double o;
@@ -589,116 +772,58 @@ __device__ __forceinline__ void stage_tile(const StageParams &p, const CUtensorM
                             p.push_hi[(long long)c * p.push_plane_hi + (long long)(jo + p.push_shift_hi) * p.pitch + i] = o;
                     }
                 }
-#pragma unroll
-                for (int j = 0; j < (NV + 1) / 2; ++j) {
-                    if (2 * j + 1 >= NV && h) continue;
-                    const int c = 2 * j + h;
-                    carry(2, c) = h ? G[2 * j + 1 < NV ? 2 * j + 1 : 2 * j] : G[2 * j];
-                    carry(3, c) = h ? E[2 * j + 1 < NV ? 2 * j + 1 : 2 * j] : E[2 * j];
-                }
-            }
-        }
-
-        // ---------------- D. keep the top-face values (Gauss point q) for row r+1 --
-        if (owned && r >= y0 - 1 && r < y0 + H && (NFGP > 1 || h == 0)) {
-#pragma unroll
-            for (int c = 0; c < NV; ++c) {
-                double cf[NDOF];
-                load_cf(c, m, cf);
-                yt_s[(q * NV + c) * CELLS + m] = face_val<N, 3>(cf, q);
-            }
-            if constexpr (VISC) {
-#pragma unroll
-                for (int g = 0; g < NG; ++g) {
-                    double uc[NDOF];
-                    load_uc(G0 + g, m, uc);
-                    ygt_s[((q * NG + g) * 2 + 0) * CELLS + m] = r1_h * face_grad<N, 3, 0>(uc, q);
-                    ygt_s[((q * NG + g) * 2 + 1) * CELLS + m] = r1_h * face_grad<N, 3, 1>(uc, q);
-                }
-            }
-        }
-
-        // ---------------- E. volume non-conservative term (rhs_function_prim.c:459-479)
-        const bool full_row = r >= y0 && r < y0 + H;
-        {
-            // rhs = 0.0; rhs += -w_q B_q for q = 0..NVGP-1; the pair holds q = 2h, 2h+1
-            constexpr int QH = NVGP > 1 ? NVGP / 2 : 1;
-            double tq[QH][NV];
-#pragma unroll
-            for (int a = 0; a < QH; ++a)
-#pragma unroll
-                for (int c = 0; c < NV; ++c) tq[a][c] = 0.0;
-            const bool doit = owned && full_row && (NVGP > 1 || h == 0);
-            if (doit) {
-                static_for<QH>([&](auto sa) {
-                    constexpr int a = decltype(sa)::value;
-                    constexpr int q0 = a, q1 = (NVGP > 1 ? QH : 0) + a;   // half 0 -> q0, half 1 -> q1
-                    double V[NV], gx[NV], gy[NV], B[NV];
-#pragma unroll
-                    for (int c = 0; c < NV; ++c) {
-                        double cf[NDOF];
-                        load_cf(c, m, cf);
-                        double v = 0.0, dx = 0.0, dy = 0.0;
-                        static_for<NDOF>([&](auto kk) {
-                            constexpr int k = decltype(kk)::value;
-                            constexpr double pv0 = QD::phi_vol(q0, k), pv1 = QD::phi_vol(q1, k);
-                            constexpr double px0 = QD::dphi_vol_x(q0, k), px1 = QD::dphi_vol_x(q1, k);
-                            constexpr double py0 = QD::dphi_vol_y(q0, k), py1 = QD::dphi_vol_y(q1, k);
-                            if constexpr (pv0 == pv1) { if constexpr (pv0 != 0.0) { if constexpr (pv0 == 1.0) v = v + cf[k]; else v = v + cf[k] * pv0; } }
-                            else v = v + cf[k] * (h ? pv1 : pv0);
-                            if constexpr (px0 == px1) { if constexpr (px0 != 0.0) { if constexpr (px0 == 1.0) dx = dx + cf[k]; else dx = dx + cf[k] * px0; } }
-                            else dx = dx + cf[k] * (h ? px1 : px0);
-                            if constexpr (py0 == py1) { if constexpr (py0 != 0.0) { if constexpr (py0 == 1.0) dy = dy + cf[k]; else dy = dy + cf[k] * py0; } }
-                            else dy = dy + cf[k] * (h ? py1 : py0);
-                        });
-                        V[c] = v; gx[c] = r1_h * dx; gy[c] = r1_h * dy;
+                g_s(c) = Gc;
+                if constexpr (z0 >= 0 || z1 >= 0) {
+                    if (z >= 0) {
+                        e_s(z) = Ec;
+                        ncp_s(z) = vol[j];
                     }
-                    if constexpr (CONS) S::ncp_cons(eos, V, gx, gy, B);
-                    else S::ncp(eos, V, gx, gy, B);
-#pragma unroll
-                    for (int c = 0; c < NV; ++c) tq[a][c] = -QD::wv(0) * B[c];
-                });
-            }
-            static_for<NV>([&](auto cc_) {
-                constexpr int c = decltype(cc_)::value;
-                if constexpr (!(CONS ? S::ncp_cons_nonzero(c) : S::ncp_nonzero(c))) {
-                    // B[c] is the constant 0.0 for every Gauss point: ((0 + -0) + -0) ... = +0
-                    if (owned && full_row && (c & 1) == h) carry(0, c) = 0.0;
-                } else if constexpr (NVGP > 1) {
-                    double parts[NVGP];
-#pragma unroll
-                    for (int a = 0; a < QH; ++a) {
-                        const double o = __shfl_xor_sync(FULL, tq[a][c], 1);
-                        parts[a] = h ? o : tq[a][c];
-                        parts[QH + a] = h ? tq[a][c] : o;
-                    }
-                    double acc = 0.0;
-#pragma unroll
-                    for (int a = 0; a < NVGP; ++a) acc += parts[a];
-                    if (owned && full_row && (c & 1) == h) carry(0, c) = acc;
-                } else {
-                    const double o = __shfl_xor_sync(FULL, tq[0][c], 1);
-                    const double acc = 0.0 + (h ? o : tq[0][c]);
-                    if (owned && full_row && (c & 1) == h) carry(0, c) = acc;
                 }
             });
+            if constexpr (VISC) {   // the top face's gradients for the row above
+                if (owned && r < y0 + H && (NFGP > 1 || h == 0)) {
+#pragma unroll
+                    for (int g = 0; g < NG; ++g) {
+                        double uc[NDOF];
+                        load_uc(G0 + g, m, uc);
+                        ygt_s[((q * NG + g) * 2 + 0) * CELLS + m] = r1_h * face_grad<N, 3, 0>(uc, q);
+                        ygt_s[((q * NG + g) * 2 + 1) * CELLS + m] = r1_h * face_grad<N, 3, 1>(uc, q);
+                    }
+                }
+            }
         }
-        __syncthreads();   // S2: every column's coefficients of row r visible
+        }   // warp_active
 
-        // ---------------- F. x-face at the left of column i: Gauss point q ----------
-        double Fx[NV], Dx[NV];
-        {
-            const bool doit = xface && full_row;
+        const bool conv = r + 3 <= row_hi;   // row r+3 is converted in this iteration
+        if (touches_x && conv) here = fetch_ghosts(r + 3) && here;
+        // the loads of the next iteration: row r's input, and row r+4 into the slot of row r-2
+        const bool load_orow = full_row && p.mode != OUT_RHS && (!p.skip_loads || r < p.skip_loads_from);
+        auto issue_next = [&] {
+            if (t != 0) return;
+            fence_proxy_async();   // the block's accesses to the slots precede the TMA writes
+            issue_rows(r + 4);
+            if (load_orow) {
+                mbar_expect_tx(&bars[SLOTS], K::ROW_BYTES);
+                tma_load_3d(orow_s, tmap, xs + p.col_off, r + p.row_off, 0, &bars[SLOTS]);
+            }
+        };
+        // S1: every column's face values of row r visible, ghost columns fetched
+        if (__syncthreads_or(!here)) {
+            give_up(finish_row && (!p.skip_loads || r - 1 < p.skip_loads_from), (unsigned)((r - y0 - 1) & 1));
+            return;   // block-uniform exit
+        }
+        if constexpr (!VISC) issue_next();
+
+        // ---------------- E. x-face at the left of column i: Gauss point q ----------
+        double Fown[(NV + 1) / 2], Down[(NV + 1) / 2];   // components 2 j + h
+        if (warp_active && full_row) {
             double Fq[NV], Dq[NV], Vq[NV];
-            if (doit) {
+            if (xface) {
                 double VL[NV], VR[NV];
 #pragma unroll
                 for (int c = 0; c < NV; ++c) {
-                    double cl[NDOF], cr[NDOF];
-                    load_cf(c, m - 1, cl);
-                    load_cf(c, m, cr);
-                    VL[c] = face_val<N, 1>(cl, q);
-                    VR[c] = face_val<N, 0>(cr, q);
+                    VL[c] = coef_s[cidx(2 * q + 1, c, m - 1)];
+                    VR[c] = coef_s[cidx(2 * q, c, m)];
                 }
                 const double s = riemann_gp<S, 0, CONS>(eos, VL, VR, Fq, Dq, bad);
                 smax_loc = fmax(smax_loc, s);
@@ -735,55 +860,47 @@ __device__ __forceinline__ void stage_tile(const StageParams &p, const CUtensorM
 #pragma unroll
                 for (int c = 0; c < NV; ++c) { Fq[c] = 0.0; Dq[c] = 0.0; Vq[c] = 0.0; }
             }
-#pragma unroll
-            for (int c = 0; c < NV; ++c) {
-                if constexpr (NFGP > 1) {
-                    const double fo = __shfl_xor_sync(FULL, Fq[c], 1), d_o = __shfl_xor_sync(FULL, Dq[c], 1);
-                    const double f0 = h ? fo : Fq[c], f1 = h ? Fq[c] : fo;
-                    const double d0 = h ? d_o : Dq[c], d1 = h ? Dq[c] : d_o;
-                    if constexpr (VISC) {
-                        const double vo = __shfl_xor_sync(FULL, Vq[c], 1);
-                        const double v0 = h ? vo : Vq[c], v1 = h ? Vq[c] : vo;
-                        Fx[c] = (((0.0 + f0) + v0) + f1) + v1;
-                    } else {
-                        Fx[c] = (0.0 + f0) + f1;
-                    }
-                    Dx[c] = (0.0 + d0) + d1;
-                } else {
-                    if constexpr (VISC) Fx[c] = (0.0 + Fq[c]) + Vq[c];
-                    else Fx[c] = 0.0 + Fq[c];
-                    Dx[c] = 0.0 + Dq[c];
-                }
-            }
+            __syncwarp();   // both halves have their left values: the fluxes may replace them
+            static_for<(NV + 1) / 2>([&](auto jj) {
+                constexpr int j = decltype(jj)::value, z0 = K::nz(2 * j), z1 = 2 * j + 1 < NV ? K::nz(2 * j + 1) : -1;
+                Fown[j] = face_sum(jj, Fq, Vq);
+                Down[j] = 0.0;
+                if constexpr (z0 >= 0 || z1 >= 0) Down[j] = fluct_sum(jj, Dq);
+                if (!xface || (2 * j + 1 >= NV && h)) return;
+                coef_s[cidx(0, 2 * j + h, m)] = Fown[j];
+                if constexpr (z0 >= 0 || z1 >= 0) coef_s[cidx(2, 2 * j + h, m)] = Down[j];
+            });
         }
-        __syncthreads();   // S3: coefficient reads done; the buffer now carries face fluxes
-        if (xface && full_row) {
-#pragma unroll
-            for (int j = 0; j < (NV + 1) / 2; ++j) {
-                if (2 * j + 1 >= NV && h) continue;
-                const int c = 2 * j + h;
-                coef_s[c * CELLS + m] = h ? Fx[2 * j + 1 < NV ? 2 * j + 1 : 2 * j] : Fx[2 * j];
-                coef_s[(NV + c) * CELLS + m] = h ? Dx[2 * j + 1 < NV ? 2 * j + 1 : 2 * j] : Dx[2 * j];
-            }
+        bool late = false;
+        if (conv) {
+            late = !wait_row(r + 3);
+            if (!late) convert_row(r + 3);
+            ++next_conv;
         }
-        __syncthreads();   // S4
+        // S2: the x-face fluxes and prim rows r-1 .. r+3 ready
+        if (__syncthreads_or(late)) {
+            --next_conv;
+            give_up(load_orow && !VISC, (unsigned)((r - y0) & 1));
+            return;   // block-uniform exit
+        }
+        if constexpr (VISC) issue_next();
         if (owned && full_row) {
-#pragma unroll
-            for (int j = 0; j < (NV + 1) / 2; ++j) {
-                if (2 * j + 1 >= NV && h) continue;
+            static_for<(NV + 1) / 2>([&](auto jj) {
+                constexpr int j = decltype(jj)::value, z0 = K::nz(2 * j), z1 = 2 * j + 1 < NV ? K::nz(2 * j + 1) : -1;
+                if (2 * j + 1 >= NV && h) return;
                 const int c = 2 * j + h;
-                const double Fc = h ? Fx[2 * j + 1 < NV ? 2 * j + 1 : 2 * j] : Fx[2 * j];
-                const double Dc = h ? Dx[2 * j + 1 < NV ? 2 * j + 1 : 2 * j] : Dx[2 * j];
-                const double F1 = coef_s[c * CELLS + m + 1], D1 = coef_s[(NV + c) * CELLS + m + 1];
-                const double X = F1 - Fc + 0.5 * (D1 + Dc);
-                carry(1, c) = -r1_h * X;
-            }
+                double X = coef_s[cidx(0, c, m + 1)] - Fown[j];
+                if constexpr (z0 >= 0 || z1 >= 0) {
+                    if ((h ? z1 : z0) >= 0) X = X + 0.5 * (coef_s[cidx(2, c, m + 1)] + Down[j]);
+                }
+                t1_s(c) = -r1_h * X;
+            });
         }
     }
 
     // ---------------- CFL maximum: warp shuffle, block, one atomic ------------
     if (bad) raise_error(p.sc, ERR_INADMISSIBLE_FACE, bad_cell);
-    __syncthreads();   // red_s is reused tile after tile
+    __syncthreads();   // the carries are done with: red_s takes their place
     if (p.reduce_smax) {
         double mx = smax_loc;
 #pragma unroll

@@ -25,8 +25,7 @@ __global__ void __launch_bounds__(2 * STAGE_CELLS, 1)
 stage_visc_kernel(const __grid_constant__ CUtensorMap tmap, const StageParams p)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ double red_s[2 * STAGE_CELLS / 32];
-    stage_tile<SYS_KAPILA, N, STAGE_CELLS, CONS, true>(p, &tmap, blockIdx.x, p.run0 + (int)blockIdx.y, smem_raw, red_s);
+    stage_tile<SYS_KAPILA, N, STAGE_CELLS, CONS, true>(p, &tmap, blockIdx.x, p.run0 + (int)blockIdx.y, smem_raw);
 }
 
 struct ViscEntry {

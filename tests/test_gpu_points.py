@@ -1,0 +1,73 @@
+"""The tile's point values and its quick admissibility test (csrc/hype_stage_tile.cuh,
+System<SYS>::pad_quick) where they can go wrong, bit for bit against the oracle.
+
+ * Values on both sides of the ranges pad_quick accepts: densities and pressures scaled far
+   out of them, negative pressures, alpha_1 at 0 and 1, gammas and P_inf that quick_eos refuses.
+   Most of these cells take the exact check, some of them the minmod fallback.
+ * Cells that are not finite: their neighbours' results carry the same NaNs.
+ * Strips that leave warps, or all but a few threads of the last warp, without a cell.
+"""
+import numpy as np
+import pytest
+
+import cases
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _same(hp, orc, cfg, U):
+    with hp.Solver(cases.to_pkg(cfg)) as s:
+        R, dt, st = s.rhs_function_prim(0.0, U)
+    Ro, dto, sto = orc.rhs(cfg, U)
+    assert (st != hp.OK) == (sto != 0)
+    if sto != 0:      # the oracle ends at an inadmissible face, its RHS is incomplete
+        return
+    nan = np.isnan(Ro)
+    assert np.array_equal(nan, np.isnan(R))
+    assert R[~nan].tobytes() == Ro[~nan].tobytes()
+    assert dt == dto or (np.isnan(dt) and np.isnan(dto))
+
+
+def _kapila(order, nx, ny, scale_r=1.0, scale_p=1.0, alpha=None, **eos):
+    cfg = O.Config(system=O.KAPILA, order=order, nx=nx, ny=ny, **{**cases.KAPILA_EOS, **eos})
+    r = np.random.default_rng(nx * 131 + ny)
+    a = np.clip(np.where(r.random((ny, nx)) < 0.5, 0.03, 0.97) + 0.02 * r.standard_normal((ny, nx)), 1e-3, 1 - 1e-3)
+    if alpha is not None:
+        a[ny // 2, nx // 3:nx // 2] = alpha
+    r1, r2 = scale_r * 1000 * r.uniform(0.5, 2, (ny, nx)), scale_r * r.uniform(0.5, 2, (ny, nx))
+    p = scale_p * r.uniform(0.1, 1.0, (ny, nx))
+    u, v = r.uniform(-1, 1, (ny, nx)), r.uniform(-1, 1, (ny, nx))
+    g1, g2 = cfg.gamma1 - 1, cfg.gamma2 - 1
+    rho = a * r1 + (1 - a) * r2
+    e = (p * (a * g2 + (1 - a) * g1) + a * cfg.gamma1 * cfg.pi1 * g2 + (1 - a) * cfg.gamma2 * cfg.pi2 * g1) / (g1 * g2)
+    Q = np.stack([a * r1, (1 - a) * r2, rho * u, rho * v, e + 0.5 * rho * (u * u + v * v), a], -1)
+    return cfg, np.ascontiguousarray(Q.reshape(-1))
+
+
+@pytest.mark.parametrize("order", [2, 3])
+@pytest.mark.parametrize("kw", [
+    dict(scale_r=2.0 ** 40, scale_p=2.0 ** 30), dict(scale_r=2.0 ** -45, scale_p=1.0), dict(scale_p=2.0 ** -24, pi1=0.0),
+    dict(scale_p=-1e5), dict(scale_p=1e5, alpha=0.0), dict(scale_p=1e5, alpha=1.0), dict(scale_p=1e5, gamma1=2000.0),
+    dict(scale_p=10.0, pi1=-0.5),
+], ids=["dense", "thin", "low_p", "tension", "alpha0", "alpha1", "gamma", "pi_neg"])
+def test_kapila_out_of_the_quick_range(hp, orc, order, kw):
+    with np.errstate(all="ignore"):
+        _same(hp, orc, *_kapila(order, 41, 23, **kw))
+
+
+@pytest.mark.parametrize("system", ["kapila", "bn", "euler"])
+@pytest.mark.parametrize("value", [np.nan, np.inf, 0.0, -1.0])
+def test_bad_cells(hp, orc, system, value):
+    name = {"kapila": "kapila_37x23_rough_mixed_bc", "bn": "bn_23x19_fixed_p2", "euler": "euler_16x16"}[system]
+    _, cfg, kind, seed = cases.case_by_name(name)
+    U = cases.state(cfg, kind, seed).copy()
+    nv = cases.to_pkg(cfg).nvar
+    U[(cfg.nx * (cfg.ny // 2) + cfg.nx // 2) * nv] = value      # a partial density
+    _same(hp, orc, cfg, U)
+
+
+@pytest.mark.parametrize("nx", [3, 15, 16, 33, 124, 125, 131, 249, 373])
+def test_strip_widths(hp, orc, nx):
+    for order in (1, 2):
+        _same(hp, orc, *_kapila(order, nx, 9, scale_p=1e5))
