@@ -1,5 +1,6 @@
 // hype_div.cuh -- IEEE round-to-nearest-even FP64 division a / b as a straight
-// line of fused multiply-adds, for the bit-exact kernels.
+// line of fused multiply-adds, for the bit-exact kernels: cr_div, and the reciprocal
+// rcp_rn with quotients that share it (div_rn).
 //
 // The compiler's division ends in a branch to its own slow path, which keeps
 // independent divisions from overlapping; this one has no branch, so the WENO
@@ -58,6 +59,43 @@ __device__ __forceinline__ double cr_div(double a, double b, bool &special)
     const bool ok_a = ea >= 1023u - 900u && ea <= 1023u + 1000u && eq >= 1023u - 900u && eq <= 1023u + 1000u;
     special |= !(ok_b && (a == 0.0 || ok_a));
     return (a == 0.0) ? a * copysign(1.0, b) : q;   // a signed zero keeps the IEEE sign
+}
+
+// 1/b correctly rounded, for b normal with |binary exponent| <= 1000 and a significand
+// that is not all ones (rcp_special):
+//   y0 ~ 1/b: the hardware approximation (PTX rcp.approx.ftz.f64, about 20 bits);
+//   y1 = y0 + y0 (e + e^2), e = 1 - b y0 (fma): the third-order iteration for the
+//        reciprocal, |y1 b - 1| below 0.51 ulp's worth, so y1 is one of the two doubles
+//        around 1/b;
+//   y2 = y1 + y1 (1 - b y1), both by fma: rounds (1/b)(1 - e1^2), |e1| <= 2^-53; no midpoint
+//        of two doubles lies between that and 1/b unless b is all ones (Markstein 2000, ch. 8).
+// Five fused multiply-adds, no branch.
+__device__ __forceinline__ double rcp_rn(double b)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    double e = fma(-b, y, 1.0);
+    e = fma(e, e, e);
+    y = fma(y, e, y);
+    e = fma(-b, y, 1.0);
+    return fma(y, e, y);
+}
+// the low words of the divisors of rcp_rn, folded together: all ones in one of them is the
+// only doubtful case (a superset of the all-ones significand, one divisor in 2^32)
+__device__ __forceinline__ unsigned rcp_low(unsigned fold, double b) { return max(fold, (unsigned)__double2loint(b)); }
+__device__ __forceinline__ bool rcp_special(unsigned fold) { return fold == 0xffffffffu; }
+
+// a / b correctly rounded from y = rcp_rn(b): quotients by one divisor share y.  q1 = a y and one
+// correction give a double next to a/b, whose remainder a - b q1 is exact; with y the correctly
+// rounded 1/b the second correction rounds correctly (Markstein 1990, theorem 5).  a, b and a/b
+// nonzero with binary exponents in [-900, 900].
+__device__ __forceinline__ double div_rn(double a, double b, double y)
+{
+    double q = a * y;
+    double r = fma(-b, q, a);
+    q = fma(r, y, q);
+    r = fma(-b, q, a);   // exact
+    return fma(r, y, q);
 }
 
 }  // namespace hype

@@ -543,27 +543,38 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
         for (int kv = 0; kv < NVH; ++kv) {
             const int c = h * NVH + kv;
             if (c >= NV) break;
-            Stencil st;
-            const double *a0 = w_0 + c * BW + ccm;
-            st.c = a0[0];
-            st.xm2 = a0[-2]; st.xm1 = a0[-1]; st.xp1 = a0[1]; st.xp2 = a0[2];
-            st.ym2 = w_m2[c * BW + ccm]; st.ym1 = w_m1[c * BW + ccm]; st.yp1 = w_p1[c * BW + ccm]; st.yp2 = w_p2[c * BW + ccm];
-            st.pp = w_p1[c * BW + ccm + 1]; st.pm = w_m1[c * BW + ccm + 1]; st.mp = w_p1[c * BW + ccm - 1]; st.mm = w_m1[c * BW + ccm - 1];
+            auto stencil = [&] {
+                Stencil st;
+                const double *a0 = w_0 + c * BW + ccm;
+                st.c = a0[0];
+                st.xm2 = a0[-2]; st.xm1 = a0[-1]; st.xp1 = a0[1]; st.xp2 = a0[2];
+                st.ym2 = w_m2[c * BW + ccm]; st.ym1 = w_m1[c * BW + ccm]; st.yp1 = w_p1[c * BW + ccm]; st.yp2 = w_p2[c * BW + ccm];
+                st.pp = w_p1[c * BW + ccm + 1]; st.pm = w_m1[c * BW + ccm + 1]; st.mp = w_p1[c * BW + ccm - 1]; st.mm = w_m1[c * BW + ccm - 1];
+                return st;
+            };
+            auto keep = [&](const double *cf) {
+#pragma unroll
+                for (int k = 1; k < NDOF; ++k) coef_s[cidx(k - 1, c, m)] = cf[k];
+            };
             double cf[NDOF];
             if constexpr (FAST) {
-                ReconFast<N>::run(st, cf);
-            } else if constexpr (SYS == SYS_BN && N == 2) {
-                // branch-free correctly rounded divisions let the weights' chains overlap
-                // (the Baer-Nunziato tile runs 8 warps per SM); the compiler's division
-                // where an operand is outside their range
-                bool special = false;
-                Recon2Cr::run(st, cf, special);
-                if (special && active) Recon<N>::run(st, cf);
+                ReconFast<N>::run(stencil(), cf);
+                keep(cf);
+            } else if constexpr (N == 2) {
+                // branch-free correctly rounded reciprocals and quotients let the weights' chains
+                // overlap; the compiler's division where an operand is outside their range
+                // (from the ring again, so that the stencil is not held for it)
+                bool special;
+                Recon2Cr::run(stencil(), cf, special);
+                keep(cf);
+                if (special && active) {
+                    Recon<N>::run(stencil(), cf);
+                    keep(cf);
+                }
             } else {
-                Recon<N>::run(st, cf);
+                Recon<N>::run(stencil(), cf);
+                keep(cf);
             }
-#pragma unroll
-            for (int k = 1; k < NDOF; ++k) coef_s[cidx(k - 1, c, m)] = cf[k];
         }
         __syncwarp();
 
