@@ -147,6 +147,7 @@ static StageParams base_params(const hype_solver *s)
     p.bc[0] = s->cfg.bc_left; p.bc[1] = s->cfg.bc_right; p.bc[2] = s->cfg.bc_bottom; p.bc[3] = s->cfg.bc_top;
     p.eos.g1 = s->cfg.gamma1; p.eos.g2 = s->cfg.gamma2; p.eos.pi1 = s->cfg.pi1; p.eos.pi2 = s->cfg.pi2;
     p.eos.fix_p2 = (s->cfg.flags & HYPE_FLAG_BN_FIX_P2) ? 1 : 0;
+    p.eos.reciprocals();
     p.eos.derive();
     p.r1_h = s->r1_h;
     p.cfl_h = s->cfl_h;

@@ -259,6 +259,7 @@ static StageParams inst_params(hype_batch *b, const Inst &in, const PlanStage &q
     p.bc[0] = c.bc_left; p.bc[1] = c.bc_right; p.bc[2] = c.bc_bottom; p.bc[3] = c.bc_top;
     p.eos.g1 = c.gamma1; p.eos.g2 = c.gamma2; p.eos.pi1 = c.pi1; p.eos.pi2 = c.pi2;
     p.eos.fix_p2 = (c.flags & HYPE_FLAG_BN_FIX_P2) ? 1 : 0;
+    p.eos.reciprocals();
     p.r1_h = 1. / in.h;
     p.cfl_h = in.cfl_h;
     p.sc = b->dSc + (&in - b->inst.data());
@@ -282,6 +283,7 @@ static MixedParams inst_mparams(hype_batch *b, const Inst &in, const PlanStage &
     p.bc[0] = c.bc_left; p.bc[1] = c.bc_right; p.bc[2] = c.bc_bottom; p.bc[3] = c.bc_top;
     p.eos.g1 = c.gamma1; p.eos.g2 = c.gamma2; p.eos.pi1 = c.pi1; p.eos.pi2 = c.pi2;
     p.eos.fix_p2 = (c.flags & HYPE_FLAG_BN_FIX_P2) ? 1 : 0;
+    p.eos.reciprocals();
     p.r1_h = 1. / in.h; p.cfl_h = in.cfl_h;
     p.in_f = in.mf[q.in]; p.in_d = in.md[q.in];
     if (q.x >= 0) { p.xn_f = in.mf[q.x]; p.xn_d = in.md[q.x]; }

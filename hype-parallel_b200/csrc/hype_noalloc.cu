@@ -141,6 +141,7 @@ extern "C" HYPE_API int hype_rhs_prim_noalloc(const hype_config *cfg, double t, 
     p.bc[0] = cfg->bc_left; p.bc[1] = cfg->bc_right; p.bc[2] = cfg->bc_bottom; p.bc[3] = cfg->bc_top;
     p.eos.g1 = cfg->gamma1; p.eos.g2 = cfg->gamma2; p.eos.pi1 = cfg->pi1; p.eos.pi2 = cfg->pi2;
     p.eos.fix_p2 = (cfg->flags & HYPE_FLAG_BN_FIX_P2) ? 1 : 0;
+    p.eos.reciprocals();
     const double h = (cfg->x_max - cfg->x_min) / (double)cfg->nx;   // hype.c:57
     p.r1_h = 1. / h;
     p.cfl_h = cfg->cfl * h;

@@ -28,6 +28,16 @@ enum : unsigned { ERR_INADMISSIBLE_FACE = 1u, ERR_NONFINITE = 2u, ERR_TMA_TIMEOU
 struct EosBase {
     double g1, g2, pi1, pi2;
     int fix_p2;   // Baer-Nunziato: 0 = flux pressure of phase 2 read from V[8] as baer_nunziato.c:271 does
+    int cr;       // 1: the constants are within CrDiv's range
+    double r_g12, r_g1, r_g2;   // the correctly rounded reciprocals of (g1 - 1)(g2 - 1), g1 - 1, g2 - 1
+    __host__ __device__ void reciprocals()
+    {
+        r_g12 = 1.0 / ((g1 - 1.0) * (g2 - 1.0));
+        r_g1 = 1.0 / (g1 - 1.0);
+        r_g2 = 1.0 / (g2 - 1.0);
+        cr = g1 >= 1.0 + 0x1p-20 && g1 <= 1024.0 && g2 >= 1.0 + 0x1p-20 && g2 <= 1024.0 && pi1 >= 0.0 && pi1 <= 0x1p100 &&
+             pi2 >= 0.0 && pi2 <= 0x1p100;
+    }
 };
 struct Eos : EosBase {
     // constants the FP64 performance form (hype_physics_fast.cuh) reads instead of
@@ -150,10 +160,40 @@ template <int N, int Q> struct DPhiVolY { template <int K> static constexpr doub
 template <int LO, int HI>
 __device__ __forceinline__ bool exp_in(double x)
 {
-    return (unsigned)__double2hiint(x) - ((1023u + LO) << 20) < ((unsigned)(HI - LO) << 20);
+    return (unsigned)__double2hiint(x) - ((unsigned)(1023 + LO) << 20) < ((unsigned)(HI - LO) << 20);
 }
 // x in [0, 1)
 __device__ __forceinline__ bool frac_in(double x) { return (unsigned)__double2hiint(x) < 0x3ff00000u; }
+
+// How a system's functions divide.  IeeeDiv: the compiler's division.  CrDiv: the
+// branch-free correctly rounded forms of hype_div.cuh, whose chains interleave; the values
+// named to pos() and frac() bound every operand, and where one is outside (or a divisor's low
+// word is all ones) special() holds and the caller repeats the function with IeeeDiv.
+struct IeeeDiv {
+    __device__ __forceinline__ double operator()(double a, double b) const { return a / b; }
+    __device__ __forceinline__ double by_const(double a, double b, double) const { return a / b; }   // third: 1/b, correctly rounded
+    __device__ __forceinline__ double rcp(double) const { return 0.0; }
+    __device__ __forceinline__ double quot(double a, double b, double) const { return a / b; }       // third: rcp(b)
+    __device__ __forceinline__ void pos(double) const {}
+    __device__ __forceinline__ void frac(double) const {}
+    __device__ __forceinline__ void num(double) const {}
+};
+struct CrDiv {
+    unsigned lo = 0;
+    bool in = true;
+    __device__ __forceinline__ double operator()(double a, double b) { return div_rn(a, b, rcp(b)); }
+    __device__ __forceinline__ double by_const(double a, double b, double rb) const { return div_rn(a, b, rb); }
+    __device__ __forceinline__ double rcp(double b) { lo = rcp_low(lo, b); return rcp_rn(b); }
+    __device__ __forceinline__ double quot(double a, double b, double y) const { return div_rn(a, b, y); }
+    __device__ __forceinline__ void pos(double x) { in = in && exp_in<-100, 100>(x); }    // a density, a p + P_inf
+    __device__ __forceinline__ void frac(double x) { in = in && exp_in<-100, 0>(x); }     // a volume fraction
+    __device__ __forceinline__ void num(double x)                                          // a numerator of any sign: 0 or |x| >= 2^-300
+    {
+        const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+        in = in && (h - ((1023u - 300u) << 20) < (500u << 20) || (h | (unsigned)__double2loint(x)) == 0u);
+    }
+    __device__ __forceinline__ bool special() const { return !in || rcp_special(lo); }
+};
 
 // ---------------------------------------------------------------------------
 // PDE systems (primitive-variable path)
@@ -197,7 +237,8 @@ template <> struct System<SYS_KAPILA> {
         cons2prim_dv(e, Q, V, [](double a, double b) { return a / b; });
     }
     // kapila_5eqn.c:41-61
-    __device__ __forceinline__ static void prim2cons(const EosBase &e, const double *V, double *Q)
+    template <class Dv>
+    __device__ __forceinline__ static void prim2cons(const EosBase &e, Dv &dv, const double *V, double *Q)
     {
         double alpha_1 = V[5];
         double alpha_2 = 1.0 - alpha_1;
@@ -205,7 +246,7 @@ template <> struct System<SYS_KAPILA> {
         double u = V[2], v = V[3], p = V[4];
         double G1m1 = e.g1 - 1.0;
         double G2m1 = e.g2 - 1.0;
-        double ei = (p * (alpha_1 * G2m1 + alpha_2 * G1m1) + alpha_1 * e.g1 * e.pi1 * G2m1 + alpha_2 * e.g2 * e.pi2 * G1m1) / (G1m1 * G2m1);
+        double ei = dv.by_const(p * (alpha_1 * G2m1 + alpha_2 * G1m1) + alpha_1 * e.g1 * e.pi1 * G2m1 + alpha_2 * e.g2 * e.pi2 * G1m1, G1m1 * G2m1, e.r_g12);
         double E = ei + 0.5 * rho * (u * u + v * v);
         Q[0] = alpha_1 * V[0];
         Q[1] = alpha_2 * V[1];
@@ -215,8 +256,8 @@ template <> struct System<SYS_KAPILA> {
         Q[5] = alpha_1;
     }
     // kapila_5eqn.c:326-371
-    template <int DIR>
-    __device__ __forceinline__ static double flux(const EosBase &e, const double *V, double *F, bool &bad)
+    template <int DIR, class Dv>
+    __device__ __forceinline__ static double flux(const EosBase &e, Dv &dv, const double *V, double *F, bool &bad)
     {
         constexpr double nx = DIR == 0 ? 1.0 : 0.0, ny = DIR == 0 ? 0.0 : 1.0;
         double alpha_1 = V[5];
@@ -226,12 +267,13 @@ template <> struct System<SYS_KAPILA> {
         double u = V[2], v = V[3], p = V[4];
         double G1m1 = e.g1 - 1.0;
         double G2m1 = e.g2 - 1.0;
-        double ei = (p * (alpha_1 * G2m1 + alpha_2 * G1m1) + alpha_1 * e.g1 * e.pi1 * G2m1 + alpha_2 * e.g2 * e.pi2 * G1m1) / (G1m1 * G2m1);
+        double ei = dv.by_const(p * (alpha_1 * G2m1 + alpha_2 * G1m1) + alpha_1 * e.g1 * e.pi1 * G2m1 + alpha_2 * e.g2 * e.pi2 * G1m1, G1m1 * G2m1, e.r_g12);
         double E = ei + 0.5 * rho * (u * u + v * v);
         double un = u * nx + v * ny;
-        double a1_sq = e.g1 * (p + e.pi1) / rho_1;
-        double a2_sq = e.g2 * (p + e.pi2) / rho_2;
-        double a_sq = (rho_1 * a1_sq * rho_2 * a2_sq) / (rho * (alpha_2 * rho_1 * a1_sq + alpha_1 * rho_2 * a2_sq));
+        dv.pos(rho_1); dv.pos(rho_2); dv.pos(p + e.pi1); dv.pos(p + e.pi2); dv.frac(alpha_1);
+        double a1_sq = dv(e.g1 * (p + e.pi1), rho_1);
+        double a2_sq = dv(e.g2 * (p + e.pi2), rho_2);
+        double a_sq = dv(rho_1 * a1_sq * rho_2 * a2_sq, rho * (alpha_2 * rho_1 * a1_sq + alpha_1 * rho_2 * a2_sq));
         bad |= (a_sq < PRS_FLOOR);
         F[0] = alpha_1 * rho_1 * un;
         F[1] = alpha_2 * rho_2 * un;
@@ -242,16 +284,18 @@ template <> struct System<SYS_KAPILA> {
         return fabs(un) + sqrt(a_sq);
     }
     // kapila_5eqn.c:417-444
-    __device__ __forceinline__ static void ncp(const EosBase &e, const double *V, const double *gx, const double *gy, double *B)
+    template <class Dv>
+    __device__ __forceinline__ static void ncp(const EosBase &e, Dv &dv, const double *V, const double *gx, const double *gy, double *B)
     {
         double alpha_1 = V[5];
         double alpha_2 = 1.0 - alpha_1;
         double rho_1 = V[0], rho_2 = V[1], u = V[2], v = V[3], p = V[4];
         double phi_x = gx[5], phi_y = gy[5];
         double u_x = gx[2], v_y = gy[3];
-        double a_1_sq = e.g1 * (p + e.pi1) / rho_1;
-        double a_2_sq = e.g2 * (p + e.pi2) / rho_2;
-        double K = (alpha_1 * alpha_2 * (rho_2 * a_2_sq - rho_1 * a_1_sq)) / (alpha_1 * rho_2 * a_2_sq + alpha_2 * rho_1 * a_1_sq);
+        dv.pos(rho_1); dv.pos(rho_2); dv.pos(p + e.pi1); dv.pos(p + e.pi2); dv.frac(alpha_1);
+        double a_1_sq = dv(e.g1 * (p + e.pi1), rho_1);
+        double a_2_sq = dv(e.g2 * (p + e.pi2), rho_2);
+        double K = dv(alpha_1 * alpha_2 * (rho_2 * a_2_sq - rho_1 * a_1_sq), alpha_1 * rho_2 * a_2_sq + alpha_2 * rho_1 * a_1_sq);
         B[0] = 0.0; B[1] = 0.0; B[2] = 0.0; B[3] = 0.0; B[4] = 0.0;
         B[5] = u * phi_x + v * phi_y - K * (u_x + v_y);
     }
@@ -456,21 +500,22 @@ template <> struct System<SYS_BN> {
         V[8] = phi_1;
     }
     // baer_nunziato.c:47-60
-    __device__ __forceinline__ static void prim2cons(const EosBase &e, const double *V, double *Q)
+    template <class Dv>
+    __device__ __forceinline__ static void prim2cons(const EosBase &e, Dv &dv, const double *V, double *Q)
     {
         Q[0] = V[8] * V[0];
         Q[1] = Q[0] * V[1];
         Q[2] = Q[0] * V[2];
-        Q[3] = Q[0] * (0.5 * (V[1] * V[1] + V[2] * V[2]) + (V[3] + e.g1 * e.pi1) / (V[0] * (e.g1 - 1.0)));
+        Q[3] = Q[0] * (0.5 * (V[1] * V[1] + V[2] * V[2]) + dv(V[3] + e.g1 * e.pi1, V[0] * (e.g1 - 1.0)));
         Q[4] = (1.0 - V[8]) * V[4];
         Q[5] = Q[4] * V[5];
         Q[6] = Q[4] * V[6];
-        Q[7] = Q[4] * (0.5 * (V[5] * V[5] + V[6] * V[6]) + (V[7] + e.g2 * e.pi2) / (V[4] * (e.g2 - 1.0)));
+        Q[7] = Q[4] * (0.5 * (V[5] * V[5] + V[6] * V[6]) + dv(V[7] + e.g2 * e.pi2, V[4] * (e.g2 - 1.0)));
         Q[8] = V[8];
     }
     // baer_nunziato.c:256-321 (phase-2 flux pressure from V[8] unless fix_p2)
-    template <int DIR>
-    __device__ __forceinline__ static double flux(const EosBase &e, const double *V, double *F, bool &bad)
+    template <int DIR, class Dv>
+    __device__ __forceinline__ static double flux(const EosBase &e, Dv &dv, const double *V, double *F, bool &bad)
     {
         constexpr double nx = DIR == 0 ? 1.0 : 0.0, ny = DIR == 0 ? 0.0 : 1.0;
         double phi_1 = V[8];
@@ -480,8 +525,9 @@ template <> struct System<SYS_BN> {
         double u_2 = V[5], v_2 = V[6];
         double p_1 = V[3];
         double p_2 = e.fix_p2 ? V[7] : V[8];
-        double E_1 = (p_1 + e.g1 * e.pi1) / (e.g1 - 1.0) + 0.5 * rho_1 * (u_1 * u_1 + v_1 * v_1);
-        double E_2 = (p_2 + e.g2 * e.pi2) / (e.g2 - 1.0) + 0.5 * rho_2 * (u_2 * u_2 + v_2 * v_2);
+        dv.pos(rho_1); dv.pos(rho_2); dv.pos(p_1 + e.pi1); dv.pos(p_2 + e.pi2); dv.pos(V[7] + e.g2 * e.pi2);
+        double E_1 = dv.by_const(p_1 + e.g1 * e.pi1, e.g1 - 1.0, e.r_g1) + 0.5 * rho_1 * (u_1 * u_1 + v_1 * v_1);
+        double E_2 = dv.by_const(p_2 + e.g2 * e.pi2, e.g2 - 1.0, e.r_g2) + 0.5 * rho_2 * (u_2 * u_2 + v_2 * v_2);
         double un_1 = nx * u_1 + ny * v_1;
         double un_2 = nx * u_2 + ny * v_2;
         bad |= (rho_1 < RHO_FLOOR) | (rho_2 < RHO_FLOOR) | ((p_1 + e.pi1) < PRS_FLOOR) | ((p_2 + e.pi2) < PRS_FLOOR);
@@ -494,12 +540,13 @@ template <> struct System<SYS_BN> {
         F[6] = phi_2 * (rho_2 * v_2 * un_2 + ny * p_2);
         F[7] = phi_2 * un_2 * (E_2 + p_2);
         F[8] = 0.0;
-        double s_1 = fabs(un_1) + sqrt(e.g1 * (p_1 + e.pi1) / rho_1);
-        double s_2 = fabs(un_2) + sqrt(e.g2 * (p_2 + e.pi2) / rho_2);
+        double s_1 = fabs(un_1) + sqrt(dv(e.g1 * (p_1 + e.pi1), rho_1));
+        double s_2 = fabs(un_2) + sqrt(dv(e.g2 * (p_2 + e.pi2), rho_2));
         return (s_1 < s_2) ? s_2 : s_1;
     }
     // baer_nunziato.c:327-344
-    __device__ __forceinline__ static void ncp(const EosBase &, const double *V, const double *gx, const double *gy, double *B)
+    template <class Dv>
+    __device__ __forceinline__ static void ncp(const EosBase &, Dv &, const double *V, const double *gx, const double *gy, double *B)
     {
         double u_I = V[1], v_I = V[2];
         double p_I = V[7];
@@ -628,9 +675,10 @@ template <> struct System<SYS_EULER> {
         V[3] = (e.g1 - 1.0) * (Q[3] - 0.5 * irho * (Q[1] * Q[1] + Q[2] * Q[2]));
     }
     // euler.c:29-38
-    __device__ __forceinline__ static void prim2cons(const EosBase &e, const double *V, double *Q)
+    template <class Dv>
+    __device__ __forceinline__ static void prim2cons(const EosBase &e, Dv &dv, const double *V, double *Q)
     {
-        double ei = (V[3]) / (e.g1 - 1.0);
+        double ei = dv.by_const(V[3], e.g1 - 1.0, e.r_g1);
         double k = 0.5 * V[0] * (V[1] * V[1] + V[2] * V[2]);
         Q[0] = V[0];
         Q[1] = V[0] * V[1];
@@ -638,24 +686,26 @@ template <> struct System<SYS_EULER> {
         Q[3] = k + ei;
     }
     // euler.c:197-236
-    template <int DIR>
-    __device__ __forceinline__ static double flux(const EosBase &e, const double *V, double *F, bool &bad)
+    template <int DIR, class Dv>
+    __device__ __forceinline__ static double flux(const EosBase &e, Dv &dv, const double *V, double *F, bool &bad)
     {
         constexpr double nx = DIR == 0 ? 1.0 : 0.0, ny = DIR == 0 ? 0.0 : 1.0;
         double rho = V[0], u = V[1], v = V[2];
         double un = nx * u + ny * v;
         double rhoun = rho * un;
         double p = V[3];
-        double E = p / (e.g1 - 1.0) + 0.5 * rho * (u * u + v * v);
+        dv.pos(rho); dv.pos(p);
+        double E = dv.by_const(p, e.g1 - 1.0, e.r_g1) + 0.5 * rho * (u * u + v * v);
         bad |= (rho < RHO_FLOOR) | (p < PRS_FLOOR);
         F[0] = rhoun;
         F[1] = rhoun * u + nx * p;
         F[2] = rhoun * v + ny * p;
         F[3] = un * (E + p);
-        return fabs(un) + sqrt(e.g1 * p / rho);
+        return fabs(un) + sqrt(dv(e.g1 * p, rho));
     }
     // euler.c:278-286
-    __device__ __forceinline__ static void ncp(const EosBase &, const double *, const double *, const double *, double *B)
+    template <class Dv>
+    __device__ __forceinline__ static void ncp(const EosBase &, Dv &, const double *, const double *, const double *, double *B)
     {
         B[0] = 0.0; B[1] = 0.0; B[2] = 0.0; B[3] = 0.0;
     }

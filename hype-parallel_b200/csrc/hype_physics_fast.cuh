@@ -61,7 +61,7 @@ template <> struct FastSystem<SYS_KAPILA> : System<SYS_KAPILA> {
         V[5] = a1;
     }
     // kapila_5eqn.c:41-61
-    __device__ __forceinline__ static void prim2cons(const Eos &e, const double *V, double *Q)
+    __device__ __forceinline__ static void prim2cons(const Eos &e, IeeeDiv &, const double *V, double *Q)
     {
         const double a1 = V[5], a2 = 1.0 - a1;
         const double rho = a1 * V[0] + a2 * V[1];
@@ -75,8 +75,8 @@ template <> struct FastSystem<SYS_KAPILA> : System<SYS_KAPILA> {
         Q[5] = a1;
     }
     // kapila_5eqn.c:326-371
-    template <int DIR>
-    __device__ __forceinline__ static double flux(const Eos &e, const double *V, double *F, bool &bad)
+    template <int DIR, class Dv>
+    __device__ __forceinline__ static double flux(const Eos &e, Dv &, const double *V, double *F, bool &bad)
     {
         const double a1 = V[5], a2 = 1.0 - a1;
         const double r1 = V[0], r2 = V[1];
@@ -97,7 +97,7 @@ template <> struct FastSystem<SYS_KAPILA> : System<SYS_KAPILA> {
         return fabs(un) + sqrt(a_sq);
     }
     // kapila_5eqn.c:417-444
-    __device__ __forceinline__ static void ncp(const Eos &e, const double *V, const double *gx, const double *gy, double *B)
+    __device__ __forceinline__ static void ncp(const Eos &e, IeeeDiv &, const double *V, const double *gx, const double *gy, double *B)
     {
         const double a1 = V[5], a2 = 1.0 - a1;
         const double p = V[4];
@@ -140,7 +140,7 @@ template <> struct FastSystem<SYS_BN> : System<SYS_BN> {
         V[8] = phi_1;
     }
     // baer_nunziato.c:47-60
-    __device__ __forceinline__ static void prim2cons(const Eos &e, const double *V, double *Q)
+    __device__ __forceinline__ static void prim2cons(const Eos &e, IeeeDiv &, const double *V, double *Q)
     {
         Q[0] = V[8] * V[0];
         Q[1] = Q[0] * V[1];
@@ -153,8 +153,8 @@ template <> struct FastSystem<SYS_BN> : System<SYS_BN> {
         Q[8] = V[8];
     }
     // baer_nunziato.c:256-321 (phase-2 flux pressure from V[8] unless fix_p2)
-    template <int DIR>
-    __device__ __forceinline__ static double flux(const Eos &e, const double *V, double *F, bool &bad)
+    template <int DIR, class Dv>
+    __device__ __forceinline__ static double flux(const Eos &e, Dv &, const double *V, double *F, bool &bad)
     {
         const double phi_1 = V[8], phi_2 = 1.0 - V[8];
         const double rho_1 = V[0], rho_2 = V[4];
@@ -193,7 +193,7 @@ template <> struct FastSystem<SYS_EULER> : System<SYS_EULER> {
         V[3] = e.g1m1 * (Q[3] - 0.5 * irho * (Q[1] * Q[1] + Q[2] * Q[2]));
     }
     // euler.c:29-38
-    __device__ __forceinline__ static void prim2cons(const Eos &e, const double *V, double *Q)
+    __device__ __forceinline__ static void prim2cons(const Eos &e, IeeeDiv &, const double *V, double *Q)
     {
         Q[0] = V[0];
         Q[1] = V[0] * V[1];
@@ -201,8 +201,8 @@ template <> struct FastSystem<SYS_EULER> : System<SYS_EULER> {
         Q[3] = 0.5 * V[0] * (V[1] * V[1] + V[2] * V[2]) + V[3] * e.inv_g1m1;
     }
     // euler.c:197-236
-    template <int DIR>
-    __device__ __forceinline__ static double flux(const Eos &e, const double *V, double *F, bool &bad)
+    template <int DIR, class Dv>
+    __device__ __forceinline__ static double flux(const Eos &e, Dv &, const double *V, double *F, bool &bad)
     {
         const double rho = V[0], u = V[1], v = V[2], p = V[3];
         const double un = DIR == 0 ? u : v;

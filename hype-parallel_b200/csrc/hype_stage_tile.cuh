@@ -230,11 +230,38 @@ __device__ __forceinline__ double face_grad(const double *uc, int q)
     return v;
 }
 
-// one face Gauss point with n = e_x (DIR 0) or e_y (DIR 1): riemann.c:112-140
-// (RiemannSolverPrim, VL/VR primitive) or, for the conservative path,
-// riemann.c:52-105 (RiemannSolver, VL/VR conserved); S is the system's physics
-// (System<SYS>, or FastSystem<SYS> for the FP64 performance form)
-template <class S, int DIR, bool CONS, class E>
+// riemann.c:112-140 (RiemannSolverPrim) at one face Gauss point, n = e_x (DIR 0) or e_y
+// (DIR 1), dividing by dv; S is the system's physics (System<SYS>, or FastSystem<SYS> for the
+// FP64 performance form)
+template <class S, int DIR, class E, class Dv>
+__device__ __forceinline__ double riemann_prim(const E &eos, Dv &dv, const double *VL, const double *VR, double *F, double *D, bool &bad)
+{
+    constexpr int NV = S::NV;
+    constexpr double nx = DIR == 0 ? 1.0 : 0.0, ny = DIR == 0 ? 0.0 : 1.0;
+    double QL[NV], QR[NV], FL[NV], FR[NV];
+    S::prim2cons(eos, dv, VL, QL);
+    S::prim2cons(eos, dv, VR, QR);
+    const double sl = S::template flux<DIR>(eos, dv, VL, FL, bad);
+    const double sr = S::template flux<DIR>(eos, dv, VR, FR, bad);
+    const double s = (sl < sr) ? sr : sl;
+    double Vav[NV], gx[NV], gy[NV];
+#pragma unroll
+    for (int c = 0; c < NV; ++c) {
+        Vav[c] = 0.5 * (VR[c] + VL[c]);
+        gx[c] = nx * (VR[c] - VL[c]);
+        gy[c] = ny * (VR[c] - VL[c]);
+        F[c] = 0.5 * (FR[c] + FL[c] - s * (QR[c] - QL[c]));
+    }
+    S::ncp(eos, dv, Vav, gx, gy, D);
+    return s;
+}
+
+// one face Gauss point: RiemannSolverPrim (VL/VR primitive) or, for the conservative path,
+// riemann.c:52-105 (RiemannSolver, VL/VR conserved).  CR: the branch-free divisions, and the
+// compiler's for the few points outside their range.  Measured: BN 1024^2 right-hand side
+// 0.780 -> 0.736 ms, Kapila N = 3 500^2 0.256 -> 0.246, Kapila N = 2 64^2 113.7 -> 110.2 us,
+// 2048^2 and Euler even
+template <class S, int DIR, bool CONS, bool CR, class E>
 __device__ __forceinline__ double riemann_gp(const E &eos, const double *VL, const double *VR, double *F, double *D, bool &bad)
 {
     constexpr int NV = S::NV;
@@ -255,22 +282,17 @@ __device__ __forceinline__ double riemann_gp(const E &eos, const double *VL, con
         S::ncp_cons(eos, Qav, gx, gy, D);
         return s;
     }
-    double QL[NV], QR[NV], FL[NV], FR[NV];
-    S::prim2cons(eos, VL, QL);
-    S::prim2cons(eos, VR, QR);
-    const double sl = S::template flux<DIR>(eos, VL, FL, bad);
-    const double sr = S::template flux<DIR>(eos, VR, FR, bad);
-    const double s = (sl < sr) ? sr : sl;
-    double Vav[NV], gx[NV], gy[NV];
-#pragma unroll
-    for (int c = 0; c < NV; ++c) {
-        Vav[c] = 0.5 * (VR[c] + VL[c]);
-        gx[c] = nx * (VR[c] - VL[c]);
-        gy[c] = ny * (VR[c] - VL[c]);
-        F[c] = 0.5 * (FR[c] + FL[c] - s * (QR[c] - QL[c]));
+    if constexpr (CR) {
+        CrDiv dv;
+        bool b = false;
+        const double s = riemann_prim<S, DIR>(eos, dv, VL, VR, F, D, b);
+        if (eos.cr && !dv.special()) {
+            bad |= b;
+            return s;
+        }
     }
-    S::ncp(eos, Vav, gx, gy, D);
-    return s;
+    IeeeDiv dv;
+    return riemann_prim<S, DIR>(eos, dv, VL, VR, F, D, bad);
 }
 
 // One tile of one grid: columns of strip `strip` (of p.strips) and rows of run
@@ -384,7 +406,7 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
                 const double v = own(jj, Vq), vo = __shfl_xor_sync(FULL, other(jj, Vq), 1);
                 return (((0.0 + (h ? fo : f)) + (h ? vo : v)) + (h ? f : fo)) + (h ? v : vo);
             } else {
-                return (0.0 + f) + fo;
+                return f + fo;   // (0.0 + f) + fo but for a zero's sign, which the right-hand side's own sums lose
             }
         } else {
             if constexpr (VISC) return (0.0 + own(jj, Fq)) + own(jj, Vq);
@@ -394,7 +416,7 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
     auto fluct_sum = [&](auto jj, const double *Dq) {
         if constexpr (NFGP > 1) {
             const double d = own(jj, Dq), d_o = __shfl_xor_sync(FULL, other(jj, Dq), 1);
-            return (0.0 + d) + d_o;
+            return d + d_o;
         } else {
             return 0.0 + own(jj, Dq);
         }
@@ -589,7 +611,7 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
         bool ok = quick_eos;                        // every node in the plainly admissible range
         // the point values from the coefficients that coef(c, cf) gives
         auto points = [&](auto coef) {
-            double Vv[QH][NV], gx[QH][NV], gy[QH][NV];
+            [[maybe_unused]] double Vv[QH][NV], gx[QH][NV], gy[QH][NV];
             static_for<NV>([&](auto sc_) {
                 constexpr int c = S::order(decltype(sc_)::value);   // the product's velocity part first: fewer values wait for it
                 double cf[NDOF];
@@ -619,7 +641,10 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
                     constexpr int a = decltype(sa)::value;
                     double B[NV];
                     if constexpr (CONS) S::ncp_cons(eos, Vv[a], gx[a], gy[a], B);
-                    else S::ncp(eos, Vv[a], gx[a], gy[a], B);
+                    else {
+                        IeeeDiv dv;   // the branch-free divisions measured slower here (2048^2 +0.6 %: registers)
+                        S::ncp(eos, dv, Vv[a], gx[a], gy[a], B);
+                    }
 #pragma unroll
                     for (int c = 0; c < NV; ++c) tq[a][c] = -QD::wv(0) * B[c];
                 });
@@ -662,7 +687,7 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
         __syncwarp();
 
         // ---------------- C. volume non-conservative term: the pair's sum
-        double vol[(NV + 1) / 2];   // of components 2 j + h; kept once row r-1 has read its own
+        double vol[(NV + 1) / 2] = {};   // of components 2 j + h; kept once row r-1 has read its own
         if constexpr (NZ > 0) {
             // rhs = 0.0; rhs += -w_q B_q for q = 0..NVGP-1; the pair holds q = 2h, 2h+1
             static_for<(NV + 1) / 2>([&](auto jj) {
@@ -695,7 +720,7 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
                 double VL[NV];
 #pragma unroll
                 for (int c = 0; c < NV; ++c) VL[c] = yt_lo[c * CELLS];
-                const double s = riemann_gp<S, 1, CONS>(eos, VL, VR, Fq, Dq, bad);
+                const double s = riemann_gp<S, 1, CONS, !FAST>(eos, VL, VR, Fq, Dq, bad);
                 smax_loc = fmax(smax_loc, s);
 #pragma unroll
                 for (int c = 0; c < NV; ++c) { Fq[c] = QD::wf(0) * Fq[c]; Dq[c] = QD::wf(0) * Dq[c]; }
@@ -836,7 +861,7 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
                     VL[c] = coef_s[cidx(2 * q + 1, c, m - 1)];
                     VR[c] = coef_s[cidx(2 * q, c, m)];
                 }
-                const double s = riemann_gp<S, 0, CONS>(eos, VL, VR, Fq, Dq, bad);
+                const double s = riemann_gp<S, 0, CONS, !FAST>(eos, VL, VR, Fq, Dq, bad);
                 smax_loc = fmax(smax_loc, s);
 #pragma unroll
                 for (int c = 0; c < NV; ++c) { Fq[c] = QD::wf(0) * Fq[c]; Dq[c] = QD::wf(0) * Dq[c]; }

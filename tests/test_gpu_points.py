@@ -71,3 +71,16 @@ def test_bad_cells(hp, orc, system, value):
 def test_strip_widths(hp, orc, nx):
     for order in (1, 2):
         _same(hp, orc, *_kapila(order, nx, 9, scale_p=1e5))
+
+
+@pytest.mark.parametrize("name", ["bn_23x19_fixed_p2", "bn_13x21_periodic_N1", "bn_12x10_N3", "euler_21x19_reflective_N1", "euler_16x16"])
+@pytest.mark.parametrize("scale", [2.0 ** -60, 2.0 ** 60, 2.0 ** -170, 2.0 ** 170])
+def test_scaled_units(hp, orc, name, scale):
+    """Densities, momenta and energies in other units: past 2^100 or below 2^-100 the Riemann
+    solver's branch-free divisions hand over to the compiler's."""
+    _, cfg, kind, seed = cases.case_by_name(name)
+    U = cases.state(cfg, kind, seed).reshape(-1, cases.to_pkg(cfg).nvar).copy()
+    k = 8 if U.shape[1] == 9 else U.shape[1]
+    U[:, :k] *= scale
+    cfg.pi1, cfg.pi2 = cfg.pi1 * scale, cfg.pi2 * scale
+    _same(hp, orc, cfg, U.reshape(-1))
