@@ -40,7 +40,9 @@
 // (3.8 k FP64 instructions a cell instead of 5.0 k) and the call takes 1.76 ms instead of
 // 2.09; Euler 1531x897 0.380 ms instead of 0.417, BN 1024^2 0.896 instead of 0.947.
 //
-// Two block barriers a row: after the first, the neighbours' face values are
+// Two block barriers a row (where the fluxes share the coefficients' memory, also a count
+// of the warps that have read their neighbours', which a warp waits for before its first
+// coefficient replaces them): after the first, the neighbours' face values are
 // there, and row r+3 (loaded in the previous iteration) is converted beside
 // the x-face problems; the second makes the x fluxes and that row visible.
 //
@@ -109,21 +111,30 @@ struct StageKernel {
     static constexpr int NZ = count_nz();
     // per-cell arrays, [k][c][cell] so consecutive cells hit consecutive banks.  Coefficients
     // k >= 1; later, by slot, the left and right face values at each Gauss point (2 q, 2 q + 1)
-    // and the x-face fluxes (slot 0) and fluctuations (slot 2)
+    // and, without FX_OWN, the x-face fluxes (slot 0) and fluctuations (slot 2)
     static constexpr int COEF_ELEMS = (NC > 3 ? NC : 3) * NV * CELLS;
     static constexpr int YT_ELEMS = 2 * QD::NFGP * NV * CELLS;                 // top-face values of rows r-1 and r, by Gauss point
     static constexpr int CARRY_ELEMS = (2 * NV + 2 * NZ) * CELLS;              // t1, G below; ncp, E below
     // the ring, the per-cell arrays and one more row slot: the conserved input of the row
     // being finished (row r-1), for the RK combination
-    static constexpr size_t SMEM = (size_t)(SLOTS + 1) * SLOT_STRIDE * 8 + (size_t)(COEF_ELEMS + YT_ELEMS + CARRY_ELEMS) * 8 +
-                                   64 /* barriers */;
-    static_assert((SLOTS + 1) * 8 <= 64, "the barriers fit their space");
-    // blocks the 228 KB of an SM's shared memory holds (1 KB reserved per block); the
-    // launch bound asks for no more than that, so no register limit is paid for blocks
-    // that could not be resident anyway (Kapila N = 3 at 128-column tiles: 1)
-    static constexpr int SMEM_FIT = (int)(233472 / (SMEM + 1024));
+    static constexpr size_t SMEM_BASE = (size_t)(SLOTS + 1) * SLOT_STRIDE * 8 +
+                                        (size_t)(COEF_ELEMS + YT_ELEMS + CARRY_ELEMS) * 8 + 64 /* barriers */;
+    // blocks the 228 KB of an SM's shared memory holds (1 KB reserved per block, and the
+    // persistent form's 256 bytes); the launch bound asks for no more than that, so no register
+    // limit is paid for blocks that could not be resident anyway (Kapila N = 3 at 128-column
+    // tiles: 1)
     static constexpr int REG_TARGET = (NV <= 6 ? 2 : 1) * (128 / CELLS);
-    static constexpr int MIN_BLOCKS = SMEM_FIT < 1 ? 1 : (SMEM_FIT < REG_TARGET ? SMEM_FIT : REG_TARGET);
+    static constexpr int fit(size_t smem) { return (int)(233472 / (smem + 1024 + 256)); }
+    static constexpr int blocks(size_t smem) { return fit(smem) < 1 ? 1 : (fit(smem) < REG_TARGET ? fit(smem) : REG_TARGET); }
+    // x-face fluxes and fluctuations, exchanged with the neighbours: an array of their own where
+    // that costs no resident block, else coefficient slots, whose reuse has to be waited for (the
+    // wait measured 3 % in the Baer-Nunziato and N = 3 tiles, nothing in Kapila N = 2)
+    static constexpr int FX_ELEMS = (NV + NZ) * CELLS;
+    static constexpr size_t SMEM_MOST = 232448 - 512;   // of one block
+    static constexpr bool FX_OWN = SMEM_BASE + FX_ELEMS * 8 <= SMEM_MOST && blocks(SMEM_BASE + FX_ELEMS * 8) == blocks(SMEM_BASE);
+    static constexpr size_t SMEM = SMEM_BASE + (FX_OWN ? FX_ELEMS * 8 : 0);
+    static constexpr int MIN_BLOCKS = blocks(SMEM);
+    static_assert((SLOTS + 2) * 8 <= 64, "the barriers fit their space");
     static constexpr size_t smem_bytes() { return SMEM; }
 };
 
@@ -330,11 +341,15 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
     double *yt_s = coef_s + K::COEF_ELEMS;                      // [row parity][q][c][cell]
     double *carry_s = yt_s + K::YT_ELEMS;                       // t1, G below [c][cell]; ncp, E below [z][cell]
     uint64_t *bars = reinterpret_cast<uint64_t *>(carry_s + K::CARRY_ELEMS);
+    // one arrival per warp and row, once it has read its neighbours' x-face fluxes: the next row's
+    // coefficients may replace them
+    uint64_t *fluxes_read = bars + SLOTS + 1;
     // VISC: gradients of the variables the viscous flux reads (primitive u, v;
     // conserved a1r1, a2r2, ru, rv) at the top face, kept for the row above:
-    // [q][g][d][cell], right behind the barriers
+    // [q][g][d][cell], at the end
     constexpr int NG = CONS ? 4 : 2, G0 = CONS ? 0 : 2;
-    double *ygt_s = carry_s + K::CARRY_ELEMS + 8;
+    double *fx_s = carry_s + K::CARRY_ELEMS + 8;                // FX_OWN: F [c][cell], D [z][cell]
+    double *ygt_s = fx_s + (K::FX_OWN ? K::FX_ELEMS : 0);
     double *red_s = carry_s;                                    // block reductions at the tile's end
 
     const int t = threadIdx.x;
@@ -370,6 +385,7 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
     __syncthreads();   // the previous tile of this block is done with every buffer
     if (t == 0) {
         for (int s = 0; s <= SLOTS; ++s) mbar_init(&bars[s], 1);
+        mbar_init(fluxes_read, K::NT / 32);
         fence_mbar_init();
     }
     __syncthreads();
@@ -379,6 +395,8 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
     auto slot_of = [&](int row) { return (row - row_lo) % SLOTS; };
     auto row_ptr = [&](int row) { return rows_s + (size_t)slot_of(row) * K::SLOT_STRIDE; };   // [c][BW]
     auto cidx = [&](int slot, int c, int cell) { return (slot * NV + c) * CELLS + cell; };     // coef_s index
+    auto flux_s = [&](int c, int cell) -> double & { return K::FX_OWN ? fx_s[c * CELLS + cell] : coef_s[cidx(0, c, cell)]; };
+    auto fluct_s = [&](int c, int z, int cell) -> double & { return K::FX_OWN ? fx_s[(NV + z) * CELLS + cell] : coef_s[cidx(2, c, cell)]; };
     auto t1_s = [&](int c) -> double & { return carry_s[c * CELLS + m]; };
     auto g_s = [&](int c) -> double & { return carry_s[(NV + c) * CELLS + m]; };
     auto ncp_s = [&](int z) -> double & { return carry_s[(2 * NV + z) * CELLS + m]; };
@@ -437,7 +455,7 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
             drained = drained && mbar_wait_until(&bars[slot_of(row)], (unsigned)(((row - row_lo) / SLOTS) & 1), deadline);
         if (orow_pending) drained = drained && mbar_wait_until(&bars[SLOTS], orow_parity, deadline);
         if (drained)
-            for (int k = 0; k <= SLOTS; ++k) mbar_inval(&bars[k]);
+            for (int k = 0; k <= SLOTS + 1; ++k) mbar_inval(&bars[k]);
     };
     // thread 0: issue the ring rows up to `last`
     auto issue_rows = [&](int last) {
@@ -575,6 +593,9 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
                 return st;
             };
             auto keep = [&](const double *cf) {
+                // the row's first store over the fluxes: most of a reconstruction after they were
+                // read, so the wait is over before it begins
+                if (!K::FX_OWN && kv == 0 && r >= y0) here = mbar_wait_bounded(fluxes_read, (unsigned)((r - y0) & 1)) && here;
 #pragma unroll
                 for (int k = 1; k < NDOF; ++k) coef_s[cidx(k - 1, c, m)] = cf[k];
             };
@@ -896,15 +917,17 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
 #pragma unroll
                 for (int c = 0; c < NV; ++c) { Fq[c] = 0.0; Dq[c] = 0.0; Vq[c] = 0.0; }
             }
-            __syncwarp();   // both halves have their left values: the fluxes may replace them
+            if constexpr (!K::FX_OWN) __syncwarp();   // both halves have their left values: the fluxes may replace them
             static_for<(NV + 1) / 2>([&](auto jj) {
                 constexpr int j = decltype(jj)::value, z0 = K::nz(2 * j), z1 = 2 * j + 1 < NV ? K::nz(2 * j + 1) : -1;
                 Fown[j] = face_sum(jj, Fq, Vq);
                 Down[j] = 0.0;
                 if constexpr (z0 >= 0 || z1 >= 0) Down[j] = fluct_sum(jj, Dq);
                 if (!xface || (2 * j + 1 >= NV && h)) return;
-                coef_s[cidx(0, 2 * j + h, m)] = Fown[j];
-                if constexpr (z0 >= 0 || z1 >= 0) coef_s[cidx(2, 2 * j + h, m)] = Down[j];
+                flux_s(2 * j + h, m) = Fown[j];
+                if constexpr (z0 >= 0 || z1 >= 0) {
+                    if ((h ? z1 : z0) >= 0) fluct_s(2 * j + h, h ? z1 : z0, m) = Down[j];
+                }
             });
         }
         bool late = false;
@@ -925,12 +948,16 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
                 constexpr int j = decltype(jj)::value, z0 = K::nz(2 * j), z1 = 2 * j + 1 < NV ? K::nz(2 * j + 1) : -1;
                 if (2 * j + 1 >= NV && h) return;
                 const int c = 2 * j + h;
-                double X = coef_s[cidx(0, c, m + 1)] - Fown[j];
+                double X = flux_s(c, m + 1) - Fown[j];
                 if constexpr (z0 >= 0 || z1 >= 0) {
-                    if ((h ? z1 : z0) >= 0) X = X + 0.5 * (coef_s[cidx(2, c, m + 1)] + Down[j]);
+                    if ((h ? z1 : z0) >= 0) X = X + 0.5 * (fluct_s(c, h ? z1 : z0, m + 1) + Down[j]);
                 }
                 t1_s(c) = -r1_h * X;
             });
+        }
+        if constexpr (!K::FX_OWN) {
+            __syncwarp();
+            if ((t & 31) == 0) mbar_arrive(fluxes_read);
         }
     }
 
@@ -964,7 +991,7 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
             }
         }
     }
-    for (int k = t; k <= SLOTS; k += K::NT) mbar_inval(&bars[k]);
+    for (int k = t; k <= SLOTS + 1; k += K::NT) mbar_inval(&bars[k]);
 }
 
 }  // namespace hype

@@ -84,3 +84,28 @@ def test_scaled_units(hp, orc, name, scale):
     U[:, :k] *= scale
     cfg.pi1, cfg.pi2 = cfg.pi1 * scale, cfg.pi2 * scale
     _same(hp, orc, cfg, U.reshape(-1))
+
+
+def test_repeated_batches_give_the_same_bits(hp):
+    """Warps of a block run up to most of a row apart; whatever their order, neighbouring columns'
+    fluxes are read before the next row's coefficients replace them."""
+    grids = [(hp.Config(nx=nx, ny=ny, cfl=0.4, bc_bottom=hp.BC_REFLECTIVE, bc_top=hp.BC_REFLECTIVE, **cases.KAPILA_EOS), k)
+             for k, (nx, ny) in enumerate([(476, 435), (380, 486), (409, 300), (230, 290)])]
+    states = [hp.initial_state(c, "shock_bubble", seed=k, nbubbles=4) for c, k in grids]
+    seen = set()
+    with hp.Batch(max_instances=len(grids), max_cells=512 * 512) as b:
+        for _ in range(8):
+            ids = [b.add(c, U, 0.0, 1e30, 12) for (c, _), U in zip(grids, states)]
+            b.advance(12)
+            b.sync()
+            seen.add(b"".join(b.get_state(i).tobytes() for i in ids))
+            for i in ids:
+                b.remove(i)
+    assert len(seen) == 1
+    lone = []
+    for (c, _), U in zip(grids, states):
+        with hp.Solver(c) as s:
+            s.set_state(U)
+            s.solve(0.0, 1e30, 12)
+            lone.append(s.get_state().tobytes())
+    assert seen == {b"".join(lone)}
