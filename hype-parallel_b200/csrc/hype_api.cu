@@ -162,10 +162,6 @@ static StageParams base_params(const hype_solver *s)
     return p;
 }
 
-// Tile width and decomposition: `waves` waves of strips x row runs (<= SMs x
-// resident blocks each), at least 8 rows per run.  Rebuilds the TMA
-// descriptors, whose box width follows the tile width, and drops the captured
-// step graph (recaptured on the next hype_begin / hype_advance).
 // FP32 (nf planes) and FP64 (nd planes) maps of a mixed state (MixedLayout), box
 // (cells + 8, 1, planes); a slab's maps also cover its halo rows and start row_off
 // rows below row 0
@@ -182,56 +178,81 @@ static int make_mixed_maps(hype_solver *s, MixedMaps *mm, float *pf, double *pd)
     return HYPE_OK;
 }
 
-static int set_tiling(hype_solver *s, int cells, int waves = 1)
+// the stage kernel of a solver for a tile width: resident blocks per SM, 0 if there is none
+static int tile_blocks(hype_solver *s, int cells)
 {
     const hype_config *cfg = &s->cfg;
+    const bool cons = (cfg->flags & HYPE_FLAG_CONSERVATIVE) != 0;
+    if (s->mixed) return mixed_blocks_per_sm(cfg->system, cells);
+    if (cfg->flags & HYPE_FLAG_VISCOUS)   // the viscous and conservative kernels come in 128-column tiles only
+        return cells == STAGE_CELLS && stage_visc_configure(cfg->order, cons) == cudaSuccess ? stage_visc_blocks_per_sm(cfg->order, cons) : 0;
+    if (cons)
+        return cells == STAGE_CELLS && stage_cons_configure(cfg->system, cfg->order) == cudaSuccess
+                   ? stage_cons_blocks_per_sm(cfg->system, cfg->order) : 0;
+    if (s->fast)
+        return stage_fast_configure(cfg->system, cfg->order, cells) == cudaSuccess ? stage_fast_blocks_per_sm(cfg->system, cfg->order, cells) : 0;
+    return stage_configure(cfg->system, cfg->order, cells) == cudaSuccess ? stage_blocks_per_sm(cfg->system, cfg->order, cells) : 0;
+}
+static int tile_strips(const hype_solver *s, int cells)
+{
+    return s->mixed ? mixed_strips(s->cfg.nx, cells) : stage_strips(s->cfg.nx, cells);
+}
+
+// Tile width and number of row runs.  Rebuilds the TMA descriptors, whose box width
+// follows the tile width, and drops the captured step graph (recaptured on the next
+// hype_begin / hype_advance).
+static int apply_tiling(hype_solver *s, int cells, int runs, int waves)
+{
     int rc;
     s->cells = cells;
+    s->bps = tile_blocks(s, cells);
+    if (s->bps < 1) return fail(s, HYPE_ERR_CUDA, "stage kernel does not fit on an SM");
+    s->strips = tile_strips(s, cells);
+    s->runs = runs;
+    s->waves = waves;
     if (s->mixed) {
-        s->bps = mixed_blocks_per_sm(cfg->system, cells);
-        if (s->bps < 1) return fail(s, HYPE_ERR_CUDA, "mixed stage kernel does not fit on an SM");
-        s->strips = mixed_strips(cfg->nx, cells);
-        s->waves = waves > 0 ? waves : 1;
-        int runs = s->sms * s->bps * s->waves / s->strips;
-        if (runs < 1) runs = 1;
-        if (runs > cfg->ny / 8) runs = cfg->ny / 8 > 0 ? cfg->ny / 8 : 1;
-        s->runs = runs;
         for (int k = 0; k < 3; ++k)
             if ((rc = make_mixed_maps(s, &s->mm[k], s->mf[k], s->md[k]))) return rc;
-        if (s->step_exec) { cudaGraphExecDestroy(s->step_exec); s->step_exec = nullptr; }
-        return HYPE_OK;
+    } else if ((rc = make_tmap(s, &s->tmU, s->dU)) || (rc = make_tmap(s, &s->tmS0, s->dS0)) || (rc = make_tmap(s, &s->tmS1, s->dS1))) {
+        return rc;
     }
-    if (cfg->flags & HYPE_FLAG_VISCOUS) {   // the viscous kernels come in 128-column tiles only
-        cells = STAGE_CELLS;
-        s->cells = cells;
-        const bool cons = (cfg->flags & HYPE_FLAG_CONSERVATIVE) != 0;
-        CUDA_TRY(s, stage_visc_configure(cfg->order, cons));
-        s->bps = stage_visc_blocks_per_sm(cfg->order, cons);
-    } else if (cfg->flags & HYPE_FLAG_CONSERVATIVE) {   // the conservative kernels come in 128-column tiles only
-        cells = STAGE_CELLS;
-        s->cells = cells;
-        CUDA_TRY(s, stage_cons_configure(cfg->system, cfg->order));
-        s->bps = stage_cons_blocks_per_sm(cfg->system, cfg->order);
-    } else if (s->fast) {
-        CUDA_TRY(s, stage_fast_configure(cfg->system, cfg->order, cells));
-        s->bps = stage_fast_blocks_per_sm(cfg->system, cfg->order, cells);
-    } else {
-        CUDA_TRY(s, stage_configure(cfg->system, cfg->order, cells));
-        s->bps = stage_blocks_per_sm(cfg->system, cfg->order, cells);
-    }
-    if (s->bps < 1) return fail(s, HYPE_ERR_CUDA, "stage kernel does not fit on an SM");
-    s->strips = stage_strips(cfg->nx, cells);
-    const int slots = s->sms * s->bps * (waves > 0 ? waves : 1);
-    s->waves = waves > 0 ? waves : 1;
-    int runs = slots / s->strips;
-    if (runs < 1) runs = 1;
-    if (runs > cfg->ny / 8) runs = cfg->ny / 8 > 0 ? cfg->ny / 8 : 1;
-    s->runs = runs;
-    if ((rc = make_tmap(s, &s->tmU, s->dU)) || (rc = make_tmap(s, &s->tmS0, s->dS0)) || (rc = make_tmap(s, &s->tmS1, s->dS1))) return rc;
     if (s->step_exec) { cudaGraphExecDestroy(s->step_exec); s->step_exec = nullptr; }
     return HYPE_OK;
 }
 
+// `waves` waves of strips x row runs (<= SMs x resident blocks each), at least 8 rows per run
+static int set_tiling(hype_solver *s, int cells, int waves)
+{
+    if (!s->mixed && (s->cfg.flags & (HYPE_FLAG_VISCOUS | HYPE_FLAG_CONSERVATIVE))) cells = STAGE_CELLS;
+    const int bps = tile_blocks(s, cells);
+    if (bps < 1) return fail(s, HYPE_ERR_CUDA, "stage kernel does not fit on an SM");
+    int runs = s->sms * bps * waves / tile_strips(s, cells);
+    if (runs > s->cfg.ny / 8) runs = s->cfg.ny / 8;
+    return apply_tiling(s, cells, runs > 0 ? runs : 1, waves);
+}
+
+// The shape a solver starts with, by estimated time (best_runs): the tile width and runs of
+// least estimate where that is at least 3 % below 128-column tiles in one wave of runs of 8
+// rows or more, else those (large grids: the estimates differ by less than they are sure of).
+// Before -> after: Kapila 64^2 device right-hand side 110 -> 48 us, N = 3 500^2 247 -> 218 us, 20 N = 1
+// steps of 128^2 with their copies 2.48 -> 0.98 ms.
+static int default_tiling(hype_solver *s)
+{
+    const int wide = s->mixed ? MIXED_CELLS : STAGE_CELLS;
+    int rc;
+    if ((rc = set_tiling(s, wide, 1))) return rc;
+    const int rows = (s->cfg.ny + s->runs - 1) / s->runs;
+    double least = 0.97 * tile_launch_cost(s->mixed, wide, s->sms, s->bps, (long long)s->strips * s->runs, rows);
+    int cells = 0, runs = 0;
+    for (int c : {64, 128}) {
+        const int bps = tile_blocks(s, c);
+        if (bps < 1) continue;
+        double cost;
+        const int r = best_runs(s->mixed, c, s->sms, bps, tile_strips(s, c), s->cfg.ny, &cost);
+        if (cost < least) { least = cost; cells = c; runs = r; }
+    }
+    return cells ? apply_tiling(s, cells, runs, 1) : HYPE_OK;
+}
 
 static const CUtensorMap &tmap_for(const hype_solver *s, const double *buf)
 {
@@ -773,7 +794,7 @@ static int create_common(hype_solver *s, const hype_config *cfg, int row_off, co
     }
 
     s->sms = prop.multiProcessorCount;
-    return set_tiling(s, s->mixed ? MIXED_CELLS : STAGE_CELLS);
+    return default_tiling(s);
 }
 
 int hype::create_block(const hype_config *global, int col0, int cols, int row0, int rows, const bool halo[4], hype_solver **out)
@@ -1368,17 +1389,22 @@ int hype_autotune(hype_solver *s, int reps, int *cells_out, int *waves_out)
     if (reps < 1) reps = 3;
     static const int cand_cells[2] = {64, 128};
     static const int cand_waves[3] = {1, 2, 4};
-    int best_c = s->cells, best_w = s->waves, rc;
+    int best_c = 0, best_w = 1, rc;
     double best = 1e300;
+    // the estimated shape first, then the candidates
+    if ((rc = default_tiling(s)) || (rc = hype_time_stage(s, reps, &best))) return rc;
+    best_c = s->cells;
+    const int best_r = s->runs;
+    bool estimated = true;
     for (int c : cand_cells)
         for (int w : cand_waves) {
             if ((rc = set_tiling(s, c, w))) return rc;
 
             double ms = 0.0;
             if ((rc = hype_time_stage(s, reps, &ms))) return rc;
-            if (ms < best) { best = ms; best_c = c; best_w = w; }
+            if (ms < best) { best = ms; best_c = c; best_w = w; estimated = false; }
         }
-    if ((rc = set_tiling(s, best_c, best_w))) return rc;
+    if ((rc = estimated ? apply_tiling(s, best_c, best_r, 1) : set_tiling(s, best_c, best_w))) return rc;
     if (cells_out) *cells_out = best_c;
     if (waves_out) *waves_out = best_w;
     return HYPE_OK;

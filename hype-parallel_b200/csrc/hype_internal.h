@@ -124,6 +124,49 @@ cudaError_t launch_path_batch(int path, int sys, int order, const StageParams *i
 // columns and the last one at most nx/S + 2 <= cells-2.
 inline int stage_strips(int nx, int cells) { return (nx + (cells - 4) - 1) / (cells - 4); }
 
+// Row runs of a grid.  A block takes (H + 2.7) row iterations for a run of H rows (one
+// reconstructed row below and above, prologue and launch), and an iteration of a 64-column
+// tile alone on its SM is mostly latency: k tiles on one SM take only f(k) times as long.
+// Measured f on a B200, 592 columns, H = 1..16, 1 = one 64-column tile (6.2 us Kapila N = 2,
+// 4.1 us N = 1, 8.3 us Baer-Nunziato, 3.9 us Euler, 5.3 us mixed Kapila):
+//   FP64   64 columns 1, 1.13-1.23, 1.33-1.58, 1.56-1.66;  128 columns 1.15-1.39, 1.58-2.07
+//   mixed  64 columns 1, 1.14-1.18, 1.32-1.41, 1.5-1.68;   128 columns 1.06, 1.31-1.44, 1.71-1.96
+// So a grid that cannot fill the SMs with long runs takes shorter ones: 64^2 Kapila as 2 strips
+// x 64 one-row runs (128 blocks) instead of 1 x 8.
+inline double tile_iteration_cost(bool mixed, int cells, int k)
+{
+    static const double f64[6] = {1.0, 1.18, 1.43, 1.65, 1.9, 2.15};
+    static const double fp64_128[3] = {1.25, 1.8, 2.3}, mixed_128[3] = {1.06, 1.4, 1.87};
+    if (cells == 64) return k <= 6 ? f64[k - 1] : f64[5] + 0.25 * (k - 6);
+    const double *f = mixed ? mixed_128 : fp64_128;
+    return k <= 3 ? f[k - 1] : f[2] + 0.5 * (k - 3);
+}
+// the estimated time of a launch of strips x runs tiles, bps resident per SM, in iterations
+// of one 64-column tile
+inline double tile_launch_cost(bool mixed, int cells, int sms, int bps, long long tiles, int rows)
+{
+    const int n = (int)((tiles + sms - 1) / sms);   // tiles of the fullest SM
+    const double f = (n / bps) * tile_iteration_cost(mixed, cells, bps) +
+                     (n % bps ? tile_iteration_cost(mixed, cells, n % bps) : 0.0);
+    return f * (rows + 2.7);
+}
+// the number of row runs (1 .. ny) with the least estimated time, and that time
+inline int best_runs(bool mixed, int cells, int sms, int bps, int strips, int ny, double *cost)
+{
+    int best = 1;
+    *cost = 1e300;
+    for (int n = 1; n <= 4 * bps; ++n) {
+        long long runs = (long long)sms * n / strips;
+        if (runs < 1) runs = 1;
+        if (runs > ny) runs = ny;
+        const int rows = (int)((ny + runs - 1) / runs);
+        runs = (ny + rows - 1) / rows;              // no more runs than that height needs
+        const double c = tile_launch_cost(mixed, cells, sms, bps, runs * strips, rows);
+        if (c < *cost) { *cost = c; best = (int)runs; }
+    }
+    return best;
+}
+
 // One stage of an SSP-RK step over a solver's state buffers (B_U = u^n, B_S0..B_S2
 // work vectors; B_NONE = unused): in -> out with OUT_* `mode` and coefficients
 // ka, kb, kc; x = second state, out2 = second output; reduce = fold the max

@@ -131,9 +131,8 @@ extern "C" HYPE_API int hype_rhs_prim_noalloc(const hype_config *cfg, double t, 
     const int bps = stage_blocks_per_sm(cfg->system, cfg->order, STAGE_CELLS);
     if (bps < 1) return HYPE_ERR_CUDA;
     const int strips = stage_strips(cfg->nx, STAGE_CELLS);
-    int runs = sms * bps / strips;
-    if (runs < 1) runs = 1;
-    if (runs > cfg->ny / 8) runs = cfg->ny / 8 > 0 ? cfg->ny / 8 : 1;
+    double cost;
+    const int runs = best_runs(false, STAGE_CELLS, sms, bps, strips, cfg->ny, &cost);
 
     StageParams p;
     std::memset(&p, 0, sizeof(p));

@@ -109,3 +109,32 @@ def test_repeated_batches_give_the_same_bits(hp):
             s.solve(0.0, 1e30, 12)
             lone.append(s.get_state().tobytes())
     assert seen == {b"".join(lone)}
+
+
+@pytest.mark.parametrize("ny", [3, 4, 7, 16, 33, 150])
+def test_run_heights(hp, orc, ny):
+    """The estimated tile shapes: short grids take row runs of one to a few rows."""
+    for order in (1, 2, 3):
+        _same(hp, orc, *_kapila(order, 131, ny, scale_p=1e5))
+
+
+@pytest.mark.parametrize("system", ["kapila", "bn", "euler"])
+@pytest.mark.parametrize("precision", ["mixed", "fast"])
+@pytest.mark.parametrize("nx,ny", [(64, 64), (131, 5), (37, 200)])
+def test_shapes_of_the_other_forms(hp, system, precision, nx, ny):
+    """The right-hand side does not depend on the tile shape: the estimated one against those the
+    autotuner tries and keeps, and against row bands of a host call."""
+    kind, eos = {"kapila": ("shock_bubble", cases.KAPILA_EOS), "bn": ("bn_discs", cases.KAPILA_EOS),
+                 "euler": ("euler_quadrants", cases.EULER_EOS)}[system]
+    cfg = hp.Config(system={"kapila": hp.KAPILA_5EQN, "bn": hp.BAER_NUNZIATO, "euler": hp.EULER}[system], nx=nx, ny=ny, cfl=0.4,
+                    precision={"mixed": hp.PREC_MIXED, "fast": hp.PREC_FP64_FAST}[precision], flags=hp.FLAG_BN_FIX_P2, **eos)
+    U = hp.initial_state(cfg, kind, seed=5)
+    got = []
+    with hp.Solver(cfg) as s:
+        for tune in (False, True):
+            if tune:
+                s.autotune(1)
+            s.set_state(U)
+            n, t, dt, st = s.solve(0.0, 1e30, 3)
+            got.append((n, t, dt, st, s.get_state().tobytes(), s.rhs_function_prim(0.0, U)[0].tobytes()))
+    assert got[0] == got[1] and got[0][3] == hp.OK
