@@ -91,6 +91,8 @@ struct Kind {
     int nstage = 0, copy_back = 0;
     PlanStage plan[MAX_PLAN];
     int cells = STAGE_CELLS, rows = 64, bps = 0;
+    bool shaped = false;               // the tile shape was set (hype_batch_set_tiling, hype_batch_autotune)
+    bool joined = false;               // members came or went since the shape was last estimated
     std::vector<int> members;
     StageParams *dParams = nullptr;    // [MAX_PLAN][M]
     MixedParams *dMParams = nullptr;   // [MAX_PLAN][M]
@@ -237,16 +239,44 @@ static int kind_init(hype_batch *b, int id, const hype_config &c)
 }
 
 // Tile decomposition of one instance for the kind's tile shape: strips of the
-// stage kernel's column tiling, runs of about `rows` rows (at least 8 each).
+// stage kernel's column tiling, runs of about `rows` rows (at least 8 each, 4 for shorter
+// tiles).
+static int inst_runs(int ny, int rows)
+{
+    int runs = (ny + rows / 2) / rows;
+    const int least = rows < 8 ? 4 : 8;
+    const int cap = ny / least > 0 ? ny / least : 1;
+    if (runs > cap) runs = cap;
+    return runs < 1 ? 1 : runs;
+}
+static int inst_strips(const Kind &k, int nx, int cells) { return k.mixed ? mixed_strips(nx, cells) : stage_strips(nx, cells); }
 static void inst_tiling(const Kind &k, Inst &in)
 {
-    const int nx = in.cfg.nx, ny = in.cfg.ny;
-    in.strips = k.mixed ? mixed_strips(nx, k.cells) : stage_strips(nx, k.cells);
-    int runs = (ny + k.rows / 2) / k.rows;
-    const int cap = ny / 8 > 0 ? ny / 8 : 1;
-    if (runs > cap) runs = cap;
-    if (runs < 1) runs = 1;
-    in.runs = runs;
+    in.strips = inst_strips(k, in.cfg.nx, k.cells);
+    in.runs = inst_runs(in.cfg.ny, k.rows);
+}
+
+// Estimated time of one stage over the kind's members with tiles of cells x rows, in the
+// unit of tile_iteration_cost.  Tiles that all fit at once take the tallest one's iterations;
+// more than that are shared out longest first, so the resident blocks end within half a tile
+// of each other (the last ones are split, rebuild_work).
+static double shape_cost(const hype_batch *b, const Kind &k, int cells, int rows, int bps)
+{
+    long long tiles = 0, iters10 = 0;
+    int tallest = 0;
+    for (int s : k.members) {
+        const hype_config &c = b->inst[s].cfg;
+        const int runs = inst_runs(c.ny, rows), strips = inst_strips(k, c.nx, cells), h = (c.ny + runs - 1) / runs;
+        tiles += (long long)strips * runs;
+        iters10 += (long long)strips * (10LL * c.ny + 27LL * runs);
+        tallest = std::max(tallest, h);
+    }
+    const long long slots = (long long)b->sms * bps;
+    // the persistent FP64 kernels spill at 128 columns (their parameters are in shared memory, not in
+    // the constant bank): 48 grids of sides 200..1024 take 34.1 ms a step with them, 31.1 with 64
+    const double spill = !k.mixed && cells == STAGE_CELLS ? 1.1 : 1.0;
+    if (tiles <= slots) return spill * tile_launch_cost(k.mixed, cells, b->sms, bps, tiles, tallest);
+    return spill * tile_iteration_cost(k.mixed, cells, bps) * (0.1 * (double)iters10 / (double)slots + 0.4 * (tallest + 2.7));
 }
 
 static StageParams inst_params(hype_batch *b, const Inst &in, const PlanStage &q)
@@ -455,6 +485,35 @@ static int kind_set_tiling(hype_batch *b, int id, int cells, int rows)
     if ((rc = rebuild_work(b, id))) return rc;
     b->dirty = true;
     return HYPE_OK;
+}
+
+// The shape of least estimate over the kind's members, if that is below `least`.
+static bool best_shape(hype_batch *b, const Kind &k, double least, int *cells, int *rows)
+{
+    bool found = false;
+    for (int c : {64, 128}) {
+        const int bps = kind_blocks_per_sm(k, c);
+        if (bps < 1) continue;
+        for (int r : {4, 8, 12, 16, 24, 32, 48, 64, 96, 128}) {
+            const double t = shape_cost(b, k, c, r, bps);
+            if (t < least) { least = t; *cells = c; *rows = r; found = true; }
+        }
+    }
+    return found;
+}
+
+// The tile shape of a kind whose members changed and whose shape nobody set: the least
+// estimate, if it is 3 % below the present shape's.  Milliseconds a step with 128 x 64 tiles ->
+// with the estimated ones: 16 Kapila grids of sides 128..512 4.33 -> 3.51 (mixed 3.31 -> 2.05),
+// 12 of 64..160 2.06 -> 0.53, 4 of 64..128 2.50 -> 0.31, 48 of 200..1024 34.1 -> 31.3.
+static int estimate_shape(hype_batch *b, int id)
+{
+    Kind &k = b->kinds[id];
+    if (!k.ready || !k.joined) return HYPE_OK;
+    k.joined = false;
+    int cells, rows;
+    if (k.shaped || k.members.empty() || !best_shape(b, k, 0.97 * shape_cost(b, k, k.cells, k.rows, k.bps), &cells, &rows)) return HYPE_OK;
+    return kind_set_tiling(b, id, cells, rows);
 }
 
 // ---------------------------------------------------------------------------
@@ -734,20 +793,25 @@ int hype_batch_add(hype_batch *b, const hype_config *cfg, const double *U0, doub
         b->hold_dirty = true;
     }
     k.members.push_back(s);
+    k.joined = true;
     if (k.members.size() == 1) b->dirty = true;
     if ((rc = upload_inst(b, s)) || (rc = rebuild_work(b, in.kind))) return rc;
     // hype.c:343: one RHS evaluation of the initial state seeds Ctx.dt
+    double seed_cost;   // a launch of its own: row runs that fill the SMs, not the batch's
+    const int seed_runs = best_runs(mixed, k.cells, b->sms, k.bps, in.strips, cfg->ny, &seed_cost);
     const PlanStage seed{B_U, mixed ? B_NONE : B_S1, OUT_RHS, 0.0, 1.0, 0.0, B_NONE, B_NONE, 1};
     if (mixed) {
         MixedMaps mm[3];
         if ((rc = inst_maps(b, k, in, nullptr, mm))) return rc;
         MixedParams p = inst_mparams(b, in, seed);
+        p.runs = seed_runs;
         p.out_rhs = b->dStage;
         BCUDA(b, launch_mixed(cfg->system, k.cells, mm[0], p, b->stream));
     } else {
         CUtensorMap tm[3];
         if ((rc = inst_maps(b, k, in, tm, nullptr))) return rc;
-        const StageParams sp = inst_params(b, in, seed);
+        StageParams sp = inst_params(b, in, seed);
+        sp.runs = seed_runs;
         if (k.path == BATCH_PATH_CONS) BCUDA(b, launch_stage_cons(k.system, k.order, tm[0], sp, b->stream));
         else if (k.path >= 0) BCUDA(b, launch_stage_visc(k.order, k.path == BATCH_PATH_VISC_CONS, tm[0], sp, b->stream));
         else BCUDA(b, launch_stage(k.system, k.order, k.cells, tm[0], sp, b->stream));
@@ -766,6 +830,7 @@ int hype_batch_remove(hype_batch *b, int id)
     Inst &in = b->inst[id];
     Kind &k = b->kinds[in.kind];
     k.members.erase(std::find(k.members.begin(), k.members.end(), id));
+    k.joined = true;
     if (k.members.empty()) b->dirty = true;
     int rc = rebuild_work(b, in.kind);   // ordered before the next step on the stream
     free_inst(b, in);                     // after the steps already queued
@@ -780,6 +845,8 @@ int hype_batch_advance(hype_batch *b, int nsteps)
     if (!b || nsteps < 0) return bfail(b, HYPE_ERR_INVALID, "bad argument");
     BCUDA(b, cudaSetDevice(b->cfg.device));
     int rc;
+    for (int id = 0; id < NKIND; ++id)
+        if ((rc = estimate_shape(b, id))) return rc;
     if (b->dirty && (rc = capture_step(b))) return rc;
     if (!b->exec) { b->timed = false; return HYPE_OK; }
     if (b->hold_dirty) {
@@ -870,8 +937,10 @@ int hype_batch_set_tiling(hype_batch *b, int cells, int rows)
         return bfail(b, HYPE_ERR_INVALID, "tile shape must be 64 or 128 columns and 16..1024 rows");
     BCUDA(b, cudaSetDevice(b->cfg.device));
     int rc;
-    for (int id = 0; id < NKIND; ++id)
+    for (int id = 0; id < NKIND; ++id) {
+        b->kinds[id].shaped = b->kinds[id].ready;
         if ((rc = kind_set_tiling(b, id, cells, rows))) return rc;
+    }
     return HYPE_OK;
 }
 
@@ -887,22 +956,25 @@ int hype_batch_autotune(hype_batch *b, int reps, int *cells_out, int *rows_out)
     for (int id = 0; id < NKIND; ++id) {
         Kind &k = b->kinds[id];
         if (!k.ready || k.members.empty()) continue;
-        int bc = k.cells, br = k.rows;
-        double best = 1e300;
-        for (int c : cand_cells)
-            for (int r : cand_rows) {
-                if (k.path >= 0 && c != STAGE_CELLS) continue;
-                if ((rc = kind_set_tiling(b, id, c, r))) return rc;
-                BCUDA(b, enqueue_kind_stage(b, id, 0, b->stream));   // warm
-                BCUDA(b, cudaEventRecord(b->ev0, b->stream));
-                for (int i = 0; i < reps; ++i) BCUDA(b, enqueue_kind_stage(b, id, 0, b->stream));
-                BCUDA(b, cudaEventRecord(b->ev1, b->stream));
-                BCUDA(b, cudaStreamSynchronize(b->stream));
-                float ms = 0.f;
-                BCUDA(b, cudaEventElapsedTime(&ms, b->ev0, b->ev1));
-                if (ms < best) { best = ms; bc = c; br = r; }
-            }
-        if ((rc = kind_set_tiling(b, id, bc, br))) return rc;
+        int bc = k.cells, br = k.rows, ec = k.cells, er = k.rows;
+        double best = 1e300, est = 1e300;
+        best_shape(b, k, 1e300, &ec, &er);
+        for (int i = 0; i <= 8; ++i) {   // the estimated shape, then the fixed candidates
+            const int c = i == 0 ? ec : cand_cells[(i - 1) / 4], r = i == 0 ? er : cand_rows[(i - 1) % 4];
+            if (k.path >= 0 && c != STAGE_CELLS) continue;
+            if ((rc = kind_set_tiling(b, id, c, r))) return rc;
+            BCUDA(b, enqueue_kind_stage(b, id, 0, b->stream));   // warm
+            BCUDA(b, cudaEventRecord(b->ev0, b->stream));
+            for (int q = 0; q < reps; ++q) BCUDA(b, enqueue_kind_stage(b, id, 0, b->stream));
+            BCUDA(b, cudaEventRecord(b->ev1, b->stream));
+            BCUDA(b, cudaStreamSynchronize(b->stream));
+            float ms = 0.f;
+            BCUDA(b, cudaEventElapsedTime(&ms, b->ev0, b->ev1));
+            if (i == 0) est = ms;
+            else if (ms < best) { best = ms; bc = c; br = r; }
+        }
+        k.shaped = best < est;   // else the estimate, which goes on following the members
+        if ((rc = k.shaped ? kind_set_tiling(b, id, bc, br) : kind_set_tiling(b, id, ec, er))) return rc;
         if (k.cost > most) {
             most = k.cost;
             if (cells_out) *cells_out = bc;

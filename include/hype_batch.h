@@ -115,7 +115,9 @@ HYPE_API int hype_batch_get_state(hype_batch *b, int id, double *U);
  * Tile shape of the persistent launches: tile width `cells` (64 or 128
  * columns) and about `rows` rows per tile (16..1024), applied to every
  * instance kind (the conservative and viscous kinds keep 128 columns).
- * Rebuilds the work-list and the step graph.
+ * Rebuilds the work-list and the step graph.  Until this call or the autotuner
+ * sets a kind's shape, it is estimated from its instances at each advance
+ * after some joined or left.
  */
 HYPE_API int hype_batch_set_tiling(hype_batch *b, int cells, int rows);
 
@@ -123,7 +125,9 @@ HYPE_API int hype_batch_set_tiling(hype_batch *b, int cells, int rows);
  * Autotuner: times the first stage of a step over the current instances
  * (inputs untouched, reps launches per candidate) for every tile width in
  * {64, 128} and rows per tile in {16, 32, 64, 128}, per instance kind, and
- * keeps the fastest; reports the choice of the kind with the most work.
+ * keeps the fastest; a kind whose estimated shape is faster than all of them
+ * keeps that (and goes on following its instances).  Reports the fastest of
+ * the candidates of the kind with the most work.
  */
 HYPE_API int hype_batch_autotune(hype_batch *b, int reps, int *cells, int *rows);
 
