@@ -911,11 +911,18 @@ template <> struct Recon<2> {
         c[5] = w0 * uxy0 + w1 * uxy1 + w2 * uxy2 + w3 * uxy3;
     }
 };
-// reconstruction.c:223-357
-template <> struct Recon<3> {
-    __device__ __forceinline__ static void run(const Stencil &s, double *coeffs)
+// reconstruction.c:223-357.  CR: the weights' quotients by the branch-free forms, checked by
+// `ck` (as Recon2Cr: every weight is gamma / d with d >= 1e-48 and then divided by the sum);
+// Kapila 500^2 right-hand side 218 -> 196 us
+struct Recon3 {
+    template <bool CR>
+    __device__ __forceinline__ static void weights(const Stencil &s, double *coeffs, CrCheck &ck)
     {
-        const double gammaHi = 0.85, gammaLo = 0.85;
+        auto over_d = [&](double g, double d) {
+            if constexpr (CR) { ck.divisor(d); return div_rn(g, d, rcp_rn(d)); }
+            else return g / d;
+        };
+        constexpr double gammaHi = 0.85, gammaLo = 0.85;
         double u_0 = s.c;
         double u_ip1 = s.xp1, u_jp1 = s.yp1, u_ip1jp1 = s.pp;
         double u_im1 = s.xm1, u_jm1 = s.ym1, u_ip1jm1 = s.pm;
@@ -937,7 +944,7 @@ template <> struct Recon<3> {
         double IS_R4 = (u_xR4 + 0.1 * u_xxxR4) * (u_xR4 + 0.1 * u_xxxR4) + R13_3 * (u_xxR4 * u_xxR4 + u_yyR4 * u_yyR4) +
                        (u_yR4 + 0.1 * u_yyyR4) * (u_yR4 + 0.1 * u_yyyR4) + 39.05 * (u_xxxR4 * u_xxxR4 + u_yyyR4 * u_yyyR4) +
                        R7_6 * u_xyR4 * u_xyR4 + 4.7 * (u_xxyR4 * u_xxyR4 + u_xyyR4 * u_xyyR4);
-        double w_R4 = gamma_R4 / (pow4(IS_R4 + SMALL_NUM));
+        double w_R4 = over_d(gamma_R4, pow4(IS_R4 + SMALL_NUM));
         double sum = w_R4;
         double u_xR3[5], u_yR3[5], u_xxR3[5], u_yyR3[5], u_xyR3[5], w_R3[5];
         u_xR3[0] = 0.5 * (-u_im1 + u_ip1);
@@ -968,13 +975,24 @@ template <> struct Recon<3> {
 #pragma unroll
         for (int i = 0; i < 5; ++i) {
             double IS = u_xR3[i] * u_xR3[i] + u_yR3[i] * u_yR3[i] + R13_3 * (u_xxR3[i] * u_xxR3[i] + u_yyR3[i] * u_yyR3[i]) + R7_6 * u_xyR3[i] * u_xyR3[i];
-            w_R3[i] = gamma_R3[i] / (pow4(IS + SMALL_NUM));
+            w_R3[i] = over_d(gamma_R3[i], pow4(IS + SMALL_NUM));
             sum += w_R3[i];
         }
-        w_R4 = w_R4 / sum;
+        double wt_ratio;
+        if constexpr (CR) {
+            ck.sum(sum);
+            const double y = rcp_rn(sum);
+            w_R4 = div_rn(w_R4, sum, y);
 #pragma unroll
-        for (int i = 0; i < 5; ++i) w_R3[i] = w_R3[i] / sum;
-        double wt_ratio = w_R4 / gamma_R4;
+            for (int i = 0; i < 5; ++i) w_R3[i] = div_rn(w_R3[i], sum, y);
+            constexpr double r_gamma = 1.0 / gammaHi;   // correctly rounded
+            wt_ratio = div_rn(w_R4, gamma_R4, r_gamma);
+        } else {
+            w_R4 = w_R4 / sum;
+#pragma unroll
+            for (int i = 0; i < 5; ++i) w_R3[i] = w_R3[i] / sum;
+            wt_ratio = w_R4 / gamma_R4;
+        }
         coeffs[0] = u_0;
 #define HYPE_W4(R4, R3) (wt_ratio * (R4 - gamma_R3[0] * R3[0] - gamma_R3[1] * R3[1] - gamma_R3[2] * R3[2] - gamma_R3[3] * R3[3] - gamma_R3[4] * R3[4]) \
                          + w_R3[0] * R3[0] + w_R3[1] * R3[1] + w_R3[2] * R3[2] + w_R3[3] * R3[3] + w_R3[4] * R3[4])
@@ -990,6 +1008,22 @@ template <> struct Recon<3> {
         coeffs[9] = wt_ratio * u_xyyR4;
     }
 };
+template <> struct Recon<3> {
+    __device__ __forceinline__ static void run(const Stencil &s, double *c)
+    {
+        CrCheck ck;
+        Recon3::weights<false>(s, c, ck);
+    }
+};
+struct Recon3Cr {
+    __device__ __forceinline__ static void run(const Stencil &s, double *c, bool &sp)
+    {
+        CrCheck ck;
+        Recon3::weights<true>(s, c, ck);
+        sp = ck.special();
+    }
+};
+template <int N> using ReconCr = std::conditional_t<N == 2, Recon2Cr, Recon3Cr>;
 
 // The unlimited central coefficients (u_coeffs) Reconstruct returns beside
 // the WENO ones (reconstruction.c:139-141, 172-174, 195-196, 217, 258-267);

@@ -603,12 +603,12 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
             if constexpr (FAST) {
                 ReconFast<N>::run(stencil(), cf);
                 keep(cf);
-            } else if constexpr (N == 2) {
+            } else if constexpr (N >= 2) {
                 // branch-free correctly rounded reciprocals and quotients let the weights' chains
                 // overlap; the compiler's division where an operand is outside their range
                 // (from the ring again, so that the stencil is not held for it)
                 bool special;
-                Recon2Cr::run(stencil(), cf, special);
+                ReconCr<N>::run(stencil(), cf, special);
                 keep(cf);
                 if (special && active) {
                     Recon<N>::run(stencil(), cf);
