@@ -411,20 +411,16 @@ __global__ void division_check_kernel(long long n, unsigned long long seed, unsi
             break;
         }
         }
-        bool sp = false;
-        const double q = hype::cr_div(a, b, sp);
         const double ref = a / b;
-        if (sp) ++spec;
-        else if (__double_as_longlong(q) != __double_as_longlong(ref)) ++mism;
-        // rcp_rn and div_rn on the same operands, within their range and low-word rule
-        const unsigned ea = hype::biased_exp(a), eb = hype::biased_exp(b), eq = hype::biased_exp(ref);
-        auto within = [](unsigned e, int lim) { return e >= 1023u - lim && e <= 1023u + lim; };
-        if (!hype::rcp_special(hype::rcp_low(0u, b)) && within(eb, 900)) {
-            const double y = hype::rcp_rn(b);
-            if (__double_as_longlong(y) != __double_as_longlong(1.0 / b)) ++mism;
-            if (within(ea, 900) && within(eq, 900) &&
-                __double_as_longlong(hype::div_rn(a, b, y)) != __double_as_longlong(ref)) ++mism;
+        if (!hype::div_in_range(a, b, ref)) {
+            ++spec;
+            continue;
         }
+        // a divisor that rcp_rn leaves to its caller (all-ones low word): the constant divisors' way
+        const bool low = hype::rcp_special(hype::rcp_low(0u, b));
+        const double y = low ? 1.0 / b : hype::rcp_rn(b);
+        if (!low && __double_as_longlong(y) != __double_as_longlong(1.0 / b)) ++mism;
+        if (__double_as_longlong(hype::div_rn(a, b, y)) != __double_as_longlong(ref)) ++mism;
     }
     for (int o = 16; o > 0; o >>= 1) {
         mism += __shfl_xor_sync(0xffffffffu, mism, o);

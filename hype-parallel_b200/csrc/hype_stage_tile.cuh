@@ -504,14 +504,12 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
 #pragma unroll
             for (int c = 0; c < NV; ++c) V[c] = Q[c];
         } else if constexpr (!FAST && ((SYS == SYS_BN && (N == 1 || N == 2)) || (SYS == SYS_KAPILA && N <= 1))) {
-            // branch-free correctly rounded divisions (hype_div.cuh): the cell's
-            // independent divisions overlap instead of each waiting on the last
-            // one's slow-path branch; the compiler's division where an operand is
-            // outside their range.  Only in the tiles where it measured faster
-            // (Kapila N = 2, 3 lose to the extra registers)
-            bool special = false;
-            S::cons2prim_dv(eos, Q, V, [&special](double a, double b) { return cr_div(a, b, special); });
-            if (special) S::cons2prim(eos, Q, V);
+            // branch-free divisions: the cell's independent ones overlap.  Only in the tiles where
+            // it measured faster (BN 1024^2 0.738 -> 0.731 ms; Kapila N = 2 -0.7 % at 128 columns,
+            // +1.4 % at 64, N = 3 +0.6 %)
+            CrDiv dv;
+            S::cons2prim_dv(eos, Q, V, dv);
+            if (!eos.cr || dv.special()) S::cons2prim(eos, Q, V);
         } else {
             S::cons2prim(eos, Q, V);
         }

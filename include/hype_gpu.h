@@ -322,14 +322,13 @@ HYPE_API int hype_test_skip_row_loads(hype_solver *s, int row);
 
 /*
  * Test hook for the branch-free correctly rounded FP64 divisions the bit-exact
- * kernels use (csrc/hype_div.cuh); no counterpart in the reference.  On device `device`, n operand pairs drawn from `seed` -- random
- * bit patterns (zeros, subnormals, infinities and NaNs included), random
- * operands of every exponent, near-midpoint quotients and divisors with an
- * all-ones significand -- are divided both ways.  *mismatches counts pairs whose
- * result differs from IEEE division bit for bit although the function reported
- * them in range, *specials the pairs it reported out of range (where its caller
- * uses IEEE division).  The shared-reciprocal forms (rcp_rn, div_rn) are compared
- * on the same pairs within their own range and counted as mismatches alike.
+ * kernels use (csrc/hype_div.cuh); no counterpart in the reference.  On device
+ * `device`, n operand pairs drawn from `seed` -- random bit patterns (zeros,
+ * subnormals, infinities and NaNs included), random operands of every exponent,
+ * near-midpoint quotients and divisors with an all-ones significand -- are
+ * divided both ways.  *mismatches counts reciprocals and quotients that differ
+ * from IEEE division bit for bit although the operands are in the functions'
+ * range, *specials the pairs out of it (where their callers use IEEE division).
  */
 HYPE_API int hype_test_division(int device, long long n, unsigned long long seed, long long *mismatches, long long *specials);
 
