@@ -3,6 +3,7 @@
 // SSP-RK time loop (captured once per solver as a CUDA graph and replayed).
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -419,7 +420,7 @@ static int check_config(const hype_config *c, hype_solver *s)
 //    never waits for SM slots (ev_cp: copied, ev_in: converted);
 //  - device->host: a band's result is converted on `cvout` once computed and
 //    copied out on `cout` (ev_dc: converted);
-//  - up to 16 bands, each launch covering half a wave of blocks (host_bands);
+//  - up to 16 bands (rhs_bands; hype_advance_host: each launch half a wave of blocks, host_bands);
 //  - hype_rhs_prim: its one RHS launch, band by band behind the uploads
 //    (banded_upload_stage).  On a 2048^2 Kapila grid a call took 5.4-5.5 ms
 //    with 8 full-wave bands and 4.8 ms this way (the copies alone: 3.6 ms each
@@ -441,20 +442,13 @@ struct Bands {
     int order[hype_solver::MAX_BANDS];     // launch order: band 0 last on a periodic y axis (it reads the last band)
 };
 
-// up to `max_bands` bands of at least `per` runs each (fewer bands on short grids,
-// so that no launch shrinks below `per` runs), at least 8 rows per run
-static Bands make_bands(const hype_solver *s, int max_bands, int per)
+// `runs` row runs in n bands; a band has at least 3 rows (band_needs), its callers see to that
+static Bands split_bands(const hype_solver *s, int runs, int n)
 {
     Bands b;
     const int ny = s->cfg.ny;
-    if (max_bands > hype_solver::MAX_BANDS) max_bands = hype_solver::MAX_BANDS;
-    if (per < 1) per = 1;
-    int runs = max_bands * per;
-    const int cap = ny / 8 > s->runs ? ny / 8 : s->runs;
-    if (runs > cap) runs = cap;
-    if (runs < 1) runs = 1;
     b.runs = runs;
-    b.n = runs / per < 1 ? 1 : (runs / per > max_bands ? max_bands : runs / per);
+    b.n = n;
     for (int k = 0; k <= b.n; ++k) {
         b.run[k] = (int)(((long long)k * runs) / b.n);
         b.row[k] = (int)(((long long)b.run[k] * ny) / runs);
@@ -464,6 +458,20 @@ static Bands make_bands(const hype_solver *s, int max_bands, int per)
     return b;
 }
 
+// up to `max_bands` bands of at least `per` runs each (fewer bands on short grids,
+// so that no launch shrinks below `per` runs), at least 8 rows per run
+static Bands make_bands(const hype_solver *s, int max_bands, int per)
+{
+    const int ny = s->cfg.ny;
+    if (max_bands > hype_solver::MAX_BANDS) max_bands = hype_solver::MAX_BANDS;
+    if (per < 1) per = 1;
+    int runs = max_bands * per;
+    const int cap = ny / 8;
+    if (runs > cap) runs = cap;
+    if (runs < 1) runs = 1;
+    return split_bands(s, runs, runs / per < 1 ? 1 : (runs / per > max_bands ? max_bands : runs / per));
+}
+
 // row runs of one wave of stage blocks
 static int wave_runs(const hype_solver *s)
 {
@@ -471,7 +479,47 @@ static int wave_runs(const hype_solver *s)
     return r > 0 ? r : 1;
 }
 
-// the bands of the host calls: launches of half a wave of blocks
+// The bands of the right-hand side's host calls, by a simulated pipeline: band k's launch waits
+// for the upload of the rows it reads and for the launch before it, its download for the launch
+// and for the download before it.  Copies run at 52 GB/s each way, the host enqueues a band in
+// about 12 us, a launch takes tile_launch_cost (a row run has to be long for the launch's own
+// sake, a band short for the pipeline's).  Launches of many bands are half a wave at most: full
+// ones wait for the SMs that other bands' conversions are on (BN 1024^2 1.95 -> 2.2 ms).  Pinned
+// arrays, 8-row runs -> estimated: Kapila 1024 x 512 0.86 -> 0.80 ms, 512^2 0.59 -> 0.49, mixed
+// 1024^2 1.64 -> 1.45, Euler 800 x 1500 1.32 -> 1.19; where the estimate gains less than 7 %
+// the former bands stay.
+static double pipeline_us(const hype_solver *s, int n, int runs)
+{
+    const int rows = (s->cfg.ny + n - 1) / n;
+    const double bytes = sizeof(double) * (double)s->cfg.nx * s->cfg.ny * s->nv;
+    const double copy = std::max(bytes / n / 52e3 + 4.0, 12.0);
+    const double launch = 5.0 + tile_iteration_us(s->cfg.system, s->cfg.order, s->mixed, s->fast) *
+                                    tile_launch_cost(s->mixed, s->cells, s->sms, s->bps, (long long)s->strips * runs, (rows + runs - 1) / runs);
+    double done = 0.0, down = 0.0;
+    for (int k = 0; k < n; ++k) {
+        const int needs = k + 1 < n ? k + 2 : n;   // uploads that band k waits for
+        done = std::max(needs * copy + 10.0, done) + launch;
+        down = std::max(done + 5.0, down) + copy;
+    }
+    return down;
+}
+static Bands rhs_bands(const hype_solver *s)
+{
+    const int ny = s->cfg.ny, half = wave_runs(s) / 2;
+    Bands best = make_bands(s, hype_solver::MAX_BANDS, half);   // runs of 8 rows or more
+    double least = 0.93 * pipeline_us(s, best.n, best.runs / best.n);
+    int best_n = 0, best_runs = 0;
+    for (int n = 1; n <= hype_solver::MAX_BANDS && (n == 1 || ny / n >= 4); ++n)
+        for (int k = 1; k <= (n <= 2 ? 4 : 2); ++k) {   // one or two bands: a whole wave each
+            const int runs = std::max(1, std::min(half * k / 2, ny / n));
+            const double t = pipeline_us(s, n, runs);
+            if (t < least) { least = t; best_n = n; best_runs = runs; }
+        }
+    return best_n ? split_bands(s, best_n * best_runs, best_n) : best;
+}
+
+// the bands of hype_advance_host, whose stages run over them as a wavefront: launches of half a
+// wave of blocks
 static Bands host_bands(const hype_solver *s) { return make_bands(s, hype_solver::MAX_BANDS, wave_runs(s) / 2); }
 
 // the last band whose rows band k's stencils read (the halo is 3 rows, bands are >= 8)
@@ -940,7 +988,7 @@ int hype_rhs_prim(hype_solver *s, double t, const double *U, double *RHS, double
     CUDA_TRY(s, cudaSetDevice(s->cfg.device));
     int rc;
     // banded: U's rows stream in while earlier bands compute, RHS rows stream out
-    const Bands b = host_bands(s);
+    const Bands b = rhs_bands(s);
     const size_t row_elems = (size_t)s->cfg.nx * s->nv;
     if ((rc = fence_copy_streams(s)) || (rc = reset_scalars(s))) return rc;
     const PlanStage q{B_S0, B_NONE, OUT_RHS, 0.0, 1.0, 0.0, B_NONE, B_NONE, 1};
@@ -996,7 +1044,7 @@ int hype_rhs_prim_slab(hype_solver *s, double t, const double *U, long long row_
     // the last band) are copied from the local array and converted, its RHS launch runs
     // once the rows its stencils read are there, and its RHS rows go to the host while
     // later bands compute
-    const Bands b = host_bands(s);
+    const Bands b = rhs_bands(s);
     if ((rc = fence_copy_streams(s)) || (rc = reset_scalars(s))) return rc;
     HostIO io = host_io(s, U, RHS);
     auto upload = [&](int k) -> int {

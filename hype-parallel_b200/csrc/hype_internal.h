@@ -141,6 +141,13 @@ inline double tile_iteration_cost(bool mixed, int cells, int k)
     const double *f = mixed ? mixed_128 : fp64_128;
     return k <= 3 ? f[k - 1] : f[2] + 0.5 * (k - 3);
 }
+// Microseconds of a row iteration of one 64-column tile alone on its SM (measured for N = 2, for
+// Kapila N = 1 and 3; the others scaled by their operation counts)
+inline double tile_iteration_us(int sys, int order, bool mixed, bool fast)
+{
+    const double n2 = sys == SYS_BN ? (mixed ? 7.4 : 8.3) : sys == SYS_EULER ? (mixed ? 3.5 : 3.9) : mixed ? 5.3 : fast ? 4.3 : 6.2;
+    return n2 * (order == 0 ? 0.5 : order == 1 ? 0.65 : order == 2 ? 1.0 : 1.35);
+}
 // the estimated time of a launch of strips x runs tiles, bps resident per SM, in iterations
 // of one 64-column tile
 inline double tile_launch_cost(bool mixed, int cells, int sms, int bps, long long tiles, int rows)

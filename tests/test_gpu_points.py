@@ -138,3 +138,23 @@ def test_shapes_of_the_other_forms(hp, system, precision, nx, ny):
             n, t, dt, st = s.solve(0.0, 1e30, 3)
             got.append((n, t, dt, st, s.get_state().tobytes(), s.rhs_function_prim(0.0, U)[0].tobytes()))
     assert got[0] == got[1] and got[0][3] == hp.OK
+
+
+@pytest.mark.parametrize("nx,ny", [(18000, 16), (2600, 12), (300, 41), (700, 130)])
+@pytest.mark.parametrize("bc", [O.TRANSMISSIVE, O.PERIODIC])
+def test_bands_of_host_calls(hp, orc, nx, ny, bc):
+    """Row bands of host right-hand sides and host steps on wide, short grids: every band has the
+    rows its neighbours' stencils read."""
+    cfg, U = _kapila(2, nx, ny, scale_p=1e5)
+    cfg.bc_left = cfg.bc_right = cfg.bc_bottom = cfg.bc_top = bc
+    _same(hp, orc, cfg, U)
+    out = np.empty_like(U)
+    with hp.Solver(cases.to_pkg(cfg)) as s:
+        s.set_state(U)
+        s.begin(0.0, 1e30, 2)
+        s.advance(1)
+        st = s.wait()
+        state = s.get_state()
+        s.set_state(U)
+        s.begin(0.0, 1e30, 2)
+        assert s.advance_host(U, out, 1) == st and out.tobytes() == state.tobytes()
