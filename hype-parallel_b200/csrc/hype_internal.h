@@ -99,6 +99,11 @@ cudaError_t stage_configure(int sys, int order, int cells);   // raises the dyna
 int stage_blocks_per_sm(int sys, int order, int cells);
 int stage_batch_blocks_per_sm(int sys, int order, int cells);   // resident blocks of the persistent form
 cudaError_t launch_stage(int sys, int order, int cells, const CUtensorMap &tmap, const StageParams &p, cudaStream_t s);
+// the right-hand side from and to cell-major arrays p.in and p.out (primitive inviscid path;
+// 16-byte aligned rows): tmap is 2-D over p.in, (nx NV, ny), box (stage_aos_box, 1)
+int stage_aos_box(int sys, int order, int cells);
+cudaError_t launch_stage_rhs(int sys, int order, int cells, const CUtensorMap &tmap, const StageParams &p, cudaStream_t s);
+cudaError_t launch_stage_fast_rhs(int sys, int order, int cells, const CUtensorMap &tmap, const StageParams &p, cudaStream_t s);
 cudaError_t launch_stage_batch(int sys, int order, int cells, const StageParams *inst, const CUtensorMap *tmaps,
                                const int2 *work, int *sched, int blocks, cudaStream_t s);
 // the FP64 performance form (primitive path, HYPE_PREC_FP64_FAST): grid form, 64- or 128-column tiles

@@ -20,6 +20,16 @@ stage_kernel(const __grid_constant__ CUtensorMap tmap, const StageParams p)
     stage_tile<SYS, N, CELLS, false>(p, &tmap, blockIdx.x, p.run0 + (int)blockIdx.y, smem_raw);
 }
 
+// The right-hand side from and to the caller's cell-major arrays (tmap: p.in, 2-D, rows of
+// nx NV values)
+template <int SYS, int N, int CELLS>
+__global__ void __launch_bounds__(2 * CELLS, (StageKernel<SYS, N, CELLS>::MIN_BLOCKS))
+stage_rhs_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ RhsParams p)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    stage_tile<SYS, N, CELLS, false, false, false, true>(p, &tmap, blockIdx.x, p.run0 + (int)blockIdx.y, smem_raw);
+}
+
 // Persistent form: the block walks a list of (grid, tile) work items; every grid
 // has its own parameters, tensor map and device scalars.
 template <int SYS, int N, int CELLS>
@@ -56,8 +66,10 @@ stage_batch_kernel(const StageParams *__restrict__ inst, const CUtensorMap *__re
 struct StageEntry {
     const void *single;
     const void *batch;
+    const void *rhs;
     size_t smem;
     int threads;
+    int aos_box;   // elements of one part of a cell-major row's box
 };
 
 template <int SYS, int N, int CELLS>
@@ -65,7 +77,8 @@ static StageEntry entry_of()
 {
     return StageEntry{reinterpret_cast<const void *>(stage_kernel<SYS, N, CELLS>),
                       reinterpret_cast<const void *>(stage_batch_kernel<SYS, N, CELLS>),
-                      StageKernel<SYS, N, CELLS>::smem_bytes(), 2 * CELLS};
+                      reinterpret_cast<const void *>(stage_rhs_kernel<SYS, N, CELLS>), StageKernel<SYS, N, CELLS>::smem_bytes(),
+                      2 * CELLS, StageKernel<SYS, N, CELLS>::AOS_BOX};
 }
 
 template <int SYS, int CELLS>
@@ -102,6 +115,7 @@ cudaError_t stage_configure(int sys, int order, int cells)
     const StageEntry e = stage_entry(sys, order, cells);
     cudaError_t r = cudaFuncSetAttribute(e.single, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem);
     if (r != cudaSuccess) return r;
+    if ((r = cudaFuncSetAttribute(e.rhs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem)) != cudaSuccess) return r;
     return cudaFuncSetAttribute(e.batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem);
 }
 
@@ -131,6 +145,19 @@ cudaError_t launch_stage(int sys, int order, int cells, const CUtensorMap &tmap,
     void *args[] = {&tm, &pp};
     const unsigned gy = (unsigned)(p.run_count > 0 ? p.run_count : p.runs);
     return cudaLaunchKernel(e.single, dim3((unsigned)p.strips, gy, 1), dim3((unsigned)e.threads, 1, 1), args, e.smem, s);
+}
+
+int stage_aos_box(int sys, int order, int cells) { return stage_entry(sys, order, cells).aos_box; }
+
+cudaError_t launch_stage_rhs(int sys, int order, int cells, const CUtensorMap &tmap, const StageParams &p, cudaStream_t s)
+{
+    const StageEntry e = stage_entry(sys, order, cells);
+    CUtensorMap tm = tmap;
+    RhsParams pp;
+    static_cast<StageParams &>(pp) = p;
+    void *args[] = {&tm, &pp};
+    const unsigned gy = (unsigned)(p.run_count > 0 ? p.run_count : p.runs);
+    return cudaLaunchKernel(e.rhs, dim3((unsigned)p.strips, gy, 1), dim3((unsigned)e.threads, 1, 1), args, e.smem, s);
 }
 
 cudaError_t launch_stage_batch(int sys, int order, int cells, const StageParams *inst, const CUtensorMap *tmaps,

@@ -18,8 +18,17 @@ stage_fast_kernel(const __grid_constant__ CUtensorMap tmap, const StageParams p)
     stage_tile<SYS, N, CELLS, false, false, true>(p, &tmap, blockIdx.x, p.run0 + (int)blockIdx.y, smem_raw);
 }
 
+template <int SYS, int N, int CELLS>
+__global__ void __launch_bounds__(2 * CELLS, (StageKernel<SYS, N, CELLS>::MIN_BLOCKS))
+stage_fast_rhs_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ RhsParams p)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    stage_tile<SYS, N, CELLS, false, false, true, true>(p, &tmap, blockIdx.x, p.run0 + (int)blockIdx.y, smem_raw);
+}
+
 struct FastEntry {
     const void *fn;
+    const void *rhs;
     size_t smem;
     int threads;
 };
@@ -27,7 +36,8 @@ struct FastEntry {
 template <int SYS, int N, int CELLS>
 static FastEntry fast_of()
 {
-    return FastEntry{reinterpret_cast<const void *>(stage_fast_kernel<SYS, N, CELLS>), StageKernel<SYS, N, CELLS>::smem_bytes(),
+    return FastEntry{reinterpret_cast<const void *>(stage_fast_kernel<SYS, N, CELLS>),
+                     reinterpret_cast<const void *>(stage_fast_rhs_kernel<SYS, N, CELLS>), StageKernel<SYS, N, CELLS>::smem_bytes(),
                      2 * CELLS};
 }
 
@@ -60,7 +70,8 @@ static FastEntry fast_entry(int sys, int order, int cells)
 cudaError_t stage_fast_configure(int sys, int order, int cells)
 {
     const FastEntry e = fast_entry(sys, order, cells);
-    return cudaFuncSetAttribute(e.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem);
+    const cudaError_t r = cudaFuncSetAttribute(e.rhs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem);
+    return r != cudaSuccess ? r : cudaFuncSetAttribute(e.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem);
 }
 
 int stage_fast_blocks_per_sm(int sys, int order, int cells)
@@ -80,6 +91,17 @@ cudaError_t launch_stage_fast(int sys, int order, int cells, const CUtensorMap &
     void *args[] = {&tm, &pp};
     const unsigned gy = (unsigned)(p.run_count > 0 ? p.run_count : p.runs);
     return cudaLaunchKernel(e.fn, dim3((unsigned)p.strips, gy, 1), dim3((unsigned)e.threads, 1, 1), args, e.smem, s);
+}
+
+cudaError_t launch_stage_fast_rhs(int sys, int order, int cells, const CUtensorMap &tmap, const StageParams &p, cudaStream_t s)
+{
+    const FastEntry e = fast_entry(sys, order, cells);
+    CUtensorMap tm = tmap;
+    RhsParams pp;
+    static_cast<StageParams &>(pp) = p;
+    void *args[] = {&tm, &pp};
+    const unsigned gy = (unsigned)(p.run_count > 0 ? p.run_count : p.runs);
+    return cudaLaunchKernel(e.rhs, dim3((unsigned)p.strips, gy, 1), dim3((unsigned)e.threads, 1, 1), args, e.smem, s);
 }
 
 // fast_rcp and IEEE division of the same arguments, for the accuracy test

@@ -85,6 +85,14 @@ struct BatchParams {
     }
 };
 
+// The parameters of a right-hand side from and to cell-major arrays: what it never needs of the
+// stage combinations, slabs and blocks is a constant.
+struct RhsParams : StageParams {
+    static constexpr int mode = OUT_RHS, out_aos = 1, row_off = 0, col_off = 0;
+    static constexpr double kb = 1.0;
+    static constexpr double *push_lo = nullptr, *push_hi = nullptr;
+};
+
 template <int SYS, int N, int CELLS_>
 struct StageKernel {
     using S = System<SYS>;
@@ -97,6 +105,13 @@ struct StageKernel {
     static constexpr int NDOF = QD::NDOF;
     static constexpr int NC = NDOF - 1;                    // stored coefficients (k >= 1)
     static constexpr int ROW_ELEMS = BW * NV;
+    // cell-major input: a row's elements (those the stencils read, rounded to 128 bytes) in
+    // boxes of at most 256, each at a 128-byte offset; the last one ends with the row, over part
+    // of the one before
+    static constexpr int AOS_ELEMS = ROW_ELEMS / 16 * 16, AOS_PARTS = (AOS_ELEMS + 255) / 256;
+    static constexpr int AOS_BOX = (AOS_ELEMS / AOS_PARTS + 15) / 16 * 16;
+    static constexpr int aos_at(int k) { return k + 1 < AOS_PARTS ? k * AOS_BOX : AOS_ELEMS - AOS_BOX; }
+    static_assert(AOS_ELEMS >= (CELLS + 5) * NV && AOS_BOX <= 256 && AOS_PARTS * AOS_BOX >= AOS_ELEMS, "cell-major boxes cover the stencils");
     static constexpr int ROW_BYTES = ROW_ELEMS * 8;
     static constexpr int SLOT_STRIDE = ((ROW_BYTES + 127) / 128) * 128 / 8;   // doubles
     // components with a non-conservative product (the same ones on the conservative path)
@@ -319,7 +334,9 @@ __device__ __forceinline__ double riemann_gp(const E &eos, const double *VL, con
 // FAST: the FP64 performance form (primitive path only): FastSystem / ReconFast
 // of hype_physics_fast.cuh, in a translation unit built with FMA contraction;
 // reads the derived constants of p.eos (Eos::derive, filled by the host).
-template <int SYS, int N, int CELLS_, bool CONS, bool VISC = false, bool FAST = false, class P>
+// AOS: the input is the caller's cell-major array (p.in, 16-byte aligned rows) instead of
+// planes: a row is loaded as it is and laid out by component when it is converted.
+template <int SYS, int N, int CELLS_, bool CONS, bool VISC = false, bool FAST = false, bool AOS = false, class P>
 __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, int strip, int run, unsigned char *smem_raw)
 {
     static_assert(!(FAST && (CONS || VISC)), "the FP64 performance form covers the primitive inviscid path");
@@ -457,49 +474,54 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
         if (drained)
             for (int k = 0; k <= SLOTS + 1; ++k) mbar_inval(&bars[k]);
     };
-    // thread 0: issue the ring rows up to `last`
+    // thread 0: issue the ring rows up to `last`.  AOS: the prologue's rows land in the memory
+    // that the coefficients take later, the others in their ring slots
+    double *land_s = coef_s;
+    static_assert(!AOS || 5 * K::SLOT_STRIDE <= K::COEF_ELEMS + K::YT_ELEMS + K::CARRY_ELEMS, "the prologue's rows fit");
     auto issue_rows = [&](int last) {
         for (; next_issue <= min(last, row_hi) && (!p.skip_loads || next_issue < p.skip_loads_from); ++next_issue) {
             const int row = next_issue;
             const int src = map_axis(row, p.ny, bcB, bcT);
             uint64_t *bar = &bars[slot_of(row)];
-            mbar_expect_tx(bar, K::ROW_BYTES);
-            tma_load_3d(row_ptr(row), tmap, xs + p.col_off, src + p.row_off, 0, bar);   // the map starts col_off columns left of column 0, row_off rows below row 0
+            mbar_expect_tx(bar, AOS ? K::AOS_PARTS * K::AOS_BOX * 8 : K::ROW_BYTES);
+            if constexpr (AOS) {
+                double *to = row <= y0 + 1 ? land_s + (row - row_lo) * K::SLOT_STRIDE : row_ptr(row);
+#pragma unroll
+                for (int k = 0; k < K::AOS_PARTS; ++k) tma_load_2d(to + K::aos_at(k), tmap, xs * NV + K::aos_at(k), src, bar);
+            } else {
+                tma_load_3d(row_ptr(row), tmap, xs + p.col_off, src + p.row_off, 0, bar);   // the map starts col_off columns left of column 0, row_off rows below row 0
+            }
         }
     };
     auto wait_row = [&](int row) { return mbar_wait_bounded(&bars[slot_of(row)], (unsigned)(((row - row_lo) / SLOTS) & 1)); };
-    // Ghost columns of a loaded row fetch their conserved source values; needs a block
-    // barrier before convert_row overwrites the sources
-    auto fetch_ghosts = [&](int row) {
-        const int cc = 1 + t, g = xs + cc;
-        if (cc > owc + 6 || (g >= 0 && g < p.nx)) return true;
-        if (!wait_row(row)) return false;
-        double *rp = row_ptr(row);
-        const int gm = map_axis(g, p.nx, bcL, bcR);
-        if (gm == g) return true;   // a block's halo column, loaded in place
-        if (gm - xs >= 0 && gm - xs < BW) {
+    // Conserved values of column cc (1 .. owc+6, the ones the stencils read) of a loaded row;
+    // ghost columns take their source's
+    auto conserved = [&](int row, const double *raw, int cc, double *Q) {
+        const int g = xs + cc;
+        int col = cc;
+        if (g < 0 || g >= p.nx) {
+            const int gm = map_axis(g, p.nx, bcL, bcR);
+            col = gm - xs;
+            if (col < 0 || col >= (AOS ? K::AOS_ELEMS / NV : BW)) {   // the far side of a periodic axis
+                const int src = map_axis(row, p.ny, bcB, bcT);
 #pragma unroll
-            for (int c = 0; c < NV; ++c) rp[c * BW + cc] = rp[c * BW + (gm - xs)];
-        } else {
-            const int src = map_axis(row, p.ny, bcB, bcT);
-#pragma unroll
-            for (int c = 0; c < NV; ++c) rp[c * BW + cc] = p.in[(long long)c * p.plane + (long long)src * p.pitch + gm];
+                for (int c = 0; c < NV; ++c)
+                    Q[c] = AOS ? p.in[((long long)src * p.nx + gm) * NV + c] : p.in[(long long)c * p.plane + (long long)src * p.pitch + gm];
+                return;
+            }
         }
-        return true;
+#pragma unroll
+        for (int c = 0; c < NV; ++c) Q[c] = AOS ? raw[col * NV + c] : raw[c * BW + col];
     };
-    // Convert a loaded row in place, apply reflections and inlet values.  Columns
-    // cc = 1 .. owc+6 are the ones the stencils read
-    auto convert_row = [&](int row) {
-        const int cc = 1 + t;
-        if (cc > owc + 6) return;
+    // Primitive values of a column's conserved ones, reflections and inlet values applied, into
+    // its ring row
+    auto put_primitive = [&](int row, int cc, const double *Q) {
         double *rp = row_ptr(row);
         const bool yg = row < 0 || row >= p.ny;
         const bool yrefl = yg && ((row < 0 ? bcB : bcT) == BC_REFLECTIVE);
         const int g = xs + cc;
         const bool isg = g < 0 || g >= p.nx;
-        double Q[NV], V[NV];
-#pragma unroll
-        for (int c = 0; c < NV; ++c) Q[c] = rp[c * BW + cc];
+        double V[NV];
         if constexpr (CONS) {
 #pragma unroll
             for (int c = 0; c < NV; ++c) V[c] = Q[c];
@@ -540,15 +562,37 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
         issue_rows(y0 + 2);
     }
     {
+        const int width = owc + 6;   // converted columns of a row
         bool here = true;
         for (int row = row_lo; row <= y0 + 1; ++row) here = here && wait_row(row);
-        if (touches_x && here)
-            for (int row = row_lo; row <= y0 + 1; ++row) here = here && fetch_ghosts(row);
+        if (!AOS && touches_x && here) {   // ghost columns first: the conversion is in place
+            for (int k = t; k < 5 * width; k += K::NT) {
+                const int row = row_lo + k / width, cc = 1 + k % width, g = xs + cc;
+                if (g >= 0 && g < p.nx) continue;
+                double Q[NV], *rp = row_ptr(row);
+                conserved(row, rp, cc, Q);
+#pragma unroll
+                for (int c = 0; c < NV; ++c) rp[c * BW + cc] = Q[c];
+            }
+        }
         if (__syncthreads_or(!here)) {
             give_up(false, 0u);
             return;   // block-uniform exit; the caller's next barrier is block-uniform too
         }
-        for (; next_conv <= y0 + 1; ++next_conv) convert_row(next_conv);
+#pragma unroll 1
+        for (int k = t; k < 5 * width; k += K::NT) {
+            const int row = row_lo + k / width, cc = 1 + k % width;
+            double Q[NV];
+            if constexpr (AOS) {
+                conserved(row, land_s + (row - row_lo) * K::SLOT_STRIDE, cc, Q);
+            } else {
+                const double *rp = row_ptr(row);
+#pragma unroll
+                for (int c = 0; c < NV; ++c) Q[c] = rp[c * BW + cc];
+            }
+            put_primitive(row, cc, Q);
+        }
+        next_conv = y0 + 2;
     }
     __syncthreads();
 
@@ -850,7 +894,23 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
         }   // warp_active
 
         const bool conv = r + 3 <= row_hi;   // row r+3 is converted in this iteration
-        if (touches_x && conv) here = fetch_ghosts(r + 3) && here;
+        const int cc = 1 + t;
+        const bool conv_me = conv && cc <= owc + 6;
+        [[maybe_unused]] double Qn[NV];   // AOS: held across S1, after which the row changes its layout in place
+        if (conv_me) {
+            here = wait_row(r + 3) && here;
+            if constexpr (AOS) {
+                if (here) conserved(r + 3, row_ptr(r + 3), cc, Qn);
+            } else {
+                const int g = xs + cc;
+                if (here && (g < 0 || g >= p.nx)) {   // ghost columns before their sources are converted
+                    double Q[NV], *rp = row_ptr(r + 3);
+                    conserved(r + 3, rp, cc, Q);
+#pragma unroll
+                    for (int c = 0; c < NV; ++c) rp[c * BW + cc] = Q[c];
+                }
+            }
+        }
         // the loads of the next iteration: row r's input, and row r+4 into the slot of row r-2
         const bool load_orow = full_row && p.mode != OUT_RHS && (!p.skip_loads || r < p.skip_loads_from);
         auto issue_next = [&] {
@@ -862,12 +922,14 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
                 tma_load_3d(orow_s, tmap, xs + p.col_off, r + p.row_off, 0, &bars[SLOTS]);
             }
         };
-        // S1: every column's face values of row r visible, ghost columns fetched
+        // S1: every column's face values of row r visible, row r+3's ghost columns fetched
         if (__syncthreads_or(!here)) {
             give_up(finish_row && (!p.skip_loads || r - 1 < p.skip_loads_from), (unsigned)((r - y0 - 1) & 1));
             return;   // block-uniform exit
         }
         if constexpr (!VISC) issue_next();
+        if (AOS && conv_me) put_primitive(r + 3, cc, Qn);
+        if (conv) ++next_conv;
 
         // ---------------- E. x-face at the left of column i: Gauss point q ----------
         double Fown[(NV + 1) / 2], Down[(NV + 1) / 2];   // components 2 j + h
@@ -928,18 +990,14 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
                 }
             });
         }
-        bool late = false;
-        if (conv) {
-            late = !wait_row(r + 3);
-            if (!late) convert_row(r + 3);
-            ++next_conv;
+        if (!AOS && conv_me) {   // beside the x-face problems: 2 % of a 256^2 step against right after S1
+            double Q[NV];
+            const double *rp = row_ptr(r + 3);
+#pragma unroll
+            for (int c = 0; c < NV; ++c) Q[c] = rp[c * BW + cc];
+            put_primitive(r + 3, cc, Q);
         }
-        // S2: the x-face fluxes and prim rows r-1 .. r+3 ready
-        if (__syncthreads_or(late)) {
-            --next_conv;
-            give_up(load_orow && !VISC, (unsigned)((r - y0) & 1));
-            return;   // block-uniform exit
-        }
+        __syncthreads();   // S2: the x-face fluxes and prim rows r-1 .. r+3 ready
         if constexpr (VISC) issue_next();
         if (owned && full_row) {
             static_for<(NV + 1) / 2>([&](auto jj) {

@@ -158,3 +158,33 @@ def test_bands_of_host_calls(hp, orc, nx, ny, bc):
         s.set_state(U)
         s.begin(0.0, 1e30, 2)
         assert s.advance_host(U, out, 1) == st and out.tobytes() == state.tobytes()
+
+
+@pytest.mark.parametrize("system", ["kapila", "bn", "euler"])
+@pytest.mark.parametrize("order", [0, 1, 2, 3])
+@pytest.mark.parametrize("nx,ny", [(3, 3), (64, 5), (65, 7), (126, 4), (131, 9), (260, 6)])
+@pytest.mark.parametrize("ends", ["walls", "periodic"])
+def test_device_calls_read_cell_major_arrays(hp, orc, system, order, nx, ny, ends):
+    """hype_rhs_prim_device loads the caller's cell-major rows by TMA where they start on 16-byte
+    boundaries (an odd Baer-Nunziato width does not, nor does an array moved by 8 bytes) and
+    converts the array to planes elsewhere: the oracle's bits either way."""
+    import torch
+    kind, eos, nv = {"kapila": ("bubble", cases.KAPILA_EOS, 6), "bn": ("discs", cases.KAPILA_EOS, 9),
+                     "euler": ("quadrants", cases.EULER_EOS, 4)}[system]
+    lr, bt = ((O.REFLECTIVE, O.TRANSMISSIVE), (O.TRANSMISSIVE, O.REFLECTIVE)) if ends == "walls" else ((O.PERIODIC,) * 2,) * 2
+    cfg = O.Config(system={"kapila": O.KAPILA, "bn": O.BN, "euler": O.EULER}[system], order=order, nx=nx, ny=ny, bc_left=lr[0],
+                   bc_right=lr[1], bc_bottom=bt[0], bc_top=bt[1], **eos)
+    if system == "bn":
+        cfg.bn_fixed_p2 = 1
+    U = cases.state(cfg, kind, 7)
+    Ro, dto, sto = orc.rhs(cfg, U)
+    room = torch.zeros(U.size + 1, dtype=torch.float64, device="cuda")
+    with hp.Solver(cases.to_pkg(cfg)) as s:
+        for shift in (0, 1):
+            dU, dR = room[shift:shift + U.size], torch.full((U.size,), np.nan, dtype=torch.float64, device="cuda")
+            dU.copy_(torch.from_numpy(U))
+            torch.cuda.synchronize()
+            dt, st = s.rhs_function_prim_device(0.0, dU.data_ptr(), dR.data_ptr())
+            assert (st != hp.OK) == (sto != 0)
+            if sto == 0:
+                assert dR.cpu().numpy().tobytes() == Ro.tobytes() and dt == dto
