@@ -528,7 +528,7 @@ static cudaError_t enqueue_kind_stage(hype_batch *b, int id, int st, cudaStream_
     const PlanStage &q = k.plan[st];
     if (k.mixed) return launch_mixed_batch(k.system, k.cells, k.dMParams + st * M, k.dMMaps + q.in * M, l.dWork, l.dSched, blocks, s);
     if (k.path >= 0) return launch_path_batch(k.path, k.system, k.order, k.dParams + st * M, k.dMaps + q.in * M, l.dWork, l.dSched, blocks, s);
-    return launch_stage_batch(k.system, k.order, k.cells, k.dParams + st * M, k.dMaps + q.in * M, l.dWork, l.dSched, blocks, s);
+    return launch_stage_batch(k.system, k.order, k.cells, q.mode, k.dParams + st * M, k.dMaps + q.in * M, l.dWork, l.dSched, blocks, s);
 }
 
 // One batch step of a kind: sub-step j steps the members with substeps > j.

@@ -104,7 +104,7 @@ cudaError_t launch_stage(int sys, int order, int cells, const CUtensorMap &tmap,
 int stage_aos_box(int sys, int order, int cells);
 cudaError_t launch_stage_rhs(int sys, int order, int cells, const CUtensorMap &tmap, const StageParams &p, cudaStream_t s);
 cudaError_t launch_stage_fast_rhs(int sys, int order, int cells, const CUtensorMap &tmap, const StageParams &p, cudaStream_t s);
-cudaError_t launch_stage_batch(int sys, int order, int cells, const StageParams *inst, const CUtensorMap *tmaps,
+cudaError_t launch_stage_batch(int sys, int order, int cells, int mode, const StageParams *inst, const CUtensorMap *tmaps,
                                const int2 *work, int *sched, int blocks, cudaStream_t s);
 // the FP64 performance form (primitive path, HYPE_PREC_FP64_FAST): grid form, 64- or 128-column tiles
 cudaError_t stage_fast_configure(int sys, int order, int cells);

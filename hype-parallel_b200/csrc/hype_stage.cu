@@ -20,6 +20,14 @@ stage_kernel(const __grid_constant__ CUtensorMap tmap, const StageParams p)
     stage_tile<SYS, N, CELLS, false>(p, &tmap, blockIdx.x, p.run0 + (int)blockIdx.y, smem_raw);
 }
 
+template <int SYS, int N, int CELLS, int MODE>
+__global__ void __launch_bounds__(2 * CELLS, (StageKernel<SYS, N, CELLS>::MIN_BLOCKS))
+stage_mode_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ ModeParams<MODE> p)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    stage_tile<SYS, N, CELLS, false>(p, &tmap, blockIdx.x, p.run0 + (int)blockIdx.y, smem_raw);
+}
+
 // The right-hand side from and to the caller's cell-major arrays (tmap: p.in, 2-D, rows of
 // nx NV values)
 template <int SYS, int N, int CELLS>
@@ -32,7 +40,7 @@ stage_rhs_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
 
 // Persistent form: the block walks a list of (grid, tile) work items; every grid
 // has its own parameters, tensor map and device scalars.
-template <int SYS, int N, int CELLS>
+template <int SYS, int N, int CELLS, int MODE>
 __global__ void __launch_bounds__(2 * CELLS, (StageKernel<SYS, N, CELLS>::MIN_BLOCKS))
 stage_batch_kernel(const StageParams *__restrict__ inst, const CUtensorMap *__restrict__ tmaps,
                    const int2 *__restrict__ work, int *__restrict__ sched)
@@ -41,7 +49,7 @@ stage_batch_kernel(const StageParams *__restrict__ inst, const CUtensorMap *__re
     __shared__ int item_s;
     // the item's parameters live in shared memory: re-read after every barrier
     // of the tile instead of pinning registers for the whole tile
-    __shared__ BatchParams p_s;
+    __shared__ BatchParamsOf<MODE> p_s;
     const int nwork = sched[0];
     const DevScalars *last = nullptr;
     for (;;) {
@@ -65,20 +73,35 @@ stage_batch_kernel(const StageParams *__restrict__ inst, const CUtensorMap *__re
 // ---------------------------------------------------------------------------
 struct StageEntry {
     const void *single;
-    const void *batch;
     const void *rhs;
+    const void *axpy, *mix;                // of the whole grid, by mode
+    const void *batch_axpy, *batch_mix, *batch_rk;   // batch_rk: N = 3's fifth stage, else null
     size_t smem;
     int threads;
     int aos_box;   // elements of one part of a cell-major row's box
+    int mix_mode;
 };
 
 template <int SYS, int N, int CELLS>
 static StageEntry entry_of()
 {
-    return StageEntry{reinterpret_cast<const void *>(stage_kernel<SYS, N, CELLS>),
-                      reinterpret_cast<const void *>(stage_batch_kernel<SYS, N, CELLS>),
-                      reinterpret_cast<const void *>(stage_rhs_kernel<SYS, N, CELLS>), StageKernel<SYS, N, CELLS>::smem_bytes(),
-                      2 * CELLS, StageKernel<SYS, N, CELLS>::AOS_BOX};
+    using K = StageKernel<SYS, N, CELLS>;
+    auto fn = [](auto *f) { return reinterpret_cast<const void *>(f); };
+    StageEntry e{};
+    e.single = fn(stage_kernel<SYS, N, CELLS>);
+    e.rhs = fn(stage_rhs_kernel<SYS, N, CELLS>);
+    e.axpy = fn(stage_mode_kernel<SYS, N, CELLS, OUT_AXPY>);
+    e.batch_axpy = fn(stage_batch_kernel<SYS, N, CELLS, OUT_AXPY>);
+    if constexpr (N > 0) {
+        e.mix = fn(stage_mode_kernel<SYS, N, CELLS, MIX_MODE<N>>);
+        e.batch_mix = fn(stage_batch_kernel<SYS, N, CELLS, MIX_MODE<N>>);
+    }
+    if constexpr (N == 3) e.batch_rk = fn(stage_batch_kernel<SYS, N, CELLS, OUT_RK104_5>);
+    e.smem = K::smem_bytes();
+    e.threads = 2 * CELLS;
+    e.aos_box = K::AOS_BOX;
+    e.mix_mode = MIX_MODE<N>;
+    return e;
 }
 
 template <int SYS, int CELLS>
@@ -113,10 +136,11 @@ int stage_threads(int cells) { return 2 * cells; }
 cudaError_t stage_configure(int sys, int order, int cells)
 {
     const StageEntry e = stage_entry(sys, order, cells);
-    cudaError_t r = cudaFuncSetAttribute(e.single, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem);
-    if (r != cudaSuccess) return r;
-    if ((r = cudaFuncSetAttribute(e.rhs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem)) != cudaSuccess) return r;
-    return cudaFuncSetAttribute(e.batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem);
+    for (const void *f : {e.single, e.rhs, e.axpy, e.mix, e.batch_axpy, e.batch_mix, e.batch_rk}) {
+        const cudaError_t r = f ? cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem) : cudaSuccess;
+        if (r != cudaSuccess) return r;
+    }
+    return cudaSuccess;
 }
 
 int stage_blocks_per_sm(int sys, int order, int cells)
@@ -133,7 +157,7 @@ int stage_batch_blocks_per_sm(int sys, int order, int cells)
     const StageEntry e = stage_entry(sys, order, cells);
     int nb = 0;
     if (stage_configure(sys, order, cells) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, e.batch, e.threads, e.smem) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, e.batch_axpy, e.threads, e.smem) != cudaSuccess) return 0;
     return nb;
 }
 
@@ -144,7 +168,9 @@ cudaError_t launch_stage(int sys, int order, int cells, const CUtensorMap &tmap,
     StageParams pp = p;
     void *args[] = {&tm, &pp};
     const unsigned gy = (unsigned)(p.run_count > 0 ? p.run_count : p.runs);
-    return cudaLaunchKernel(e.single, dim3((unsigned)p.strips, gy, 1), dim3((unsigned)e.threads, 1, 1), args, e.smem, s);
+    const bool whole = !p.out_aos && !p.row_off && !p.col_off && !p.push_lo && !p.push_hi;
+    const void *f = whole && p.mode == OUT_AXPY ? e.axpy : whole && e.mix && p.mode == e.mix_mode ? e.mix : e.single;
+    return cudaLaunchKernel(f, dim3((unsigned)p.strips, gy, 1), dim3((unsigned)e.threads, 1, 1), args, e.smem, s);
 }
 
 int stage_aos_box(int sys, int order, int cells) { return stage_entry(sys, order, cells).aos_box; }
@@ -160,12 +186,14 @@ cudaError_t launch_stage_rhs(int sys, int order, int cells, const CUtensorMap &t
     return cudaLaunchKernel(e.rhs, dim3((unsigned)p.strips, gy, 1), dim3((unsigned)e.threads, 1, 1), args, e.smem, s);
 }
 
-cudaError_t launch_stage_batch(int sys, int order, int cells, const StageParams *inst, const CUtensorMap *tmaps,
+cudaError_t launch_stage_batch(int sys, int order, int cells, int mode, const StageParams *inst, const CUtensorMap *tmaps,
                                const int2 *work, int *sched, int blocks, cudaStream_t s)
 {
     const StageEntry e = stage_entry(sys, order, cells);
     void *args[] = {&inst, &tmaps, &work, &sched};
-    return cudaLaunchKernel(e.batch, dim3((unsigned)blocks, 1, 1), dim3((unsigned)e.threads, 1, 1), args, e.smem, s);
+    const void *f = mode == OUT_AXPY ? e.batch_axpy : mode == OUT_RK104_5 ? e.batch_rk : mode == e.mix_mode ? e.batch_mix : nullptr;
+    if (!f) return cudaErrorInvalidValue;
+    return cudaLaunchKernel(f, dim3((unsigned)blocks, 1, 1), dim3((unsigned)e.threads, 1, 1), args, e.smem, s);
 }
 
 }  // namespace hype

@@ -26,9 +26,19 @@ stage_fast_rhs_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_con
     stage_tile<SYS, N, CELLS, false, false, true, true>(p, &tmap, blockIdx.x, p.run0 + (int)blockIdx.y, smem_raw);
 }
 
+template <int SYS, int N, int CELLS, int MODE>
+__global__ void __launch_bounds__(2 * CELLS, (StageKernel<SYS, N, CELLS>::MIN_BLOCKS))
+stage_fast_mode_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ ModeParams<MODE> p)
+{
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    stage_tile<SYS, N, CELLS, false, false, true>(p, &tmap, blockIdx.x, p.run0 + (int)blockIdx.y, smem_raw);
+}
+
 struct FastEntry {
     const void *fn;
     const void *rhs;
+    const void *axpy, *mix;   // of the whole grid, by mode
+    int mix_mode;
     size_t smem;
     int threads;
 };
@@ -36,9 +46,16 @@ struct FastEntry {
 template <int SYS, int N, int CELLS>
 static FastEntry fast_of()
 {
-    return FastEntry{reinterpret_cast<const void *>(stage_fast_kernel<SYS, N, CELLS>),
-                     reinterpret_cast<const void *>(stage_fast_rhs_kernel<SYS, N, CELLS>), StageKernel<SYS, N, CELLS>::smem_bytes(),
-                     2 * CELLS};
+    auto fn = [](auto *f) { return reinterpret_cast<const void *>(f); };
+    FastEntry e{};
+    e.fn = fn(stage_fast_kernel<SYS, N, CELLS>);
+    e.rhs = fn(stage_fast_rhs_kernel<SYS, N, CELLS>);
+    e.axpy = fn(stage_fast_mode_kernel<SYS, N, CELLS, OUT_AXPY>);
+    if constexpr (N > 0) e.mix = fn(stage_fast_mode_kernel<SYS, N, CELLS, MIX_MODE<N>>);
+    e.mix_mode = MIX_MODE<N>;
+    e.smem = StageKernel<SYS, N, CELLS>::smem_bytes();
+    e.threads = 2 * CELLS;
+    return e;
 }
 
 template <int SYS, int CELLS>
@@ -70,8 +87,11 @@ static FastEntry fast_entry(int sys, int order, int cells)
 cudaError_t stage_fast_configure(int sys, int order, int cells)
 {
     const FastEntry e = fast_entry(sys, order, cells);
-    const cudaError_t r = cudaFuncSetAttribute(e.rhs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem);
-    return r != cudaSuccess ? r : cudaFuncSetAttribute(e.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem);
+    for (const void *f : {e.fn, e.rhs, e.axpy, e.mix}) {
+        const cudaError_t r = f ? cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem) : cudaSuccess;
+        if (r != cudaSuccess) return r;
+    }
+    return cudaSuccess;
 }
 
 int stage_fast_blocks_per_sm(int sys, int order, int cells)
@@ -90,7 +110,9 @@ cudaError_t launch_stage_fast(int sys, int order, int cells, const CUtensorMap &
     StageParams pp = p;
     void *args[] = {&tm, &pp};
     const unsigned gy = (unsigned)(p.run_count > 0 ? p.run_count : p.runs);
-    return cudaLaunchKernel(e.fn, dim3((unsigned)p.strips, gy, 1), dim3((unsigned)e.threads, 1, 1), args, e.smem, s);
+    const bool whole = !p.out_aos && !p.row_off && !p.col_off && !p.push_lo && !p.push_hi;
+    const void *f = whole && p.mode == OUT_AXPY ? e.axpy : whole && e.mix && p.mode == e.mix_mode ? e.mix : e.fn;
+    return cudaLaunchKernel(f, dim3((unsigned)p.strips, gy, 1), dim3((unsigned)e.threads, 1, 1), args, e.smem, s);
 }
 
 cudaError_t launch_stage_fast_rhs(int sys, int order, int cells, const CUtensorMap &tmap, const StageParams &p, cudaStream_t s)

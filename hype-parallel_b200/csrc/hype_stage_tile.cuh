@@ -60,8 +60,10 @@ namespace hype {
 // work item.  What a batch instance never has (slab and block offsets, interleaved output,
 // a run range, the test hook) is a constant: the tile drops its code, and the struct leaves
 // room for two blocks per SM.
-struct BatchParams {
-    int nx, ny, pitch, strips, runs, mode, reduce_smax;
+template <int MODE>
+struct BatchParamsOf {
+    static constexpr int mode = MODE;
+    int nx, ny, pitch, strips, runs, reduce_smax;
     int bc[4];
     long long plane;
     EosBase eos;
@@ -76,12 +78,21 @@ struct BatchParams {
     __device__ __forceinline__ void load(const StageParams &p, int refine)
     {
         nx = p.nx; ny = p.ny; pitch = p.pitch; strips = p.strips; runs = p.runs * refine;
-        mode = p.mode; reduce_smax = p.reduce_smax;
+        reduce_smax = p.reduce_smax;
         for (int k = 0; k < 4; ++k) bc[k] = p.bc[k];
         plane = p.plane;
         eos = p.eos;
         r1_h = p.r1_h; ka = p.ka; kb = p.kb; kc = p.kc; mu1 = p.mu1; mu2 = p.mu2;
         in = p.in; xn = p.xn; inlet = p.inlet; out = p.out; out2 = p.out2; sc = p.sc;
+    }
+};
+
+struct BatchParams : BatchParamsOf<OUT_AXPY> {   // the mode at run time (conservative and viscous kinds)
+    int mode;
+    __device__ __forceinline__ void load(const StageParams &p, int refine)
+    {
+        BatchParamsOf<OUT_AXPY>::load(p, refine);
+        mode = p.mode;
     }
 };
 
@@ -92,6 +103,19 @@ struct RhsParams : StageParams {
     static constexpr double kb = 1.0;
     static constexpr double *push_lo = nullptr, *push_hi = nullptr;
 };
+
+// The parameters of a stage combination of a whole grid (no slab, block or interleaved output).
+// The kernels of the time loop know their mode: 10 steps of 256^2 Kapila 2.56 -> 2.42 ms, a
+// 2048^2 stage 1.50 -> 1.45.
+template <int MODE>
+struct ModeParams : StageParams {
+    static constexpr int mode = MODE, out_aos = 0, row_off = 0, col_off = 0;
+    static constexpr double *push_lo = nullptr, *push_hi = nullptr;
+};
+
+// The SSP plans (ssp_plan) add OUT_AXPY stages, one that mixes in u^n, and for N = 3 a fifth one
+// of its own
+template <int N> constexpr int MIX_MODE = N == 2 ? OUT_ZXS : OUT_ZSX;
 
 template <int SYS, int N, int CELLS_>
 struct StageKernel {
