@@ -55,6 +55,7 @@ struct MixedKernel {
 struct MixedEos {
     double g1, g2, pi1, pi2, G1m1, G2m1, c1, c2, inv_G12;
     float g1f, g2f;
+    bool quick;   // pad_quick's accept holds for these constants
     __device__ __forceinline__ explicit MixedEos(const Eos &e)
     {
         g1 = e.g1; g2 = e.g2; pi1 = e.pi1; pi2 = e.pi2;
@@ -62,6 +63,7 @@ struct MixedEos {
         c1 = g1 * pi1 * G2m1; c2 = g2 * pi2 * G1m1;
         inv_G12 = 1.0 / (G1m1 * G2m1);
         g1f = (float)g1; g2f = (float)g2;
+        quick = g1 >= 1.0 && g1 <= 1024.0 && g2 >= 1.0 && g2 <= 1024.0 && pi1 >= 0.0 && pi1 <= 0x1p60 && pi2 >= 0.0 && pi2 <= 0x1p60;
     }
 };
 
@@ -102,6 +104,16 @@ __device__ __forceinline__ bool pad_mixed(const MixedEos &e, const PrimM &V)
     if (asq < 1.0e-12f) return false;
     if (V.a < 0.0 || V.a > 1.0) return false;
     return true;
+}
+
+// Whether pad_mixed is plainly true, by exponents only (almost every point; the rest takes
+// pad_mixed): rho_k in [2^-20, 2^16), p in [2^-10, 2^60), alpha_1 in [0, 1) and the constants of
+// `quick` give rho >= 2^-21 and a^2 >= 2^-10 / 2^16 up to FP32 rounding, far above both floors;
+// the mixture's denominator stays below 2^90, within __fdividef's range
+__device__ __forceinline__ bool pad_quick(const PrimM &V)
+{
+    auto in = [](float r) { return __float_as_uint(r) - (107u << 23) < (36u << 23); };
+    return in(V.r1) && in(V.r2) && exp_in<-10, 60>(V.p) && frac_in(V.a);
 }
 
 // K = a1 a2 (rho2 a2^2 - rho1 a1^2) / (a1 rho2 a2^2 + a2 rho1 a1^2)  (kapila_5eqn.c:432-434)
@@ -226,6 +238,16 @@ __device__ __forceinline__ void mixed_tile(const MixedParams &p, const MixedMaps
         return [v, p5](int k1) -> float { return k1 == 0 ? v.x : k1 == 1 ? v.y : k1 == 2 ? v.z : k1 == 3 ? v.w : *p5; };
     };
 
+    // Mean of a face's two Gauss point fluxes, components 2 j + h: each half sends the other the
+    // component it needs, components 0..3 as the FP32 values they are
+    auto pair_mean = [&](const double *F, double *mean) {
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const double mine = h ? F[2 * j + 1] : F[2 * j], give = h ? F[2 * j] : F[2 * j + 1];
+            const double got = j < 2 ? (double)__shfl_xor_sync(FULL, (float)give, 1) : __shfl_xor_sync(FULL, give, 1);
+            mean[j] = 0.5 * mine + 0.5 * got;
+        }
+    };
     float smax_loc = 0.0f;
     bool bad = false;
     unsigned bad_cell = 0xffffffffu;
@@ -384,7 +406,7 @@ __device__ __forceinline__ void mixed_tile(const MixedParams &p, const MixedMaps
                 constexpr int s0 = decltype(sq)::value, s1 = 4 + s0;
                 if (!ok) return;
                 const PrimM V = prim_at(m, PhiNode<2, s0>{}, PhiNode<2, s1>{});
-                ok = pad_mixed(e, V);
+                ok = (e.quick && pad_quick(V)) || pad_mixed(e, V);
             });
         }
         {
@@ -432,9 +454,8 @@ __device__ __forceinline__ void mixed_tile(const MixedParams &p, const MixedMaps
 #pragma unroll
                 for (int c = 0; c < NV; ++c) Fq[c] = 0.0;
             }
-            double G[NV];
-#pragma unroll
-            for (int c = 0; c < NV; ++c) G[c] = 0.5 * Fq[c] + 0.5 * __shfl_xor_sync(FULL, Fq[c], 1);
+            double G[3];   // of components 2 j + h
+            pair_mean(Fq, G);
             const double E5 = 0.5 * (double)Dq + 0.5 * (double)__shfl_xor_sync(FULL, Dq, 1);
             if (doit) {
                 if (r > y0) {
@@ -444,7 +465,7 @@ __device__ __forceinline__ void mixed_tile(const MixedParams &p, const MixedMaps
 #pragma unroll
                     for (int j = 0; j < 3; ++j) {
                         const int c = 2 * j + h;
-                        double Y = (h ? G[2 * j + 1] : G[2 * j]) - carry[(6 + c) * CELLS + m];
+                        double Y = G[j] - carry[(6 + c) * CELLS + m];
                         if (c == 5) Y += 0.5 * (E5 + carry[12 * CELLS + m]);
                         const double rhs = (c == 5 ? carry[13 * CELLS + m] : 0.0) + (carry[c * CELLS + m] - r1_h * Y);
                         if (p.mode == OUT_RHS) {
@@ -477,7 +498,7 @@ __device__ __forceinline__ void mixed_tile(const MixedParams &p, const MixedMaps
                     }
                 }
 #pragma unroll
-                for (int j = 0; j < 3; ++j) carry[(6 + 2 * j + h) * CELLS + m] = h ? G[2 * j + 1] : G[2 * j];
+                for (int j = 0; j < 3; ++j) carry[(6 + 2 * j + h) * CELLS + m] = G[j];
                 if (h == 1) carry[12 * CELLS + m] = E5;
             }
         }
@@ -518,7 +539,7 @@ __device__ __forceinline__ void mixed_tile(const MixedParams &p, const MixedMaps
         __syncthreads();   // S2: every column's coefficients of row r visible
 
         // ---------------- F. x-face at the left of column i, Gauss point q
-        double Fx[NV];
+        double Fx[3];   // of components 2 j + h
         double Dx5;
         {
             double Fq[NV];
@@ -533,14 +554,13 @@ __device__ __forceinline__ void mixed_tile(const MixedParams &p, const MixedMaps
 #pragma unroll
                 for (int c = 0; c < NV; ++c) Fq[c] = 0.0;
             }
-#pragma unroll
-            for (int c = 0; c < NV; ++c) Fx[c] = 0.5 * Fq[c] + 0.5 * __shfl_xor_sync(FULL, Fq[c], 1);
+            pair_mean(Fq, Fx);
             Dx5 = 0.5 * (double)Dq + 0.5 * (double)__shfl_xor_sync(FULL, Dq, 1);
         }
         __syncthreads();   // S3
         if (xface && full_row) {
 #pragma unroll
-            for (int j = 0; j < 3; ++j) exch[(2 * j + h) * CELLS + m] = h ? Fx[2 * j + 1] : Fx[2 * j];
+            for (int j = 0; j < 3; ++j) exch[(2 * j + h) * CELLS + m] = Fx[j];
             if (h == 1) exch[6 * CELLS + m] = Dx5;
         }
         __syncthreads();   // S4
@@ -548,7 +568,7 @@ __device__ __forceinline__ void mixed_tile(const MixedParams &p, const MixedMaps
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
                 const int c = 2 * j + h;
-                double X = exch[c * CELLS + m + 1] - (h ? Fx[2 * j + 1] : Fx[2 * j]);
+                double X = exch[c * CELLS + m + 1] - Fx[j];
                 if (c == 5) X += 0.5 * (exch[6 * CELLS + m + 1] + Dx5);
                 carry[c * CELLS + m] = -r1_h * X;
             }
