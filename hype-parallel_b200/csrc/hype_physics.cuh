@@ -177,6 +177,8 @@ struct IeeeDiv {
     __device__ __forceinline__ void pos(double) const {}
     __device__ __forceinline__ void frac(double) const {}
     __device__ __forceinline__ void num(double) const {}
+    __device__ __forceinline__ void mag(double) const {}
+    __device__ __forceinline__ void den(double) const {}
 };
 struct CrDiv {
     unsigned lo = 0;
@@ -187,6 +189,10 @@ struct CrDiv {
     __device__ __forceinline__ double quot(double a, double b, double y) const { return div_rn(a, b, y); }
     __device__ __forceinline__ void pos(double x) { in = in && exp_in<-100, 100>(x); }    // a density, a p + P_inf
     __device__ __forceinline__ void frac(double x) { in = in && exp_in<-100, 0>(x); }     // a volume fraction
+    // of any sign: a p + P_inf (negative in the trace gas of a liquid under tension), a divisor that
+    // may cancel
+    __device__ __forceinline__ void mag(double x) { in = in && exp_in<-100, 100>(fabs(x)); }
+    __device__ __forceinline__ void den(double x) { in = in && exp_in<-300, 300>(fabs(x)); }
     __device__ __forceinline__ void num(double x)                                          // a numerator of any sign: 0 or |x| >= 2^-300
     {
         const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
@@ -274,10 +280,12 @@ template <> struct System<SYS_KAPILA> {
         double ei = dv.by_const(p * (alpha_1 * G2m1 + alpha_2 * G1m1) + alpha_1 * e.g1 * e.pi1 * G2m1 + alpha_2 * e.g2 * e.pi2 * G1m1, G1m1 * G2m1, e.r_g12);
         double E = ei + 0.5 * rho * (u * u + v * v);
         double un = u * nx + v * ny;
-        dv.pos(rho_1); dv.pos(rho_2); dv.pos(p + e.pi1); dv.pos(p + e.pi2); dv.frac(alpha_1);
+        dv.pos(rho_1); dv.pos(rho_2); dv.mag(p + e.pi1); dv.mag(p + e.pi2); dv.mag(alpha_1);
         double a1_sq = dv(e.g1 * (p + e.pi1), rho_1);
         double a2_sq = dv(e.g2 * (p + e.pi2), rho_2);
-        double a_sq = dv(rho_1 * a1_sq * rho_2 * a2_sq, rho * (alpha_2 * rho_1 * a1_sq + alpha_1 * rho_2 * a2_sq));
+        const double a_den = rho * (alpha_2 * rho_1 * a1_sq + alpha_1 * rho_2 * a2_sq);
+        dv.den(a_den);
+        double a_sq = dv(rho_1 * a1_sq * rho_2 * a2_sq, a_den);
         bad |= (a_sq < PRS_FLOOR);
         F[0] = alpha_1 * rho_1 * un;
         F[1] = alpha_2 * rho_2 * un;
@@ -296,10 +304,12 @@ template <> struct System<SYS_KAPILA> {
         double rho_1 = V[0], rho_2 = V[1], u = V[2], v = V[3], p = V[4];
         double phi_x = gx[5], phi_y = gy[5];
         double u_x = gx[2], v_y = gy[3];
-        dv.pos(rho_1); dv.pos(rho_2); dv.pos(p + e.pi1); dv.pos(p + e.pi2); dv.frac(alpha_1);
+        dv.pos(rho_1); dv.pos(rho_2); dv.mag(p + e.pi1); dv.mag(p + e.pi2); dv.mag(alpha_1);
         double a_1_sq = dv(e.g1 * (p + e.pi1), rho_1);
         double a_2_sq = dv(e.g2 * (p + e.pi2), rho_2);
-        double K = dv(alpha_1 * alpha_2 * (rho_2 * a_2_sq - rho_1 * a_1_sq), alpha_1 * rho_2 * a_2_sq + alpha_2 * rho_1 * a_1_sq);
+        const double k_den = alpha_1 * rho_2 * a_2_sq + alpha_2 * rho_1 * a_1_sq;
+        dv.den(k_den);
+        double K = dv(alpha_1 * alpha_2 * (rho_2 * a_2_sq - rho_1 * a_1_sq), k_den);
         B[0] = 0.0; B[1] = 0.0; B[2] = 0.0; B[3] = 0.0; B[4] = 0.0;
         B[5] = u * phi_x + v * phi_y - K * (u_x + v_y);
     }
@@ -322,21 +332,30 @@ template <> struct System<SYS_KAPILA> {
         else if constexpr (C == 5) return frac_in(v);
         else return true;
     }
-    // kapila_5eqn.c:450-479
-    __device__ __forceinline__ static bool pad(const EosBase &e, const double *V)
+    // kapila_5eqn.c:450-479 (every test rejects: the one without a division first)
+    template <class Dv>
+    __device__ __forceinline__ static bool pad_dv(const EosBase &e, Dv &dv, const double *V)
     {
         double alpha_1 = V[5];
+        if (alpha_1 < 0.0 || alpha_1 > 1.0) return false;
         double alpha_2 = 1.0 - alpha_1;
         double rho_1 = V[0], rho_2 = V[1];
         double rho = alpha_1 * rho_1 + alpha_2 * rho_2;
         double p = V[4];
-        double a1_sq = e.g1 * (p + e.pi1) / rho_1;
-        double a2_sq = e.g2 * (p + e.pi2) / rho_2;
-        double a_sq = (rho_1 * a1_sq * rho_2 * a2_sq) / (rho * (alpha_2 * rho_1 * a1_sq + alpha_1 * rho_2 * a2_sq));
+        dv.pos(rho_1); dv.pos(rho_2); dv.mag(p + e.pi1); dv.mag(p + e.pi2); dv.mag(alpha_1);
+        double a1_sq = dv(e.g1 * (p + e.pi1), rho_1);
+        double a2_sq = dv(e.g2 * (p + e.pi2), rho_2);
+        const double a_den = rho * (alpha_2 * rho_1 * a1_sq + alpha_1 * rho_2 * a2_sq);
+        dv.den(a_den);
+        double a_sq = dv(rho_1 * a1_sq * rho_2 * a2_sq, a_den);
         if (rho < RHO_FLOOR) return false;
         if (a_sq < PRS_FLOOR) return false;
-        if (alpha_1 < 0.0 || alpha_1 > 1.0) return false;
         return true;
+    }
+    __device__ __forceinline__ static bool pad(const EosBase &e, const double *V)
+    {
+        IeeeDiv dv;
+        return pad_dv(e, dv, V);
     }
 
     // ---- viscous fluxes (the VISCOUS build, hype.h:36) ----

@@ -752,7 +752,13 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
                     double V[NV];
 #pragma unroll
                     for (int c = 0; c < NV; ++c) V[c] = f == 0 ? VR[c] : f < 3 ? coef_s[cidx(2 * q + f - 1, c, m)] : yt_up[c * CELLS];
-                    ok = CONS ? S::pad_cons(eos, V) : S::pad(eos, V);
+                    if constexpr (SYS == SYS_KAPILA && !CONS && !FAST) {   // whole regions of a liquid under tension come here
+                        CrDiv dv;
+                        ok = S::pad_dv(eos, dv, V);
+                        if (!eos.cr || dv.special()) ok = S::pad(eos, V);
+                    } else {
+                        ok = CONS ? S::pad_cons(eos, V) : S::pad(eos, V);
+                    }
                 }
             }
             // every lane takes part in the shuffle (no short-circuit around it)

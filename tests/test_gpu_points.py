@@ -188,3 +188,21 @@ def test_device_calls_read_cell_major_arrays(hp, orc, system, order, nx, ny, end
             assert (st != hp.OK) == (sto != 0)
             if sto == 0:
                 assert dR.cpu().numpy().tobytes() == Ro.tobytes() and dt == dto
+
+
+@pytest.mark.parametrize("order", [1, 2, 3])
+def test_liquid_under_tension(hp, orc, order):
+    """Negative pressures above -P_inf in an almost pure liquid: the trace gas's p + pi_2 is negative,
+    the quick range refuses every cell and the mixture's denominators may cancel."""
+    cfg, U = _kapila(order, 67, 21, scale_p=-1e5)
+    U = U.reshape(-1, 6)
+    a0, a1 = U[:, 5].copy(), 1.0 - 1e-6 * (1.0 + np.arange(U.shape[0]) % 7)
+    U[:, 0] *= a1 / a0
+    U[:, 1] *= (1.0 - a1) / (1.0 - a0)
+    U[:, 5] = a1
+    rho = U[:, 0] + U[:, 1]
+    U[:, 2:4] = 0.01 * rho[:, None] * np.sin(np.arange(2 * U.shape[0]).reshape(-1, 2))
+    g1, g2 = cfg.gamma1 - 1, cfg.gamma2 - 1
+    p = -1e3 * (1.0 + (np.arange(U.shape[0]) % 13))
+    U[:, 4] = (p * (a1 * g2 + (1 - a1) * g1) + a1 * cfg.gamma1 * cfg.pi1 * g2) / (g1 * g2) + 0.5 * (U[:, 2] ** 2 + U[:, 3] ** 2) / rho
+    _same(hp, orc, cfg, np.ascontiguousarray(U.reshape(-1)))
