@@ -36,9 +36,11 @@ __device__ __forceinline__ double rcp_rn(double b)
     e = fma(-b, y, 1.0);
     return fma(y, e, y);
 }
-// the low words of the divisors of rcp_rn, folded together: all ones in one of them is the
-// only doubtful case (a superset of the all-ones significand, one divisor in 2^32)
-__device__ __forceinline__ unsigned rcp_low(unsigned fold, double b) { return max(fold, (unsigned)__double2loint(b)); }
+// the divisors of rcp_rn folded together: all ones in one significand is the only doubtful case
+__device__ __forceinline__ unsigned rcp_low(unsigned fold, double b)
+{
+    return max(fold, (unsigned)__double2loint(b) & ((unsigned)__double2hiint(b) | 0xfff00000u));
+}
 __device__ __forceinline__ bool rcp_special(unsigned fold) { return fold == 0xffffffffu; }
 
 // a / b correctly rounded from y = rcp_rn(b): quotients by one divisor share y.  q1 = a y and one

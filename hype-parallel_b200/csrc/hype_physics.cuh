@@ -167,7 +167,7 @@ __device__ __forceinline__ bool frac_in(double x) { return (unsigned)__double2hi
 
 // How a system's functions divide.  IeeeDiv: the compiler's division.  CrDiv: the
 // branch-free correctly rounded forms of hype_div.cuh, whose chains interleave; the values
-// named to pos() and frac() bound every operand, and where one is outside (or a divisor's low
+// named to pos() and frac() bound every operand, and where one is outside (or a divisor's
 // word is all ones) special() holds and the caller repeats the function with IeeeDiv.
 struct IeeeDiv {
     __device__ __forceinline__ double operator()(double a, double b) const { return a / b; }
