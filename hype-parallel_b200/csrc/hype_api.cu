@@ -282,14 +282,18 @@ static cudaError_t stage(hype_solver *s, const double *in, double *out, int mode
 }
 
 // Whether the right-hand side of a cell-major array can read it as it is: the primitive
-// inviscid FP64 forms, rows that start on 16-byte boundaries (TMA).  The other calls convert it
-// to planes first.  Device calls, planes -> as it is (with a kernel that knows its mode): Kapila
+// inviscid FP64 forms, rows that start on 16-byte boundaries (TMA), a result that shares no byte
+// with it (blocks store their rows while others still load their stencils').  The other calls
+// convert it to planes first.  Device calls, planes -> as it is (with a kernel that knows its mode): Kapila
 // 64^2 48 -> 42 us, 2048^2 1.57 -> 1.43 ms, BN 1024^2 0.727 -> 0.646, Euler 1531 x 897 0.319 -> 0.278,
 // performance form 1024^2 0.318 -> 0.264.
-static bool reads_aos(const hype_solver *s, const double *aos)
+static bool reads_aos(const hype_solver *s, const double *aos, const double *out)
 {
+    const size_t a = reinterpret_cast<size_t>(aos), o = reinterpret_cast<size_t>(out);
+    const size_t bytes = sizeof(double) * (size_t)s->cfg.nx * s->cfg.ny * s->nv;
+    if (a < o + bytes && o < a + bytes) return false;
     return !s->mixed && s->row_off == 0 && !(s->cfg.flags & (HYPE_FLAG_VISCOUS | HYPE_FLAG_CONSERVATIVE)) &&
-           (reinterpret_cast<size_t>(aos) & 15) == 0 && ((size_t)s->cfg.nx * s->nv) % 2 == 0;
+           (a & 15) == 0 && ((size_t)s->cfg.nx * s->nv) % 2 == 0;
 }
 // the right-hand side of runs run0 .. run0+run_count-1 (0: all) of `aos` into `out`, both cell-major
 static cudaError_t stage_rhs(hype_solver *s, const double *aos, double *out, int run0 = 0, int run_count = 0)
@@ -995,11 +999,11 @@ static cudaError_t store_state(hype_solver *s, int k, double *aos)
     return launch_planes_to_aos(k == 0 ? s->dU : s->dS0, aos, s->cfg.nx, s->cfg.ny, s->nv, s->pitch, s->plane, s->stream);
 }
 
-// RHS of the interleaved device array dU into another
+// RHS of the interleaved device array dU into another, which may share memory with it
 static int rhs_common(hype_solver *s, const double *dU, double *dRHS_aos, double *dt)
 {
     int rc;
-    const bool aos = reads_aos(s, dU);
+    const bool aos = reads_aos(s, dU, dRHS_aos);
     if (!aos) CUDA_TRY(s, load_state(s, dU, 1));
     if ((rc = reset_scalars(s))) return rc;
     if (aos) CUDA_TRY(s, stage_rhs(s, dU, dRHS_aos));

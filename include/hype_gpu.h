@@ -142,7 +142,7 @@ HYPE_API const char *hype_last_error(const hype_solver *s);
 HYPE_API int hype_rhs_prim(hype_solver *s, double t, const double *U, double *RHS, double *dt);
 
 /* Same with U and RHS in device memory of the solver's device (e.g. a PETSc
- * VECCUDA array); the call is synchronous. */
+ * VECCUDA array); the call is synchronous.  RHS may be U itself or overlap it. */
 HYPE_API int hype_rhs_prim_device(hype_solver *s, double t, const double *dU, double *dRHS, double *dt);
 
 /* One MPI rank's share of a grid decomposed over ranks in y: HyPE-2D's DMDA
