@@ -4,6 +4,9 @@
 // host dispatch over (system, order, tile width).  The tile itself is
 // stage_tile in hype_stage_tile.cuh.
 //
+// Compiled once with HYPE_STAGE_SYS and HYPE_STAGE_CELLS for each system and tile width (the
+// kernels, side by side in as many compiler processes) and once without (the dispatch).
+//
 // Built with --fmad=false: arithmetic rounds exactly as the reference's C does.
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -12,6 +15,21 @@
 
 namespace hype {
 
+// the kernels of a system, order and tile width
+struct StageEntry {
+    const void *single;
+    const void *rhs;
+    const void *axpy, *mix;                // of the whole grid, by mode
+    const void *batch_axpy, *batch_mix, *batch_rk;   // batch_rk: N = 3's fifth stage, else null
+    size_t smem;
+    int threads;
+    int aos_box;   // elements of one part of a cell-major row's box
+    int mix_mode;
+};
+
+template <int SYS, int CELLS> StageEntry stage_entry_of(int order);
+
+#ifdef HYPE_STAGE_SYS
 template <int SYS, int N, int CELLS>
 __global__ void __launch_bounds__(2 * CELLS, (StageKernel<SYS, N, CELLS>::MIN_BLOCKS))
 stage_kernel(const __grid_constant__ CUtensorMap tmap, const StageParams p)
@@ -68,20 +86,6 @@ stage_batch_kernel(const StageParams *__restrict__ inst, const CUtensorMap *__re
     work_finish(sched);
 }
 
-// ---------------------------------------------------------------------------
-// host dispatch over (system, order, tile width)
-// ---------------------------------------------------------------------------
-struct StageEntry {
-    const void *single;
-    const void *rhs;
-    const void *axpy, *mix;                // of the whole grid, by mode
-    const void *batch_axpy, *batch_mix, *batch_rk;   // batch_rk: N = 3's fifth stage, else null
-    size_t smem;
-    int threads;
-    int aos_box;   // elements of one part of a cell-major row's box
-    int mix_mode;
-};
-
 template <int SYS, int N, int CELLS>
 static StageEntry entry_of()
 {
@@ -105,7 +109,7 @@ static StageEntry entry_of()
 }
 
 template <int SYS, int CELLS>
-static StageEntry entry_sys(int order)
+StageEntry stage_entry_of(int order)
 {
     switch (order) {
     case 0: return entry_of<SYS, 0, CELLS>();
@@ -115,13 +119,18 @@ static StageEntry entry_sys(int order)
     }
 }
 
+template StageEntry stage_entry_of<HYPE_STAGE_SYS, HYPE_STAGE_CELLS>(int order);
+#else
+// ---------------------------------------------------------------------------
+// host dispatch over (system, order, tile width)
+// ---------------------------------------------------------------------------
 template <int CELLS>
 static StageEntry entry_cells(int sys, int order)
 {
     switch (sys) {
-    case SYS_EULER: return entry_sys<SYS_EULER, CELLS>(order);
-    case SYS_KAPILA: return entry_sys<SYS_KAPILA, CELLS>(order);
-    default: return entry_sys<SYS_BN, CELLS>(order);
+    case SYS_EULER: return stage_entry_of<SYS_EULER, CELLS>(order);
+    case SYS_KAPILA: return stage_entry_of<SYS_KAPILA, CELLS>(order);
+    default: return stage_entry_of<SYS_BN, CELLS>(order);
     }
 }
 
@@ -195,5 +204,7 @@ cudaError_t launch_stage_batch(int sys, int order, int cells, int mode, const St
     if (!f) return cudaErrorInvalidValue;
     return cudaLaunchKernel(f, dim3((unsigned)blocks, 1, 1), dim3((unsigned)e.threads, 1, 1), args, e.smem, s);
 }
+
+#endif
 
 }  // namespace hype
