@@ -470,6 +470,9 @@ template <> struct System<SYS_KAPILA> {
         B[5] = u * alpha1_x + v * alpha1_y - K * (u_x + v_y);
     }
     static constexpr bool ncp_cons_nonzero(int c) { return c == 5; }
+    // a node value of alpha_1 that does not refuse the cell by itself: pad_cons's first test
+    static constexpr int CONS_SCREEN = 5;
+    __device__ __forceinline__ static bool cons_screen(double alpha_1) { return !(alpha_1 < 1.0 || alpha_1 > 1.0); }
     // kapila_5eqn.c:247-283; its alpha test (line 278) rejects every alpha_1 != 1
     __device__ __forceinline__ static bool pad_cons(const EosBase &e, const double *Q)
     {
@@ -665,6 +668,8 @@ template <> struct System<SYS_BN> {
         B[8] = u_1 * phi_x + v_1 * phi_y;
     }
     static constexpr bool ncp_cons_nonzero(int c) { return c != 0 && c != 4; }
+    static constexpr int CONS_SCREEN = -1;   // pad_cons has no test of one variable
+    __device__ __forceinline__ static bool cons_screen(double) { return true; }
     // baer_nunziato.c:207-250
     __device__ __forceinline__ static bool pad_cons(const EosBase &e, const double *Q)
     {
@@ -781,6 +786,8 @@ template <> struct System<SYS_EULER> {
         B[0] = 0.0; B[1] = 0.0; B[2] = 0.0; B[3] = 0.0;
     }
     static constexpr bool ncp_cons_nonzero(int) { return false; }
+    static constexpr int CONS_SCREEN = -1;
+    __device__ __forceinline__ static bool cons_screen(double) { return true; }
     // euler.c:169-191
     __device__ __forceinline__ static bool pad_cons(const EosBase &e, const double *Q)
     {

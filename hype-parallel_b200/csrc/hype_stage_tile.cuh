@@ -694,7 +694,7 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
         double VR[NV];                              // bottom values
         const double *yt_lo = yt_s + ((((r - y0) & 1) * NFGP + q) * NV) * CELLS + m;     // top values of row r-1,
         double *yt_up = yt_s + ((((r - y0 + 1) & 1) * NFGP + q) * NV) * CELLS + m;       // and of row r
-        double tq[QH][NV];                          // weighted volume products
+        double tq[QH][NV] = {};                          // weighted volume products
         bool ok = quick_eos;                        // every node in the plainly admissible range
         // the point values from the coefficients that coef(c, cf) gives
         auto points = [&](auto coef) {
@@ -722,9 +722,10 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
                     });
                 }
             });
-            // the volume non-conservative products (rhs_function_prim.c:459-479)
+            // the volume non-conservative products (rhs_function_prim.c:459-479).  CONS: of the run's own
+            // rows (many divisions a point: Kapila N = 2 64^2 69.5 -> 61.5 us, 1024^2 0.752 -> 0.740 ms)
             if constexpr (NZ > 0) {
-                static_for<QH>([&](auto sa) {
+                if (!CONS || full_row) static_for<QH>([&](auto sa) {
                     constexpr int a = decltype(sa)::value;
                     double B[NV];
                     if constexpr (CONS) S::ncp_cons(eos, Vv[a], gx[a], gy[a], B);
@@ -737,15 +738,54 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
                 });
             }
         };
+        // CONS (rhs_function.c:380-420): a refused cell keeps its mean alone, so what refuses it cheaply
+        // is looked at before its pass: the node values of a variable that can do so by itself (for
+        // Kapila nearly every time), and for N = 1 the whole check (a half's two of the four nodes
+        // are two terms each).  The other cells are checked on the pass's values, and refused ones
+        // take a second pass.  1024^2 right-hand sides, all cells checked after -> this way (and the
+        // volume products of own rows only): Kapila N = 1 0.515 -> 0.456 ms, N = 2 0.850 -> 0.738, N = 3
+        // 1.224 -> 1.082, BN N = 1 0.800 -> 0.715; checked before for every N: BN N = 2 1.195 -> 1.218,
+        // N = 3 1.279 -> 1.401, Euler N = 2 0.267 -> 0.287
+        bool whole = true;
+        if constexpr (CONS && HAS_PAD && (N == 1 || S::CONS_SCREEN >= 0)) {
+            constexpr int NODES = NFGP > 1 ? 4 : 2;   // of this half: the four faces at q = h, or two of the four faces
+            auto node = [&](auto ff, int c) {
+                constexpr int f = decltype(ff)::value;
+                double cf[NDOF];
+                cf[0] = w_0[c * BW + ccm];
+#pragma unroll
+                for (int k = 1; k < NDOF; ++k) cf[k] = coef_s[cidx(k - 1, c, m)];
+                if constexpr (NFGP > 1) return face_pt<N, f, FAST>(cf, mask0);
+                double v = cf[0];
+                static_for<NDOF - 1>([&](auto kk) {
+                    constexpr int k = decltype(kk)::value + 1;
+                    v = v + cf[k] * (h ? FacePt<N, 2 + f % 2, k>::p0() : FacePt<N, f % 2, k>::p0());
+                });
+                return v;
+            };
+            if constexpr (S::CONS_SCREEN >= 0)
+                static_for<NODES>([&](auto ff) { whole = whole && S::cons_screen(node(ff, S::CONS_SCREEN)); });
+            if constexpr (N == 1)
+                static_for<NODES>([&](auto ff) {
+                    if (!whole || !active) return;
+                    double V[NV];
+#pragma unroll
+                    for (int c = 0; c < NV; ++c) V[c] = node(ff, c);
+                    whole = S::pad_cons(eos, V);
+                });
+            // every lane takes part in the shuffle (no short-circuit around it)
+            const int pair = __shfl_xor_sync(FULL, (int)whole, 1);
+            whole = whole && pair;
+        }
         points([&](int c, double *cf) {
 #pragma unroll
-            for (int k = 1; k < NDOF; ++k) cf[k] = coef_s[cidx(k - 1, c, m)];
+            for (int k = 1; k < NDOF; ++k) cf[k] = whole ? coef_s[cidx(k - 1, c, m)] : 0.0;
             __syncwarp();   // both halves have the variable's coefficients: its face values may replace them
         });
-        if constexpr (HAS_PAD) {
+        if constexpr (HAS_PAD && !(CONS && N == 1)) {
             // admissibility at the nodes (rhs_function_prim.c:382-404): the four faces' values at
             // this half's Gauss point
-            if (active && (CONS || !ok)) {
+            if (active && whole && (CONS || !ok)) {
                 ok = true;
 #pragma unroll 1
                 for (int f = 0; f < 4 && ok; ++f) {
@@ -763,7 +803,7 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
             }
             // every lane takes part in the shuffle (no short-circuit around it)
             const int ok_pair = __shfl_xor_sync(FULL, (int)ok, 1);
-            if (active && !(ok && ok_pair)) {
+            if (active && whole && !(ok && ok_pair)) {
                 // the fallback's coefficients: [w, minmod_x, minmod_y, 0 ...] (rhs_function_prim.c:407-421);
                 // conservative path: the mean alone (rhs_function.c:410-420)
                 points([&](int c, double *cf) {
