@@ -180,37 +180,45 @@ static int make_mixed_maps(hype_solver *s, MixedMaps *mm, float *pf, double *pd)
 }
 
 // the stage kernel of a solver for a tile width: resident blocks per SM, 0 if there is none
-static int tile_blocks(hype_solver *s, int cells)
+static int tile_blocks(const hype_solver *s, int cells)
 {
     const hype_config *cfg = &s->cfg;
     const bool cons = (cfg->flags & HYPE_FLAG_CONSERVATIVE) != 0;
     if (s->mixed) return mixed_blocks_per_sm(cfg->system, cells);
     if (cfg->flags & HYPE_FLAG_VISCOUS)   // the viscous and conservative kernels come in 128-column tiles only
-        return cells == STAGE_CELLS && stage_visc_configure(cfg->order, cons) == cudaSuccess ? stage_visc_blocks_per_sm(cfg->order, cons) : 0;
-    if (cons)
-        return cells == STAGE_CELLS && stage_cons_configure(cfg->system, cfg->order) == cudaSuccess
-                   ? stage_cons_blocks_per_sm(cfg->system, cfg->order) : 0;
-    if (s->fast)
-        return stage_fast_configure(cfg->system, cfg->order, cells) == cudaSuccess ? stage_fast_blocks_per_sm(cfg->system, cfg->order, cells) : 0;
-    return stage_configure(cfg->system, cfg->order, cells) == cudaSuccess ? stage_blocks_per_sm(cfg->system, cfg->order, cells) : 0;
+        return cells == STAGE_CELLS ? stage_visc_blocks_per_sm(cfg->order, cons) : 0;
+    if (cons) return cells == STAGE_CELLS ? stage_cons_blocks_per_sm(cfg->system, cfg->order) : 0;
+    return s->fast ? stage_fast_blocks_per_sm(cfg->system, cfg->order, cells) : stage_blocks_per_sm(cfg->system, cfg->order, cells);
+}
+// lets the other kernels that the solver launches at this width take their shared memory
+static cudaError_t tile_configure(const hype_solver *s, int cells)
+{
+    const hype_config *cfg = &s->cfg;
+    if (s->mixed || (cfg->flags & (HYPE_FLAG_VISCOUS | HYPE_FLAG_CONSERVATIVE))) return cudaSuccess;   // one kernel
+    return s->fast ? stage_fast_configure(cfg->system, cfg->order, cells) : stage_configure(cfg->system, cfg->order, cells);
 }
 static int tile_strips(const hype_solver *s, int cells)
 {
     return s->mixed ? mixed_strips(s->cfg.nx, cells) : stage_strips(s->cfg.nx, cells);
 }
 
+struct Shape {
+    int cells, bps, runs, waves;
+};
+
 // Tile width and number of row runs.  Rebuilds the TMA descriptors, whose box width
 // follows the tile width, and drops the captured step graph (recaptured on the next
 // hype_begin / hype_advance).
-static int apply_tiling(hype_solver *s, int cells, int runs, int waves)
+static int apply_tiling(hype_solver *s, const Shape &shape)
 {
     int rc;
-    s->cells = cells;
-    s->bps = tile_blocks(s, cells);
-    if (s->bps < 1) return fail(s, HYPE_ERR_CUDA, "stage kernel does not fit on an SM");
-    s->strips = tile_strips(s, cells);
-    s->runs = runs;
-    s->waves = waves;
+    if (shape.bps < 1) return fail(s, HYPE_ERR_CUDA, "stage kernel does not fit on an SM");
+    s->cells = shape.cells;
+    s->bps = shape.bps;
+    CUDA_TRY(s, tile_configure(s, s->cells));
+    s->strips = tile_strips(s, s->cells);
+    s->runs = shape.runs;
+    s->waves = shape.waves;
     if (s->mixed) {
         for (int k = 0; k < 3; ++k)
             if ((rc = make_mixed_maps(s, &s->mm[k], s->mf[k], s->md[k]))) return rc;
@@ -222,14 +230,12 @@ static int apply_tiling(hype_solver *s, int cells, int runs, int waves)
 }
 
 // `waves` waves of strips x row runs (<= SMs x resident blocks each), at least 8 rows per run
-static int set_tiling(hype_solver *s, int cells, int waves)
+static Shape waves_shape(const hype_solver *s, int cells, int waves)
 {
     if (!s->mixed && (s->cfg.flags & (HYPE_FLAG_VISCOUS | HYPE_FLAG_CONSERVATIVE))) cells = STAGE_CELLS;
     const int bps = tile_blocks(s, cells);
-    if (bps < 1) return fail(s, HYPE_ERR_CUDA, "stage kernel does not fit on an SM");
-    int runs = s->sms * bps * waves / tile_strips(s, cells);
-    if (runs > s->cfg.ny / 8) runs = s->cfg.ny / 8;
-    return apply_tiling(s, cells, runs > 0 ? runs : 1, waves);
+    const int runs = std::min(s->sms * bps * waves / tile_strips(s, cells), s->cfg.ny / 8);
+    return Shape{cells, bps, std::max(runs, 1), waves};
 }
 
 // The shape a solver starts with, by estimated time (best_runs): the tile width and runs of
@@ -237,22 +243,20 @@ static int set_tiling(hype_solver *s, int cells, int waves)
 // rows or more, else those (large grids: the estimates differ by less than they are sure of).
 // Before -> after: Kapila 64^2 device right-hand side 110 -> 48 us, N = 3 500^2 247 -> 218 us, 20 N = 1
 // steps of 128^2 with their copies 2.48 -> 0.98 ms.
-static int default_tiling(hype_solver *s)
+static Shape estimated_shape(const hype_solver *s)
 {
-    const int wide = s->mixed ? MIXED_CELLS : STAGE_CELLS;
-    int rc;
-    if ((rc = set_tiling(s, wide, 1))) return rc;
-    const int rows = (s->cfg.ny + s->runs - 1) / s->runs;
-    double least = 0.97 * tile_launch_cost(s->mixed, wide, s->sms, s->bps, (long long)s->strips * s->runs, rows);
-    int cells = 0, runs = 0;
+    Shape best = waves_shape(s, s->mixed ? MIXED_CELLS : STAGE_CELLS, 1);
+    if (best.bps < 1) return best;
+    const int rows = (s->cfg.ny + best.runs - 1) / best.runs;
+    double least = 0.97 * tile_launch_cost(s->mixed, best.cells, s->sms, best.bps, (long long)tile_strips(s, best.cells) * best.runs, rows);
     for (int c : {64, 128}) {
         const int bps = tile_blocks(s, c);
         if (bps < 1) continue;
         double cost;
-        const int r = best_runs(s->mixed, c, s->sms, bps, tile_strips(s, c), s->cfg.ny, &cost);
-        if (cost < least) { least = cost; cells = c; runs = r; }
+        const int runs = best_runs(s->mixed, c, s->sms, bps, tile_strips(s, c), s->cfg.ny, &cost);
+        if (cost < least) { least = cost; best = Shape{c, bps, runs, 1}; }
     }
-    return cells ? apply_tiling(s, cells, runs, 1) : HYPE_OK;
+    return best;
 }
 
 static const CUtensorMap &tmap_for(const hype_solver *s, const double *buf)
@@ -876,7 +880,7 @@ static int create_common(hype_solver *s, const hype_config *cfg, int row_off, co
     }
 
     s->sms = prop.multiProcessorCount;
-    return default_tiling(s);
+    return apply_tiling(s, estimated_shape(s));
 }
 
 int hype::create_block(const hype_config *global, int col0, int cols, int row0, int rows, const bool halo[4], hype_solver **out)
@@ -1471,26 +1475,21 @@ int hype_autotune(hype_solver *s, int reps, int *cells_out, int *waves_out)
 {
     if (!s) return HYPE_ERR_INVALID;
     if (reps < 1) reps = 3;
-    static const int cand_cells[2] = {64, 128};
-    static const int cand_waves[3] = {1, 2, 4};
-    int best_c = 0, best_w = 1, rc;
-    double best = 1e300;
-    // the estimated shape first, then the candidates
-    if ((rc = default_tiling(s)) || (rc = hype_time_stage(s, reps, &best))) return rc;
-    best_c = s->cells;
-    const int best_r = s->runs;
-    bool estimated = true;
-    for (int c : cand_cells)
-        for (int w : cand_waves) {
-            if ((rc = set_tiling(s, c, w))) return rc;
-
+    // the estimated shape first, then the listed ones
+    Shape best = estimated_shape(s);
+    double least = 1e300;
+    int rc;
+    if ((rc = apply_tiling(s, best)) || (rc = hype_time_stage(s, reps, &least))) return rc;
+    for (int c : {64, 128})
+        for (int w : {1, 2, 4}) {
+            const Shape shape = waves_shape(s, c, w);
             double ms = 0.0;
-            if ((rc = hype_time_stage(s, reps, &ms))) return rc;
-            if (ms < best) { best = ms; best_c = c; best_w = w; estimated = false; }
+            if ((rc = apply_tiling(s, shape)) || (rc = hype_time_stage(s, reps, &ms))) return rc;
+            if (ms < least) { least = ms; best = shape; }
         }
-    if ((rc = estimated ? apply_tiling(s, best_c, best_r, 1) : set_tiling(s, best_c, best_w))) return rc;
-    if (cells_out) *cells_out = best_c;
-    if (waves_out) *waves_out = best_w;
+    if ((rc = apply_tiling(s, best))) return rc;
+    if (cells_out) *cells_out = best.cells;
+    if (waves_out) *waves_out = best.waves;
     return HYPE_OK;
 }
 

@@ -95,9 +95,11 @@ constexpr int stage_box_width(int cells, int nv)
 
 size_t stage_smem_bytes(int sys, int order, int cells);
 int stage_threads(int cells);
-cudaError_t stage_configure(int sys, int order, int cells);   // raises the dynamic smem limit
+cudaError_t stage_configure(int sys, int order, int cells);   // raises the dynamic smem limit of a solver's kernels
+// resident blocks of the general grid form and of the persistent form; both raise that limit for
+// the kernels they name, the second for a batch's
 int stage_blocks_per_sm(int sys, int order, int cells);
-int stage_batch_blocks_per_sm(int sys, int order, int cells);   // resident blocks of the persistent form
+int stage_batch_blocks_per_sm(int sys, int order, int cells);
 cudaError_t launch_stage(int sys, int order, int cells, const CUtensorMap &tmap, const StageParams &p, cudaStream_t s);
 // the right-hand side from and to cell-major arrays p.in and p.out (primitive inviscid path;
 // 16-byte aligned rows): tmap is 2-D over p.in, (nx NV, ny), box (stage_aos_box, 1)

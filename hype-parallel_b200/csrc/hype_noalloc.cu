@@ -125,7 +125,6 @@ extern "C" HYPE_API int hype_rhs_prim_noalloc(const hype_config *cfg, double t, 
                                               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return HYPE_ERR_CUDA;
 
-    if (stage_configure(cfg->system, cfg->order, STAGE_CELLS) != cudaSuccess) return HYPE_ERR_CUDA;
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg->device) != cudaSuccess) return HYPE_ERR_CUDA;
     const int bps = stage_blocks_per_sm(cfg->system, cfg->order, STAGE_CELLS);

@@ -4,13 +4,14 @@
 // host dispatch over (system, order, tile width).  The tile itself is
 // stage_tile in hype_stage_tile.cuh.
 //
-// Compiled once with HYPE_STAGE_SYS and HYPE_STAGE_CELLS for each system and tile width (the
-// kernels, side by side in as many compiler processes) and once without (the dispatch).
+// Compiled once with HYPE_STAGE_SYS and HYPE_STAGE_ORDER for each system and order (the kernels, side
+// by side in as many compiler processes) and once without (the dispatch).  An object is one module,
+// which a process loads whole with its first kernel.
 //
 // Built with --fmad=false: arithmetic rounds exactly as the reference's C does.
 #include <cuda.h>
 #include <cuda_runtime.h>
-#include <cstdio>
+#include <initializer_list>
 #include "hype_stage_tile.cuh"
 
 namespace hype {
@@ -27,7 +28,7 @@ struct StageEntry {
     int mix_mode;
 };
 
-template <int SYS, int CELLS> StageEntry stage_entry_of(int order);
+template <int SYS, int N> StageEntry stage_entry_of(int cells);
 
 #ifdef HYPE_STAGE_SYS
 template <int SYS, int N, int CELLS>
@@ -108,55 +109,59 @@ static StageEntry entry_of()
     return e;
 }
 
-template <int SYS, int CELLS>
-StageEntry stage_entry_of(int order)
+template <int SYS, int N>
+StageEntry stage_entry_of(int cells)
 {
-    switch (order) {
-    case 0: return entry_of<SYS, 0, CELLS>();
-    case 1: return entry_of<SYS, 1, CELLS>();
-    case 2: return entry_of<SYS, 2, CELLS>();
-    default: return entry_of<SYS, 3, CELLS>();
-    }
+    return cells == 64 ? entry_of<SYS, N, 64>() : entry_of<SYS, N, 128>();
 }
-
-template StageEntry stage_entry_of<HYPE_STAGE_SYS, HYPE_STAGE_CELLS>(int order);
+template StageEntry stage_entry_of<HYPE_STAGE_SYS, HYPE_STAGE_ORDER>(int cells);
 #else
 // ---------------------------------------------------------------------------
 // host dispatch over (system, order, tile width)
 // ---------------------------------------------------------------------------
-template <int CELLS>
-static StageEntry entry_cells(int sys, int order)
+template <int SYS>
+static StageEntry entry_sys(int order, int cells)
 {
-    switch (sys) {
-    case SYS_EULER: return stage_entry_of<SYS_EULER, CELLS>(order);
-    case SYS_KAPILA: return stage_entry_of<SYS_KAPILA, CELLS>(order);
-    default: return stage_entry_of<SYS_BN, CELLS>(order);
+    switch (order) {
+    case 0: return stage_entry_of<SYS, 0>(cells);
+    case 1: return stage_entry_of<SYS, 1>(cells);
+    case 2: return stage_entry_of<SYS, 2>(cells);
+    default: return stage_entry_of<SYS, 3>(cells);
     }
 }
 
 static StageEntry stage_entry(int sys, int order, int cells)
 {
-    return cells == 64 ? entry_cells<64>(sys, order) : entry_cells<128>(sys, order);
+    switch (sys) {
+    case SYS_EULER: return entry_sys<SYS_EULER>(order, cells);
+    case SYS_KAPILA: return entry_sys<SYS_KAPILA>(order, cells);
+    default: return entry_sys<SYS_BN>(order, cells);
+    }
 }
 
 size_t stage_smem_bytes(int sys, int order, int cells) { return stage_entry(sys, order, cells).smem; }
 int stage_threads(int cells) { return 2 * cells; }
 
-cudaError_t stage_configure(int sys, int order, int cells)
+static cudaError_t allow_smem(std::initializer_list<const void *> kernels, size_t smem)
 {
-    const StageEntry e = stage_entry(sys, order, cells);
-    for (const void *f : {e.single, e.rhs, e.axpy, e.mix, e.batch_axpy, e.batch_mix, e.batch_rk}) {
-        const cudaError_t r = f ? cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem) : cudaSuccess;
+    for (const void *f : kernels) {
+        const cudaError_t r = f ? cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : cudaSuccess;
         if (r != cudaSuccess) return r;
     }
     return cudaSuccess;
+}
+
+cudaError_t stage_configure(int sys, int order, int cells)
+{
+    const StageEntry e = stage_entry(sys, order, cells);
+    return allow_smem({e.single, e.rhs, e.axpy, e.mix}, e.smem);
 }
 
 int stage_blocks_per_sm(int sys, int order, int cells)
 {
     const StageEntry e = stage_entry(sys, order, cells);
     int nb = 0;
-    if (stage_configure(sys, order, cells) != cudaSuccess) return 0;
+    if (allow_smem({e.single}, e.smem) != cudaSuccess) return 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, e.single, e.threads, e.smem) != cudaSuccess) return 0;
     return nb;
 }
@@ -165,7 +170,8 @@ int stage_batch_blocks_per_sm(int sys, int order, int cells)
 {
     const StageEntry e = stage_entry(sys, order, cells);
     int nb = 0;
-    if (stage_configure(sys, order, cells) != cudaSuccess) return 0;
+    // `single` gives the dt of an instance that joins
+    if (allow_smem({e.single, e.batch_axpy, e.batch_mix, e.batch_rk}, e.smem) != cudaSuccess) return 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, e.batch_axpy, e.threads, e.smem) != cudaSuccess) return 0;
     return nb;
 }

@@ -4,12 +4,27 @@
 // (no --fmad=false): products and sums fuse where the compiler finds them, so
 // its results differ from the reference's in the last bits; the tests hold
 // them to a relative L-infinity difference of 1e-12 per RHS evaluation.
+//
+// Compiled once with HYPE_STAGE_SYS and HYPE_STAGE_ORDER for each system and order and once
+// without, as hype_stage.cu.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include "hype_stage_tile.cuh"
 
 namespace hype {
 
+struct FastEntry {
+    const void *fn;
+    const void *rhs;
+    const void *axpy, *mix;   // of the whole grid, by mode
+    int mix_mode;
+    size_t smem;
+    int threads;
+};
+
+template <int SYS, int N> FastEntry fast_entry_of(int cells);
+
+#ifdef HYPE_STAGE_SYS
 template <int SYS, int N, int CELLS>
 __global__ void __launch_bounds__(2 * CELLS, (StageKernel<SYS, N, CELLS>::MIN_BLOCKS))
 stage_fast_kernel(const __grid_constant__ CUtensorMap tmap, const StageParams p)
@@ -34,15 +49,6 @@ stage_fast_mode_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_co
     stage_tile<SYS, N, CELLS, false, false, true>(p, &tmap, blockIdx.x, p.run0 + (int)blockIdx.y, smem_raw);
 }
 
-struct FastEntry {
-    const void *fn;
-    const void *rhs;
-    const void *axpy, *mix;   // of the whole grid, by mode
-    int mix_mode;
-    size_t smem;
-    int threads;
-};
-
 template <int SYS, int N, int CELLS>
 static FastEntry fast_of()
 {
@@ -58,30 +64,33 @@ static FastEntry fast_of()
     return e;
 }
 
-template <int SYS, int CELLS>
-static FastEntry fast_sys(int order)
+template <int SYS, int N>
+FastEntry fast_entry_of(int cells)
+{
+    return cells == 64 ? fast_of<SYS, N, 64>() : fast_of<SYS, N, 128>();
+}
+template FastEntry fast_entry_of<HYPE_STAGE_SYS, HYPE_STAGE_ORDER>(int cells);
+
+}  // namespace hype
+#else
+template <int SYS>
+static FastEntry fast_sys(int order, int cells)
 {
     switch (order) {
-    case 0: return fast_of<SYS, 0, CELLS>();
-    case 1: return fast_of<SYS, 1, CELLS>();
-    case 2: return fast_of<SYS, 2, CELLS>();
-    default: return fast_of<SYS, 3, CELLS>();
-    }
-}
-
-template <int CELLS>
-static FastEntry fast_cells(int sys, int order)
-{
-    switch (sys) {
-    case SYS_EULER: return fast_sys<SYS_EULER, CELLS>(order);
-    case SYS_KAPILA: return fast_sys<SYS_KAPILA, CELLS>(order);
-    default: return fast_sys<SYS_BN, CELLS>(order);
+    case 0: return fast_entry_of<SYS, 0>(cells);
+    case 1: return fast_entry_of<SYS, 1>(cells);
+    case 2: return fast_entry_of<SYS, 2>(cells);
+    default: return fast_entry_of<SYS, 3>(cells);
     }
 }
 
 static FastEntry fast_entry(int sys, int order, int cells)
 {
-    return cells == 64 ? fast_cells<64>(sys, order) : fast_cells<128>(sys, order);
+    switch (sys) {
+    case SYS_EULER: return fast_sys<SYS_EULER>(order, cells);
+    case SYS_KAPILA: return fast_sys<SYS_KAPILA>(order, cells);
+    default: return fast_sys<SYS_BN>(order, cells);
+    }
 }
 
 cudaError_t stage_fast_configure(int sys, int order, int cells)
@@ -98,7 +107,7 @@ int stage_fast_blocks_per_sm(int sys, int order, int cells)
 {
     const FastEntry e = fast_entry(sys, order, cells);
     int nb = 0;
-    if (stage_fast_configure(sys, order, cells) != cudaSuccess) return 0;
+    if (cudaFuncSetAttribute(e.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)e.smem) != cudaSuccess) return 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, e.fn, e.threads, e.smem) != cudaSuccess) return 0;
     return nb;
 }
@@ -160,3 +169,4 @@ extern "C" HYPE_API int hype_test_fast_rcp(int device, const double *x, int n, d
     cudaFree(d);
     return rc;
 }
+#endif
