@@ -258,14 +258,14 @@ def batch_leg(hp, args, local_rank):
     for prec, name in ((hp.PREC_FP64, "fp64"), (hp.PREC_MIXED, "mixed")):
         with hp.Batch(max_instances=64, max_cells=1024 * 1024, device=local_rank) as b:
             ids = [b.add(cfg(nx, ny, prec), U0[k], 0.0, 1e30, 1 << 30) for k, (nx, ny) in enumerate(sizes)]
-            tile = b.autotune(3)
+            b.autotune(3)
             b.advance(3)
             b.sync()
             b.advance(steps)
             b.sync()
             ms = b.last_elapsed_ms()
             st = [b.status(i) for i in ids]
-            info = b.info()
+            tile, info = b.tiling(), b.info()
             finals[name] = [b.get_state(i).reshape(-1, 6) for i in ids]
         out[name] = {"value": cells * steps / (ms * 1e-3), "unit": UNIT, "ms_per_step": ms / steps,
                      "autotuned_tile": {"cells": tile[0], "rows": tile[1]}, "work_items_per_stage": info["work_items"],

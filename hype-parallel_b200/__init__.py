@@ -211,6 +211,7 @@ def lib() -> ctypes.CDLL:
         L.hype_batch_set_substeps.argtypes = [vp, ctypes.c_int, ctypes.c_int]
         L.hype_batch_set_tiling.argtypes = [vp, ctypes.c_int, ctypes.c_int]
         L.hype_batch_autotune.argtypes = [vp, ctypes.c_int, IP, IP]
+        L.hype_batch_tiling.argtypes = [vp, IP, IP]
         L.hype_batch_info.argtypes = [vp, IP, IP, ctypes.POINTER(ctypes.c_size_t), ctypes.POINTER(ctypes.c_size_t)]
         L.hype_batch_last_elapsed_ms.argtypes = [vp, _DP]
         # include/hype_serve.h
@@ -410,7 +411,7 @@ class Solver:
         return ms.value
 
     def autotune(self, reps: int = 3):
-        """Pick the fastest stage-kernel tile shape; returns (tile width, waves)."""
+        """Pick the fastest stage-kernel tile shape; returns its (tile width, waves of blocks)."""
         c, w = ctypes.c_int(0), ctypes.c_int(0)
         self._check(lib().hype_autotune(self._h, reps, ctypes.byref(c), ctypes.byref(w)))
         return c.value, w.value
@@ -648,6 +649,12 @@ class Batch:
     def autotune(self, reps: int = 3):
         c, r = ctypes.c_int(0), ctypes.c_int(0)
         self._check(lib().hype_batch_autotune(self._h, reps, ctypes.byref(c), ctypes.byref(r)))
+        return c.value, r.value
+
+    def tiling(self):
+        """(tile width, rows per tile) in use of the kind with the most cells."""
+        c, r = ctypes.c_int(0), ctypes.c_int(0)
+        self._check(lib().hype_batch_tiling(self._h, ctypes.byref(c), ctypes.byref(r)))
         return c.value, r.value
 
     def info(self) -> dict:

@@ -254,7 +254,8 @@ static Shape estimated_shape(const hype_solver *s)
         if (bps < 1) continue;
         double cost;
         const int runs = best_runs(s->mixed, c, s->sms, bps, tile_strips(s, c), s->cfg.ny, &cost);
-        if (cost < least) { least = cost; best = Shape{c, bps, runs, 1}; }
+        const int slots = s->sms * bps, tiles = tile_strips(s, c) * runs;
+        if (cost < least) { least = cost; best = Shape{c, bps, runs, (tiles + slots - 1) / slots}; }
     }
     return best;
 }

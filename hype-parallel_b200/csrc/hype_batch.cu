@@ -985,6 +985,17 @@ int hype_batch_autotune(hype_batch *b, int reps, int *cells_out, int *rows_out)
     return HYPE_OK;
 }
 
+int hype_batch_tiling(const hype_batch *b, int *cells, int *rows)
+{
+    if (!b) return HYPE_ERR_INVALID;
+    const Kind *most = nullptr;
+    for (const Kind &k : b->kinds)
+        if (k.ready && !k.members.empty() && (!most || k.cost > most->cost)) most = &k;
+    if (cells) *cells = most ? most->cells : 0;
+    if (rows) *rows = most ? most->rows : 0;
+    return HYPE_OK;
+}
+
 int hype_batch_info(const hype_batch *b, int *instances, int *work_items, size_t *bytes_in_use, size_t *budget)
 {
     if (!b) return HYPE_ERR_INVALID;

@@ -127,9 +127,14 @@ HYPE_API int hype_batch_set_tiling(hype_batch *b, int cells, int rows);
  * {64, 128} and rows per tile in {16, 32, 64, 128}, per instance kind, and
  * keeps the fastest; a kind whose estimated shape is faster than all of them
  * keeps that (and goes on following its instances).  Reports the fastest of
- * the candidates of the kind with the most work.
+ * the candidates of the kind with the most work; hype_batch_tiling tells what
+ * was kept.
  */
 HYPE_API int hype_batch_autotune(hype_batch *b, int reps, int *cells, int *rows);
+
+/* The tile shape in use of the kind with the most cells: tile width and about
+ * how many rows a tile has; 0 and 0 for an empty batch. */
+HYPE_API int hype_batch_tiling(const hype_batch *b, int *cells, int *rows);
 
 /* Instances held, work items per stage launch (all kinds), device bytes held,
  * the admission budget. */

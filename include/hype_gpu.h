@@ -287,10 +287,12 @@ HYPE_API int hype_launch_info(const hype_solver *s, int *grid_x, int *grid_y, in
 HYPE_API int hype_time_stage(hype_solver *s, int reps, double *ms_per_launch);
 
 /* Autotuner: times the stage kernel (hype_time_stage, `reps` launches each) for
- * every tile shape -- tile width 64 or 128 columns, 1, 2 or 4 waves of row runs
- * -- on the solver's current state and keeps the fastest.  Results are
- * unchanged by the choice (bit for bit).  Call before hype_begin or between
- * steps; reports the chosen width and wave count. */
+ * the shape that a new solver has (an estimate, of short row runs on grids that
+ * do not fill the GPU) and for every tile width of 64 or 128 columns with as many
+ * row runs, of 8 rows or more, as 1, 2 or 4 waves of blocks hold, on the solver's
+ * current state, and keeps the fastest.  Results are unchanged by the choice (bit
+ * for bit).  Call before hype_begin or between steps; reports the width and the
+ * waves of the shape kept, of which hype_launch_info gives the launch. */
 HYPE_API int hype_autotune(hype_solver *s, int reps, int *cells, int *waves);
 
 /* Device time of the last hype_solve/hype_wait interval, in milliseconds
