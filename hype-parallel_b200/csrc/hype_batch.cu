@@ -93,6 +93,9 @@ struct Kind {
     int cells = STAGE_CELLS, rows = 64, bps = 0;
     bool shaped = false;               // the tile shape was set (hype_batch_set_tiling, hype_batch_autotune)
     bool joined = false;               // members came or went since the shape was last estimated
+    int est_cells = 0, est_rows = 0;   // the shape of least estimate
+    double est_gain = 0.0;             // microseconds that it saves a stage, 0 if the present one stays
+    double lost = 0.0;                 // of steps taken since the shape was last set
     std::vector<int> members;
     StageParams *dParams = nullptr;    // [MAX_PLAN][M]
     MixedParams *dMParams = nullptr;   // [MAX_PLAN][M]
@@ -446,12 +449,7 @@ static int rebuild_work(hype_batch *b, int id)
         if (n > l.work_cap) {
             int cap = l.work_cap > 0 ? l.work_cap : 1024;
             while (cap < n) cap *= 2;
-            if (b->exec) {   // the captured graph holds the old pointer
-                BCUDA(b, cudaStreamSynchronize(b->stream));
-                cudaGraphExecDestroy(b->exec);
-                b->exec = nullptr;
-            }
-            pool_free(b, l.dWork);
+            pool_free(b, l.dWork);   // behind the queued steps; the graph that holds it is out of date from here
             BCUDA(b, pool_alloc(b, &l.dWork, sizeof(int2) * cap));
             l.work_cap = cap;
             b->dirty = true;
@@ -479,6 +477,7 @@ static int kind_set_tiling(hype_batch *b, int id, int cells, int rows)
     k.cells = cells;
     k.rows = rows;
     k.bps = bps;
+    k.lost = k.est_gain = 0.0;
     int rc;
     for (int s : k.members)
         if ((rc = upload_inst(b, s))) return rc;
@@ -486,6 +485,10 @@ static int kind_set_tiling(hype_batch *b, int id, int cells, int rows)
     b->dirty = true;
     return HYPE_OK;
 }
+
+// Host time of a new shape, its graph update included: measured 40 us for 2 members, 121 for 8,
+// 425 for 32, 1608 for 128
+constexpr double SHAPE_COST_US = 15.0, SHAPE_COST_MEMBER_US = 13.0;
 
 // The shape of least estimate over the kind's members, if that is below `least`.
 static bool best_shape(hype_batch *b, const Kind &k, double least, int *cells, int *rows)
@@ -503,17 +506,29 @@ static bool best_shape(hype_batch *b, const Kind &k, double least, int *cells, i
 }
 
 // The tile shape of a kind whose members changed and whose shape nobody set: the least
-// estimate, if it is 3 % below the present shape's.  Milliseconds a step with 128 x 64 tiles ->
+// estimate, if it is 3 % below the present shape's.  A new shape costs host time for every member
+// (SHAPE_COST_*), so it waits until the steps since the last one, those of the coming advance
+// included, would have gained that much; where the graph is captured anew anyway it does not
+// wait.  Members that come and go by turns thus cost at most twice what the better of their
+// shapes would.  Milliseconds a step with 128 x 64 tiles ->
 // with the estimated ones: 16 Kapila grids of sides 128..512 4.33 -> 3.51 (mixed 3.31 -> 2.05),
 // 12 of 64..160 2.06 -> 0.53, 4 of 64..128 2.50 -> 0.31, 48 of 200..1024 34.1 -> 31.3.
-static int estimate_shape(hype_batch *b, int id)
+static int estimate_shape(hype_batch *b, int id, int nsteps)
 {
     Kind &k = b->kinds[id];
-    if (!k.ready || !k.joined) return HYPE_OK;
-    k.joined = false;
-    int cells, rows;
-    if (k.shaped || k.members.empty() || !best_shape(b, k, 0.97 * shape_cost(b, k, k.cells, k.rows, k.bps), &cells, &rows)) return HYPE_OK;
-    return kind_set_tiling(b, id, cells, rows);
+    if (!k.ready || k.shaped || k.members.empty()) return HYPE_OK;
+    if (k.joined) {
+        k.joined = false;
+        const double now = shape_cost(b, k, k.cells, k.rows, k.bps);
+        k.est_gain = 0.0;
+        if (best_shape(b, k, 0.97 * now, &k.est_cells, &k.est_rows))
+            k.est_gain = tile_iteration_us(k.system, k.order, k.mixed, false) *
+                         (now - shape_cost(b, k, k.est_cells, k.est_rows, kind_blocks_per_sm(k, k.est_cells)));
+    }
+    if (k.est_gain <= 0.0) return HYPE_OK;
+    k.lost += k.est_gain * k.nstage * k.nsub * (double)nsteps;
+    if (!b->dirty && k.lost < SHAPE_COST_US + SHAPE_COST_MEMBER_US * (double)k.members.size()) return HYPE_OK;
+    return kind_set_tiling(b, id, k.est_cells, k.est_rows);
 }
 
 // ---------------------------------------------------------------------------
@@ -548,19 +563,29 @@ static cudaError_t enqueue_kind_step(hype_batch *b, int id, cudaStream_t s)
     return cudaSuccess;
 }
 
-// Captures one step of every non-empty kind; kinds run on parallel branches.
+static int drop_exec(hype_batch *b)
+{
+    if (!b->exec) return HYPE_OK;
+    BCUDA(b, cudaStreamSynchronize(b->stream));
+    cudaGraphExecDestroy(b->exec);
+    b->exec = nullptr;
+    return HYPE_OK;
+}
+
+// Captures one step of every non-empty kind; kinds run on parallel branches.  A graph of the same
+// nodes (another tile shape, a longer work-list) takes the place of the present one behind the
+// steps that are queued; one of other nodes waits for them.
 static int capture_step(hype_batch *b)
 {
-    if (b->exec) {
-        BCUDA(b, cudaStreamSynchronize(b->stream));
-        cudaGraphExecDestroy(b->exec);
-        b->exec = nullptr;
-    }
+    int rc;
     std::vector<int> live;
     for (int id = 0; id < NKIND; ++id)
         if (b->kinds[id].ready && !b->kinds[id].members.empty()) live.push_back(id);
-    b->dirty = false;
-    if (live.empty()) return HYPE_OK;
+    if (live.empty()) {
+        if ((rc = drop_exec(b))) return rc;
+        b->dirty = false;
+        return HYPE_OK;
+    }
     cudaGraph_t g;
     BCUDA(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t e = cudaSuccess;
@@ -581,9 +606,20 @@ static int capture_step(hype_batch *b)
         return bfail(b, HYPE_ERR_CUDA, "batch step capture: %s", cudaGetErrorString(e));
     }
     if (e2 != cudaSuccess) return bfail(b, HYPE_ERR_CUDA, "batch step capture end: %s", cudaGetErrorString(e2));
-    e = cudaGraphInstantiate(&b->exec, g, 0);
+    if (b->exec) {
+        cudaGraphExecUpdateResultInfo info;
+        if (cudaGraphExecUpdate(b->exec, g, &info) != cudaSuccess) {
+            cudaGetLastError();
+            if ((rc = drop_exec(b))) {
+                cudaGraphDestroy(g);
+                return rc;
+            }
+        }
+    }
+    if (!b->exec) e = cudaGraphInstantiate(&b->exec, g, 0);
     cudaGraphDestroy(g);
-    if (e != cudaSuccess) { b->dirty = true; return bfail(b, HYPE_ERR_CUDA, "batch graph instantiate: %s", cudaGetErrorString(e)); }
+    if (e != cudaSuccess) return bfail(b, HYPE_ERR_CUDA, "batch graph instantiate: %s", cudaGetErrorString(e));
+    b->dirty = false;
     return HYPE_OK;
 }
 
@@ -846,7 +882,7 @@ int hype_batch_advance(hype_batch *b, int nsteps)
     BCUDA(b, cudaSetDevice(b->cfg.device));
     int rc;
     for (int id = 0; id < NKIND; ++id)
-        if ((rc = estimate_shape(b, id))) return rc;
+        if ((rc = estimate_shape(b, id, nsteps))) return rc;
     if (b->dirty && (rc = capture_step(b))) return rc;
     if (!b->exec) { b->timed = false; return HYPE_OK; }
     if (b->hold_dirty) {

@@ -16,7 +16,8 @@
  * Instances join and leave between steps (continuous batching): the work-list,
  * member lists and per-instance parameters live in device memory, so adding or
  * removing an instance re-captures nothing unless the set of instance kinds
- * changes.  Each instance stops on its own at its t_final or max_steps; its
+ * or the estimated tile shape changes (the latter behind the queued steps,
+ * without waiting for them).  Each instance stops on its own at its t_final or max_steps; its
  * tiles then cost one flag read per stage until it is removed.
  *
  * Admission is bounded by an HBM budget: hype_batch_add refuses with
@@ -116,8 +117,9 @@ HYPE_API int hype_batch_get_state(hype_batch *b, int id, double *U);
  * columns) and about `rows` rows per tile (16..1024), applied to every
  * instance kind (the conservative and viscous kinds keep 128 columns).
  * Rebuilds the work-list and the step graph.  Until this call or the autotuner
- * sets a kind's shape, it is estimated from its instances at each advance
- * after some joined or left.
+ * sets a kind's shape, it is estimated from its instances after some joined
+ * or left, and changes once the steps asked for would have gained what the
+ * change costs the host (about 13 us per instance).
  */
 HYPE_API int hype_batch_set_tiling(hype_batch *b, int cells, int rows);
 
