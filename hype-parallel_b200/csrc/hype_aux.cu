@@ -386,7 +386,8 @@ __device__ __forceinline__ double wide_double(unsigned long long u, unsigned lon
     return (v >> 63) ? -x : x;
 }
 // the cases of hype_test_division, by index: 0 raw bit patterns, 1 operands of every
-// exponent, 2 quotients next to a midpoint of two doubles, 3 all-ones divisors
+// exponent, 2 quotients next to a midpoint of two doubles, 3 all-ones divisors, 4 divisors whose
+// low word alone is all ones (one in 2^32 otherwise), 5 zeros of both signs over any divisor
 __global__ void division_check_kernel(long long n, unsigned long long seed, unsigned long long *counts)
 {
     unsigned long long mism = 0, spec = 0;
@@ -395,7 +396,7 @@ __global__ void division_check_kernel(long long n, unsigned long long seed, unsi
         const unsigned long long u0 = mix64(k), u1 = mix64(k ^ 0x5851F42D4C957F2Dull), u2 = mix64(k + 0x14057B7EF767814Full),
                                  u3 = mix64(k * 3 + 1);
         double a, b;
-        switch ((int)(i & 3)) {
+        switch ((int)(i % 6)) {
         case 0: a = __longlong_as_double((long long)u0); b = __longlong_as_double((long long)u1); break;
         case 1: a = wide_double(u0, u1); b = wide_double(u2, u3); break;
         case 2: {   // a = RN(b * q_mid), q_mid = 1 + (2m + 1) 2^-53: a/b lies within an ulp or so of a midpoint
@@ -404,6 +405,14 @@ __global__ void division_check_kernel(long long n, unsigned long long seed, unsi
             a = b * qmid;
             break;
         }
+        case 4:
+            b = __hiloint2double(__double2hiint(wide_double(u2, u3)), -1);
+            a = wide_double(u0, u1);
+            break;
+        case 5:
+            b = wide_double(u2, u3);
+            a = (u0 & 1) ? 0.0 : -0.0;
+            break;
         default: {   // divisor with an all-ones significand
             const long long eb = (long long)(u3 % 2000ull) + 20;
             b = __longlong_as_double((long long)(((u1 >> 63) << 63) | ((unsigned long long)eb << 52) | 0x000FFFFFFFFFFFFFull));
@@ -412,15 +421,52 @@ __global__ void division_check_kernel(long long n, unsigned long long seed, unsi
         }
         }
         const double ref = a / b;
-        if (!hype::div_in_range(a, b, ref)) {
+        // the same bits, or two zeros where the numerator is one
+        auto wrong = [&](double q, double r) { return a == 0.0 ? !(q == r) : __double_as_longlong(q) != __double_as_longlong(r); };
+        // the functions in their whole range
+        if (hype::div_in_range(a, b, ref)) {
+            // a divisor that rcp_rn leaves to its caller (all ones): the constant divisors' way
+            const bool ones = hype::rcp_special(hype::rcp_low(0u, b));
+            const double y = ones ? 1.0 / b : hype::rcp_rn(b);
+            if (!ones && __double_as_longlong(y) != __double_as_longlong(1.0 / b)) ++mism;
+            if (wrong(hype::div_rn(a, b, y), ref)) ++mism;
+        } else {
             ++spec;
-            continue;
         }
-        // a divisor that rcp_rn leaves to its caller (all-ones low word): the constant divisors' way
-        const bool low = hype::rcp_special(hype::rcp_low(0u, b));
-        const double y = low ? 1.0 / b : hype::rcp_rn(b);
-        if (!low && __double_as_longlong(y) != __double_as_longlong(1.0 / b)) ++mism;
-        if (__double_as_longlong(hype::div_rn(a, b, y)) != __double_as_longlong(ref)) ++mism;
+        // what their callers' own tests accept: CrDiv's numerators and divisors of any sign, positive
+        // values and fractions, and CrCheck's WENO denominators, which are at least 1e-48
+        {
+            hype::CrDiv dv;
+            dv.num(a);
+            dv.den(b);
+            const double q = dv(a, b);
+            if (!dv.special() && wrong(q, ref)) ++mism;
+        }
+        {
+            hype::CrDiv dv;
+            dv.num(a);
+            dv.pos(fabs(b));
+            const double q = dv.quot(a, fabs(b), dv.rcp(fabs(b)));
+            if (!dv.special() && wrong(q, a / fabs(b))) ++mism;
+        }
+        {
+            hype::CrDiv dv;
+            const double f = __hiloint2double((__double2hiint(b) & 0xfffff) | (int)((1023u - 1u - (unsigned)(u1 % 120)) << 20), __double2loint(b));
+            dv.num(a);
+            dv.frac(f);
+            const double q = dv.quot(a, f, dv.rcp(f));
+            if (!dv.special() && wrong(q, a / f)) ++mism;
+        }
+        {
+            hype::CrCheck ck;
+            const double d = fmax(fabs(b), 1e-48);
+            ck.divisor(d);
+            if (!ck.special()) {
+                const double y = hype::rcp_rn(d);
+                if (__double_as_longlong(y) != __double_as_longlong(1.0 / d)) ++mism;
+                if (__double_as_longlong(hype::div_rn(100.0, d, y)) != __double_as_longlong(100.0 / d)) ++mism;
+            }
+        }
     }
     for (int o = 16; o > 0; o >>= 1) {
         mism += __shfl_xor_sync(0xffffffffu, mism, o);

@@ -45,8 +45,11 @@ __device__ __forceinline__ bool rcp_special(unsigned fold) { return fold == 0xff
 
 // a / b correctly rounded from y = rcp_rn(b): quotients by one divisor share y.  q1 = a y and one
 // correction give a double next to a/b, whose remainder a - b q1 is exact; with y the correctly
-// rounded 1/b the second correction rounds correctly (Markstein 1990, theorem 5).  a, b and a/b
-// nonzero with binary exponents in [-900, 1000].
+// rounded 1/b the second correction rounds correctly (Markstein 1990, theorem 5).  b and a/b of
+// binary exponents in [-1000, 1000] and [-900, 1000], a in [-900, 1000] or zero.  A zero's quotient
+// is a zero, but +0 for -0 over a positive divisor too: callers may pass zeros only where the sign
+// of a zero reaches no result (velocities, pressures and volume products end up as terms of sums
+// that begin with +0).
 __device__ __forceinline__ double div_rn(double a, double b, double y)
 {
     double q = a * y;
@@ -56,12 +59,12 @@ __device__ __forceinline__ double div_rn(double a, double b, double y)
     return fma(r, y, q);
 }
 
-// whether div_rn holds for a, b and the correctly rounded 1/b: what its callers ensure by the
-// ranges of densities, pressures and weights, tested operand by operand (hype_test_division)
+// whether a, b and a/b are in div_rn's range (hype_test_division; the callers ensure it by the ranges
+// of densities, pressures and weights, CrDiv and CrCheck, which that test checks too)
 __device__ __forceinline__ bool div_in_range(double a, double b, double quotient)
 {
     auto within = [](unsigned e, unsigned lo) { return e >= 1023u - lo && e <= 1023u + 1000u; };
-    return within(biased_exp(a), 900u) && within(biased_exp(b), 1000u) && within(biased_exp(quotient), 900u);
+    return (a == 0.0 || within(biased_exp(a), 900u)) && within(biased_exp(b), 1000u) && (a == 0.0 || within(biased_exp(quotient), 900u));
 }
 
 }  // namespace hype

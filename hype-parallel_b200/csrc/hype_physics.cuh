@@ -167,8 +167,9 @@ __device__ __forceinline__ bool frac_in(double x) { return (unsigned)__double2hi
 
 // How a system's functions divide.  IeeeDiv: the compiler's division.  CrDiv: the
 // branch-free correctly rounded forms of hype_div.cuh, whose chains interleave; the values
-// named to pos() and frac() bound every operand, and where one is outside (or a divisor's
-// word is all ones) special() holds and the caller repeats the function with IeeeDiv.
+// named to pos(), frac(), mag(), den() and num() bound every operand, and where one is outside
+// (or a divisor's significand is all ones) special() holds and the caller repeats the function
+// with IeeeDiv.
 struct IeeeDiv {
     __device__ __forceinline__ double operator()(double a, double b) const { return a / b; }
     __device__ __forceinline__ double by_const(double a, double b, double) const { return a / b; }   // third: 1/b, correctly rounded
@@ -845,7 +846,7 @@ __device__ __forceinline__ void weno3_1d(double u_m2, double u_m1, double u_0, d
 // reciprocals and quotients of hype_div.cuh: the bits of weno3_1d / Recon<2>.  Every weight
 // is gamma_k / d_k with d_k = (IS_k + 1e-12)^4 >= 1e-48 and is then divided by the weights'
 // sum.  With every d_k below 2^400 all operands and quotients lie in div_rn's range; that and
-// the divisors' low words are tested on the integer pipe, once per direction.  Where a test
+// the divisors' significands (all ones) are tested on the integer pipe, once per direction.  Where a test
 // fails (or for a NaN) `special` is set and the caller recomputes with Recon<2>.  The
 // compiler's divisions each end in a branch, so a warp waits out one chain after the other;
 // these interleave: Kapila 2048^2 right-hand side 1.76 -> 1.59 ms, BN 1024^2 0.896 -> 0.780,

@@ -327,10 +327,11 @@ HYPE_API int hype_test_skip_row_loads(hype_solver *s, int row);
  * kernels use (csrc/hype_div.cuh); no counterpart in the reference.  On device
  * `device`, n operand pairs drawn from `seed` -- random bit patterns (zeros,
  * subnormals, infinities and NaNs included), random operands of every exponent,
- * near-midpoint quotients and divisors with an all-ones significand -- are
- * divided both ways.  *mismatches counts reciprocals and quotients that differ
- * from IEEE division bit for bit although the operands are in the functions'
- * range, *specials the pairs out of it (where their callers use IEEE division).
+ * near-midpoint quotients, divisors with an all-ones significand or low word,
+ * zero numerators -- are divided both ways.  *mismatches counts reciprocals and
+ * quotients that differ from IEEE division bit for bit (zeros: in value) although
+ * the operands are in the functions' range or accepted by one of the kernels' own
+ * tests of their operands, *specials the pairs out of the functions' range.
  */
 HYPE_API int hype_test_division(int device, long long n, unsigned long long seed, long long *mismatches, long long *specials);
 
