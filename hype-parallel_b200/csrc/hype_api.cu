@@ -218,7 +218,6 @@ static int apply_tiling(hype_solver *s, const Shape &shape)
     CUDA_TRY(s, tile_configure(s, s->cells));
     s->strips = tile_strips(s, s->cells);
     s->runs = shape.runs;
-    s->waves = shape.waves;
     if (s->mixed) {
         for (int k = 0; k < 3; ++k)
             if ((rc = make_mixed_maps(s, &s->mm[k], s->mf[k], s->md[k]))) return rc;
@@ -300,8 +299,8 @@ static bool reads_aos(const hype_solver *s, const double *aos, const double *out
     return !s->mixed && s->row_off == 0 && !(s->cfg.flags & (HYPE_FLAG_VISCOUS | HYPE_FLAG_CONSERVATIVE)) &&
            (a & 15) == 0 && ((size_t)s->cfg.nx * s->nv) % 2 == 0;
 }
-// the right-hand side of runs run0 .. run0+run_count-1 (0: all) of `aos` into `out`, both cell-major
-static cudaError_t stage_rhs(hype_solver *s, const double *aos, double *out, int run0 = 0, int run_count = 0)
+// the right-hand side of `aos` into `out`, both cell-major
+static cudaError_t stage_rhs(hype_solver *s, const double *aos, double *out)
 {
     PFN_tmapEncodeTiled enc = get_encode();
     CUtensorMap m;
@@ -314,8 +313,6 @@ static cudaError_t stage_rhs(hype_solver *s, const double *aos, double *out, int
     StageParams p = base_params(s);
     p.in = aos; p.out = out; p.out_aos = 1; p.mode = OUT_RHS;
     p.reduce_smax = 1;
-    p.run0 = run0;
-    p.run_count = run_count;
     return s->fast ? launch_stage_fast_rhs(s->cfg.system, s->cfg.order, s->cells, m, p, s->stream)
                    : launch_stage_rhs(s->cfg.system, s->cfg.order, s->cells, m, p, s->stream);
 }
@@ -462,8 +459,9 @@ static int check_config(const hype_config *c, hype_solver *s)
 //  - up to 16 bands (rhs_bands; hype_advance_host: each launch half a wave of blocks, host_bands);
 //  - hype_rhs_prim: its one RHS launch, band by band behind the uploads
 //    (banded_upload_stage).  On a 2048^2 Kapila grid a call took 5.4-5.5 ms
-//    with 8 full-wave bands and 4.8 ms this way (the copies alone: 3.6 ms each
-//    way, 4.1 ms both ways at once);
+//    with 8 full-wave bands and takes 4.8-5.6 this way, from run to run, whether a
+//    stage takes 2.1 ms or 1.5 (the copies alone: 3.6 ms each way, 4.1 ms both
+//    ways at once);
 //  - hype_advance_host: every stage of the step as a wavefront over the bands
 //    (enqueue_step_banded).  Stage s runs on compute stream s % 4, so the four
 //    SSPRK(4,3) stages advance together, each band of stage s waiting only for
@@ -561,7 +559,7 @@ static Bands rhs_bands(const hype_solver *s)
 // wave of blocks
 static Bands host_bands(const hype_solver *s) { return make_bands(s, hype_solver::MAX_BANDS, wave_runs(s) / 2); }
 
-// the last band whose rows band k's stencils read (the halo is 3 rows, bands are >= 8)
+// the last band whose rows band k's stencils read (the halo is 3 rows, a band has 3 or more)
 static int band_needs(const hype_solver *s, const Bands &b, int k)
 {
     if (k == 0 && s->cfg.bc_bottom == HYPE_BC_PERIODIC) return b.n - 1;
@@ -1259,7 +1257,7 @@ int hype_advance(hype_solver *s, int nsteps)
 
 // One step enqueued by hand (the graph's content) as a wavefront of row bands:
 // band k of stage s reads the rows of bands k-1..k+1 of stage s-1 (3-row stencils,
-// bands of >= 8 rows; bands 0 and n-1 are neighbours on a periodic y axis) and
+// bands of 3 rows or more; bands 0 and n-1 are neighbours on a periodic y axis) and
 // waits for their events, stage 0 for the uploads of those bands (U_in).  Stage s
 // writes a buffer that only stage s-1 (or, for the combination's second operand,
 // the same band of an earlier stage) still reads, so the same dependency covers

@@ -275,8 +275,11 @@ static double shape_cost(const hype_batch *b, const Kind &k, int cells, int rows
         tallest = std::max(tallest, h);
     }
     const long long slots = (long long)b->sms * bps;
-    // the persistent FP64 kernels spill at 128 columns (their parameters are in shared memory, not in
-    // the constant bank): 48 grids of sides 200..1024 take 34.1 ms a step with them, 31.1 with 64
+    // the persistent FP64 kernels lose more at 128 columns than lone solvers' do (their parameters
+    // are in shared memory, not in the constant bank).  128 columns against 64 with the same rows,
+    // 16..128, 24 grids of sides 200..700: Kapila N = 1 0.99-1.02, N = 2 0.95-1.08, N = 3 1.12-1.16, BN
+    // 1.07-1.13, Euler N = 2 1.04-1.12, N = 3 0.94-0.97; 48 grids of 200..1024, Kapila N = 2, 1.10.  With
+    // it the estimated step is within 6 % of the best of those shapes in 12 of 14 such batches
     const double spill = !k.mixed && cells == STAGE_CELLS ? 1.1 : 1.0;
     if (tiles <= slots) return spill * tile_launch_cost(k.mixed, cells, b->sms, bps, tiles, tallest);
     return spill * tile_iteration_cost(k.mixed, cells, bps) * (0.1 * (double)iters10 / (double)slots + 0.4 * (tallest + 2.7));

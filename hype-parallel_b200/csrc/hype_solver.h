@@ -41,7 +41,6 @@ struct hype_solver {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaGraphExec_t step_exec = nullptr;
     int cells = hype::STAGE_CELLS;          // tile width of the stage kernel
-    int waves = 1;                    // row runs per strip = waves x (SM slots / strips)
     int sms = 0;
     int strips = 1, runs = 1;         // tile decomposition of the grid
     int bps = 0;                      // stage blocks per SM

@@ -34,11 +34,12 @@
 // bottom and volume values in registers.
 //
 // What bounds the tile is FP64 issue: dependent FP64 chains at 8 or 16 warps per SM.
-// With the point values in one pass, the admissibility divisions left to the few cells
-// that need them and no sums or shuffles of products that are zero, the Kapila N = 2
-// tile executes 9.54e8 warp instructions per 2048^2 right-hand side instead of 1.21e9
-// (3.8 k FP64 instructions a cell instead of 5.0 k) and the call takes 1.76 ms instead of
-// 2.09; Euler 1531x897 0.380 ms instead of 0.417, BN 1024^2 0.896 instead of 0.947.
+// Point values come from one pass, the admissibility divisions are left to the few cells
+// that need them, products that are zero take no sums or shuffles, and divisions are
+// branch-free chains that interleave (hype_div.cuh).  Right-hand sides from and to device
+// memory: Kapila N = 2 2048^2 1.48 ms, Euler 1531x897 0.288, BN 1024^2 0.652, Kapila N = 3 500^2
+// 0.167; with a pass per use of the point values, the compiler's divisions and a conversion
+// to planes 2.09, 0.414, 0.945 and 0.278.
 //
 // Two block barriers a row (where the fluxes share the coefficients' memory, also a count
 // of the warps that have read their neighbours', which a warp waits for before its first
@@ -177,7 +178,6 @@ struct StageKernel {
     static constexpr size_t smem_bytes() { return SMEM; }
 };
 
-__device__ __forceinline__ int hi_word(double x) { return __double2hiint(x); }
 // x with its sign flipped where mask = 0x80000000 (0: unchanged)
 __device__ __forceinline__ double flip_sign(double x, unsigned mask)
 {
@@ -257,7 +257,7 @@ __device__ __forceinline__ double vol_grad(const double *cf, unsigned mask)
 // Gradient component D (0: x, 1: y) of one variable at Gauss point q of face
 // F from its unlimited coefficients uc: sum_k uc[k] gradphiFace_D(F, q, k) from
 // 0.0 in ascending k (rhs_function_prim.c:362-369), before the 1/h factor.
-// Zero basis gradients are dropped as in face_val.
+// Terms of zero basis gradients are dropped (add_term).
 template <int N, int F, int D>
 __device__ __forceinline__ double face_grad(const double *uc, int q)
 {
