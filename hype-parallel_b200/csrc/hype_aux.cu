@@ -425,10 +425,8 @@ __global__ void division_check_kernel(long long n, unsigned long long seed, unsi
         auto wrong = [&](double q, double r) { return a == 0.0 ? !(q == r) : __double_as_longlong(q) != __double_as_longlong(r); };
         // the functions in their whole range
         if (hype::div_in_range(a, b, ref)) {
-            // a divisor that rcp_rn leaves to its caller (all ones): the constant divisors' way
-            const bool ones = hype::rcp_special(hype::rcp_low(0u, b));
-            const double y = ones ? 1.0 / b : hype::rcp_rn(b);
-            if (!ones && __double_as_longlong(y) != __double_as_longlong(1.0 / b)) ++mism;
+            const double y = hype::rcp_rn(b);
+            if (__double_as_longlong(y) != __double_as_longlong(1.0 / b)) ++mism;
             if (wrong(hype::div_rn(a, b, y), ref)) ++mism;
         } else {
             ++spec;
@@ -441,6 +439,8 @@ __global__ void division_check_kernel(long long n, unsigned long long seed, unsi
             dv.den(b);
             const double q = dv(a, b);
             if (!dv.special() && wrong(q, ref)) ++mism;
+            // operands well within the range are accepted, whatever their significands
+            if (dv.special() && (a == 0.0 || (fabs(a) > 0x1p-299 && fabs(a) < 0x1p199)) && fabs(b) > 0x1p-299 && fabs(b) < 0x1p299) ++mism;
         }
         {
             hype::CrDiv dv;
@@ -462,7 +462,7 @@ __global__ void division_check_kernel(long long n, unsigned long long seed, unsi
             const double d = fmax(fabs(b), 1e-48);
             ck.divisor(d);
             if (!ck.special()) {
-                const double y = hype::rcp_rn(d);
+                const double y = hype::rcp_near(d);
                 if (__double_as_longlong(y) != __double_as_longlong(1.0 / d)) ++mism;
                 if (__double_as_longlong(hype::div_rn(100.0, d, y)) != __double_as_longlong(100.0 / d)) ++mism;
             }

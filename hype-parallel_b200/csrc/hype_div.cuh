@@ -18,7 +18,7 @@ namespace hype {
 __device__ __forceinline__ unsigned biased_exp(double x) { return (unsigned)((__double_as_longlong(x) >> 52) & 0x7ff); }
 
 // 1/b correctly rounded, for b normal with |binary exponent| <= 1000 and a significand
-// that is not all ones (rcp_special):
+// that is not all ones (rcp_ones):
 //   y0 ~ 1/b: the hardware approximation (PTX rcp.approx.ftz.f64, about 20 bits);
 //   y1 = y0 + y0 (e + e^2), e = 1 - b y0 (fma): the third-order iteration for the
 //        reciprocal, |y1 b - 1| below 0.51 ulp's worth, so y1 is one of the two doubles
@@ -26,7 +26,7 @@ __device__ __forceinline__ unsigned biased_exp(double x) { return (unsigned)((__
 //   y2 = y1 + y1 (1 - b y1), both by fma: rounds (1/b)(1 - e1^2), |e1| <= 2^-53; no midpoint
 //        of two doubles lies between that and 1/b unless b is all ones (Markstein 2000, ch. 8).
 // Five fused multiply-adds, no branch.
-__device__ __forceinline__ double rcp_rn(double b)
+__device__ __forceinline__ double rcp_near(double b)
 {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
@@ -36,12 +36,22 @@ __device__ __forceinline__ double rcp_rn(double b)
     e = fma(-b, y, 1.0);
     return fma(y, e, y);
 }
-// the divisors of rcp_rn folded together: all ones in one significand is the only doubtful case
-__device__ __forceinline__ unsigned rcp_low(unsigned fold, double b)
+// the low word of b, all ones only if the whole significand is
+__device__ __forceinline__ unsigned rcp_low(double b) { return (unsigned)__double2loint(b) & ((unsigned)__double2hiint(b) | 0xfff00000u); }
+__device__ __forceinline__ bool rcp_ones(unsigned low) { return low == 0xffffffffu; }
+
+// 1/b correctly rounded whatever the significand.  For b = 2^k (2 - 2^-52) (all ones) 1/b =
+// 2^-(k+1) (1 + 2^-53 + 2^-106 + ...) rounds to 2^-(k+1) (1 + 2^-52), and rcp_near gives that or the
+// double below it, 2^-(k+1), whose last bit is 0: setting the last bit is right for both.  Such
+// divisors are common: the density 1 - 2^-53 that (alpha rho) / alpha gives in quiescent gas, which
+// a Kapila N = 0 step of 2048^2 took 0.94 ms for when they were left to the compiler's
+// division, and takes 0.77.  The weights' divisors (CrCheck) are not, and there the three
+// integer operations cost 1 to 2 % (N = 3 500^2 168 -> 171 us, 256^2 steps 2.45 -> 2.48 ms).
+__device__ __forceinline__ double rcp_rn(double b)
 {
-    return max(fold, (unsigned)__double2loint(b) & ((unsigned)__double2hiint(b) | 0xfff00000u));
+    const double y = rcp_near(b);
+    return __hiloint2double(__double2hiint(y), __double2loint(y) | (rcp_ones(rcp_low(b)) ? 1 : 0));
 }
-__device__ __forceinline__ bool rcp_special(unsigned fold) { return fold == 0xffffffffu; }
 
 // a / b correctly rounded from y = rcp_rn(b): quotients by one divisor share y.  q1 = a y and one
 // correction give a double next to a/b, whose remainder a - b q1 is exact; with y the correctly

@@ -168,8 +168,7 @@ __device__ __forceinline__ bool frac_in(double x) { return (unsigned)__double2hi
 // How a system's functions divide.  IeeeDiv: the compiler's division.  CrDiv: the
 // branch-free correctly rounded forms of hype_div.cuh, whose chains interleave; the values
 // named to pos(), frac(), mag(), den() and num() bound every operand, and where one is outside
-// (or a divisor's significand is all ones) special() holds and the caller repeats the function
-// with IeeeDiv.
+// special() holds and the caller repeats the function with IeeeDiv.
 struct IeeeDiv {
     __device__ __forceinline__ double operator()(double a, double b) const { return a / b; }
     __device__ __forceinline__ double by_const(double a, double b, double) const { return a / b; }   // third: 1/b, correctly rounded
@@ -182,11 +181,10 @@ struct IeeeDiv {
     __device__ __forceinline__ void den(double) const {}
 };
 struct CrDiv {
-    unsigned lo = 0;
     bool in = true;
-    __device__ __forceinline__ double operator()(double a, double b) { return div_rn(a, b, rcp(b)); }
+    __device__ __forceinline__ double operator()(double a, double b) const { return div_rn(a, b, rcp_rn(b)); }
     __device__ __forceinline__ double by_const(double a, double b, double rb) const { return div_rn(a, b, rb); }
-    __device__ __forceinline__ double rcp(double b) { lo = rcp_low(lo, b); return rcp_rn(b); }
+    __device__ __forceinline__ double rcp(double b) const { return rcp_rn(b); }
     __device__ __forceinline__ double quot(double a, double b, double y) const { return div_rn(a, b, y); }
     __device__ __forceinline__ void pos(double x) { in = in && exp_in<-100, 100>(x); }    // a density, a p + P_inf
     __device__ __forceinline__ void frac(double x) { in = in && exp_in<-100, 0>(x); }     // a volume fraction
@@ -199,7 +197,7 @@ struct CrDiv {
         const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
         in = in && (h - ((1023u - 300u) << 20) < (500u << 20) || (h | (unsigned)__double2loint(x)) == 0u);
     }
-    __device__ __forceinline__ bool special() const { return !in || rcp_special(lo); }
+    __device__ __forceinline__ bool special() const { return !in; }
 };
 
 // ---------------------------------------------------------------------------
@@ -846,16 +844,16 @@ __device__ __forceinline__ void weno3_1d(double u_m2, double u_m1, double u_0, d
 // reciprocals and quotients of hype_div.cuh: the bits of weno3_1d / Recon<2>.  Every weight
 // is gamma_k / d_k with d_k = (IS_k + 1e-12)^4 >= 1e-48 and is then divided by the weights'
 // sum.  With every d_k below 2^400 all operands and quotients lie in div_rn's range; that and
-// the divisors' significands (all ones) are tested on the integer pipe, once per direction.  Where a test
-// fails (or for a NaN) `special` is set and the caller recomputes with Recon<2>.  The
+// significands of all ones are tested on the integer pipe, once per cell and variable.  Where a
+// test fails (or for a NaN) `special` is set and the caller recomputes with Recon<2>.  The
 // compiler's divisions each end in a branch, so a warp waits out one chain after the other;
 // these interleave: Kapila 2048^2 right-hand side 1.76 -> 1.59 ms, BN 1024^2 0.896 -> 0.780,
 // Euler 1531x897 0.380 -> 0.334.
 struct CrCheck {
     unsigned hi = 0, lo = 0;
-    __device__ __forceinline__ void divisor(double d) { hi = max(hi, (unsigned)__double2hiint(d)); lo = rcp_low(lo, d); }
-    __device__ __forceinline__ void sum(double t) { lo = rcp_low(lo, t); }
-    __device__ __forceinline__ bool special() const { return hi >= ((1023u + 400u) << 20) || rcp_special(lo); }
+    __device__ __forceinline__ void divisor(double d) { hi = max(hi, (unsigned)__double2hiint(d)); sum(d); }
+    __device__ __forceinline__ void sum(double t) { lo = max(lo, rcp_low(t)); }
+    __device__ __forceinline__ bool special() const { return hi >= ((1023u + 400u) << 20) || rcp_ones(lo); }
 };
 
 __device__ __forceinline__ void weno3_1d_cr(double u_m2, double u_m1, double u_0, double u_p1, double u_p2, double &slope,
@@ -871,12 +869,12 @@ __device__ __forceinline__ void weno3_1d_cr(double u_m2, double u_m1, double u_0
     double IS1 = ux1 * ux1 + R13_3 * uxx1 * uxx1; const double d1 = pow4(IS1 + SMALL_NUM);
     double IS2 = ux2 * ux2 + R13_3 * uxx2 * uxx2; const double d2 = pow4(IS2 + SMALL_NUM);
     ck.divisor(d0); ck.divisor(d1); ck.divisor(d2);
-    double w0 = rcp_rn(d0);
-    double w1 = div_rn(central_cell_wt, d1, rcp_rn(d1));
-    double w2 = rcp_rn(d2);
+    double w0 = rcp_near(d0);
+    double w1 = div_rn(central_cell_wt, d1, rcp_near(d1));
+    double w2 = rcp_near(d2);
     const double total = w0 + w1 + w2;
     ck.sum(total);
-    const double y = rcp_rn(total);
+    const double y = rcp_near(total);
     w0 = div_rn(w0, total, y);
     w1 = div_rn(w1, total, y);
     w2 = div_rn(w2, total, y);
@@ -901,10 +899,10 @@ struct Recon2Cr {
         double IS2 = temp + uxy2 * uxy2; const double d2 = pow4(IS2 + SMALL_NUM);
         double IS3 = temp + uxy3 * uxy3; const double d3 = pow4(IS3 + SMALL_NUM);
         ck.divisor(d0); ck.divisor(d1); ck.divisor(d2); ck.divisor(d3);
-        double w0 = rcp_rn(d0), w1 = rcp_rn(d1), w2 = rcp_rn(d2), w3 = rcp_rn(d3);
+        double w0 = rcp_near(d0), w1 = rcp_near(d1), w2 = rcp_near(d2), w3 = rcp_near(d3);
         const double total = w0 + w1 + w2 + w3;
         ck.sum(total);
-        const double y = rcp_rn(total);
+        const double y = rcp_near(total);
         w0 = div_rn(w0, total, y); w1 = div_rn(w1, total, y); w2 = div_rn(w2, total, y); w3 = div_rn(w3, total, y);
         c[5] = w0 * uxy0 + w1 * uxy1 + w2 * uxy2 + w3 * uxy3;
         sp = ck.special();
@@ -954,7 +952,7 @@ struct Recon3 {
     __device__ __forceinline__ static void weights(const Stencil &s, double *coeffs, CrCheck &ck)
     {
         auto over_d = [&](double g, double d) {
-            if constexpr (CR) { ck.divisor(d); return div_rn(g, d, rcp_rn(d)); }
+            if constexpr (CR) { ck.divisor(d); return div_rn(g, d, rcp_near(d)); }
             else return g / d;
         };
         constexpr double gammaHi = 0.85, gammaLo = 0.85;
@@ -1016,7 +1014,7 @@ struct Recon3 {
         double wt_ratio;
         if constexpr (CR) {
             ck.sum(sum);
-            const double y = rcp_rn(sum);
+            const double y = rcp_near(sum);
             w_R4 = div_rn(w_R4, sum, y);
 #pragma unroll
             for (int i = 0; i < 5; ++i) w_R3[i] = div_rn(w_R3[i], sum, y);
