@@ -20,9 +20,9 @@ __device__ __forceinline__ unsigned biased_exp(double x) { return (unsigned)((__
 // 1/b correctly rounded, for b normal with |binary exponent| <= 1000 and a significand
 // that is not all ones (rcp_ones):
 //   y0 ~ 1/b: the hardware approximation (PTX rcp.approx.ftz.f64, about 20 bits);
-//   y1 = y0 + y0 (e + e^2), e = 1 - b y0 (fma): the third-order iteration for the
-//        reciprocal, |y1 b - 1| below 0.51 ulp's worth, so y1 is one of the two doubles
-//        around 1/b;
+//   y1 = y0 + e s, s = y0 + y0 e, e = 1 - b y0: Chebyshev's third-order iteration y0 (1 + e + e^2)
+//        by Horner's rule.  s rounds to 2^-53 of itself, 2^-73 of y1, and e^3 is about 2^-60, so y1
+//        is one of the two doubles around 1/b;
 //   y2 = y1 + y1 (1 - b y1), both by fma: rounds (1/b)(1 - e1^2), |e1| <= 2^-53; no midpoint
 //        of two doubles lies between that and 1/b unless b is all ones (Markstein 2000, ch. 8).
 // Five fused multiply-adds, no branch.
@@ -30,11 +30,10 @@ __device__ __forceinline__ double rcp_near(double b)
 {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    double e = fma(-b, y, 1.0);
-    e = fma(e, e, e);
-    y = fma(y, e, y);
-    e = fma(-b, y, 1.0);
-    return fma(y, e, y);
+    const double e = fma(-b, y, 1.0);
+    const double s = fma(y, e, y);
+    y = fma(e, s, y);
+    return fma(y, fma(-b, y, 1.0), y);
 }
 // the low word of b, all ones only if the whole significand is
 __device__ __forceinline__ unsigned rcp_low(double b) { return (unsigned)__double2loint(b) & ((unsigned)__double2hiint(b) | 0xfff00000u); }
