@@ -722,10 +722,10 @@ __device__ __forceinline__ void stage_tile(const P &p, const CUtensorMap *tmap, 
                     });
                 }
             });
-            // the volume non-conservative products (rhs_function_prim.c:459-479).  CONS: of the run's own
+            // the volume non-conservative products (rhs_function_prim.c:459-479).  CONS, N > 0: of the run's own
             // rows (many divisions a point: Kapila N = 2 64^2 69.5 -> 61.5 us, 1024^2 0.752 -> 0.740 ms)
             if constexpr (NZ > 0) {
-                if (!CONS || full_row) static_for<QH>([&](auto sa) {
+                if (!CONS || N == 0 || full_row) static_for<QH>([&](auto sa) {
                     constexpr int a = decltype(sa)::value;
                     double B[NV];
                     if constexpr (CONS) S::ncp_cons(eos, Vv[a], gx[a], gy[a], B);
