@@ -452,8 +452,10 @@ static int rebuild_work(hype_batch *b, int id)
         if (n > l.work_cap) {
             int cap = l.work_cap > 0 ? l.work_cap : 1024;
             while (cap < n) cap *= 2;
+            int2 *grown = nullptr;   // before the present one goes: if there is no memory the graph still holds that
+            BCUDA(b, pool_alloc(b, &grown, sizeof(int2) * cap));
             pool_free(b, l.dWork);   // behind the queued steps; the graph that holds it is out of date from here
-            BCUDA(b, pool_alloc(b, &l.dWork, sizeof(int2) * cap));
+            l.dWork = grown;
             l.work_cap = cap;
             b->dirty = true;
         }
