@@ -540,9 +540,26 @@ static double pipeline_us(const hype_solver *s, int n, int runs)
     }
     return down;
 }
-static Bands rhs_bands(const hype_solver *s)
+// Pageable arrays (`staged`) are copied by the host copy pool, a band after the other, in parts of 1 MiB
+// or more for each of its threads: four bands, each of 512 KiB or more.  Milliseconds a call with
+// bands of 8-row runs, the estimated ones, four: Kapila 1021 x 767 2.59, 4.90, 2.35; 1024^2 4.24, 5.27,
+// 3.36; 512^2 1.38, 1.46, 0.90; 256^2 0.99, 0.91, 0.48; 2048^2 16.6, 14.6, 14.1; Euler 800 x 1500 2.81, 5.20,
+// 2.61; a slab of 2048 x 1024 8.98, 9.06, 6.94.
+static Bands rhs_bands(const hype_solver *s, bool staged)
 {
     const int ny = s->cfg.ny, half = wave_runs(s) / 2;
+    if (staged) {
+        const size_t bytes = sizeof(double) * (size_t)s->cfg.nx * ny * s->nv;
+        const int n = (int)std::max<size_t>(1, std::min<size_t>({4, bytes >> 19, (size_t)ny / 4}));
+        int runs = 1;
+        double least = 1e300;
+        for (int k = 1; k <= 4; ++k) {
+            const int r = std::max(1, std::min(half * k / 2, ny / n));
+            const double t = pipeline_us(s, n, r);
+            if (t < least) { least = t; runs = r; }
+        }
+        return split_bands(s, n * runs, n);
+    }
     Bands best = make_bands(s, hype_solver::MAX_BANDS, half);   // runs of 8 rows or more
     double least = 0.93 * pipeline_us(s, best.n, best.runs / best.n);
     int best_n = 0, best_runs = 0;
@@ -1028,11 +1045,11 @@ int hype_rhs_prim(hype_solver *s, double t, const double *U, double *RHS, double
     CUDA_TRY(s, cudaSetDevice(s->cfg.device));
     int rc;
     // banded: U's rows stream in while earlier bands compute, RHS rows stream out
-    const Bands b = rhs_bands(s);
+    HostIO io = host_io(s, U, RHS);
+    const Bands b = rhs_bands(s, io.stage_in || io.stage_out);
     const size_t row_elems = (size_t)s->cfg.nx * s->nv;
     if ((rc = fence_copy_streams(s)) || (rc = reset_scalars(s))) return rc;
     const PlanStage q{B_S0, B_NONE, OUT_RHS, 0.0, 1.0, 0.0, B_NONE, B_NONE, 1};
-    HostIO io = host_io(s, U, RHS);
     rc = banded_upload_stage(s, b, [&](int k) { return upload_band(s, b, k, U, B_S0, io); }, q, 1, s->dAosOut, [&](int k) -> int {
         // band k's RHS rows are final: copy them out while later bands compute
         const int r0 = b.row[k], nr = b.row[k + 1] - r0;
@@ -1084,9 +1101,9 @@ int hype_rhs_prim_slab(hype_solver *s, double t, const double *U, long long row_
     // the last band) are copied from the local array and converted, its RHS launch runs
     // once the rows its stencils read are there, and its RHS rows go to the host while
     // later bands compute
-    const Bands b = rhs_bands(s);
-    if ((rc = fence_copy_streams(s)) || (rc = reset_scalars(s))) return rc;
     HostIO io = host_io(s, U, RHS);
+    const Bands b = rhs_bands(s, io.stage_in || io.stage_out);
+    if ((rc = fence_copy_streams(s)) || (rc = reset_scalars(s))) return rc;
     auto upload = [&](int k) -> int {
         const int a = b.row[k] - (k == 0 ? lo : 0), e = b.row[k + 1] + (k == b.n - 1 ? hi : 0);   // local rows a .. e-1
         double *stg = s->dAosIn + (size_t)(a + 3) * srow;
