@@ -459,9 +459,8 @@ static int check_config(const hype_config *c, hype_solver *s)
 //  - up to 16 bands (rhs_bands; hype_advance_host: each launch half a wave of blocks, host_bands);
 //  - hype_rhs_prim: its one RHS launch, band by band behind the uploads
 //    (banded_upload_stage).  On a 2048^2 Kapila grid a call took 5.4-5.5 ms
-//    with 8 full-wave bands and takes 4.8-5.6 this way, from run to run, whether a
-//    stage takes 2.1 ms or 1.5 (the copies alone: 3.6 ms each way, 4.1 ms both
-//    ways at once);
+//    with 8 full-wave bands and takes 4.75 this way (the copies alone: 3.6 ms each
+//    way, 4.1 ms both ways at once);
 //  - hype_advance_host: every stage of the step as a wavefront over the bands
 //    (enqueue_step_banded).  Stage s runs on compute stream s % 4, so the four
 //    SSPRK(4,3) stages advance together, each band of stage s waiting only for
@@ -1047,17 +1046,30 @@ int hype_rhs_prim(hype_solver *s, double t, const double *U, double *RHS, double
     // banded: U's rows stream in while earlier bands compute, RHS rows stream out
     HostIO io = host_io(s, U, RHS);
     const Bands b = rhs_bands(s, io.stage_in || io.stage_out);
-    const size_t row_elems = (size_t)s->cfg.nx * s->nv;
     if ((rc = fence_copy_streams(s)) || (rc = reset_scalars(s))) return rc;
     const PlanStage q{B_S0, B_NONE, OUT_RHS, 0.0, 1.0, 0.0, B_NONE, B_NONE, 1};
-    rc = banded_upload_stage(s, b, [&](int k) { return upload_band(s, b, k, U, B_S0, io); }, q, 1, s->dAosOut, [&](int k) -> int {
-        // band k's RHS rows are final: copy them out while later bands compute
-        const int r0 = b.row[k], nr = b.row[k + 1] - r0;
-        CUDA_TRY(s, cudaEventRecord(s->ev_done[k], s->stream));
+    // band k's rows leave once its launch is done, between pinned arrays at the end of the next launch's
+    // upload: a download that begins amid an upload slows both (2048^2 Kapila 5.30 ms a call, Euler
+    // 3.77, this way 4.74 and 3.20; another upload later 4.94 and 3.34; pageable arrays lose by it)
+    const size_t row_elems = (size_t)s->cfg.nx * s->nv;
+    const bool late = !io.stage_in && !io.stage_out;
+    int held = -1;   // launched, its download not enqueued
+    auto download = [&](int upload) -> int {
+        const int k = held, r0 = b.row[k], nr = b.row[k + 1] - r0;
+        held = -1;
         CUDA_TRY(s, cudaStreamWaitEvent(s->cout, s->ev_done[k], 0));
+        if (upload >= 0) CUDA_TRY(s, cudaStreamWaitEvent(s->cout, s->ev_cp[upload], 0));
         return download_rows(s, io, k, RHS, r0 * row_elems, row_elems * nr);
+    };
+    rc = banded_upload_stage(s, b, [&](int k) { return upload_band(s, b, k, U, B_S0, io); }, q, 1, s->dAosOut, [&](int k) -> int {
+        int r;
+        if (held >= 0 && (r = download(band_needs(s, b, k)))) return r;
+        CUDA_TRY(s, cudaEventRecord(s->ev_done[k], s->stream));
+        held = k;
+        return late ? HYPE_OK : download(-1);
     });
     if (rc) return rc;
+    if (held >= 0 && (rc = download(-1))) return rc;
     if ((rc = finish_downloads(s, io, RHS))) return rc;
     if ((rc = read_scalars(s)) && rc != HYPE_ERR_INADMISSIBLE) return rc;
     if (dt) {
