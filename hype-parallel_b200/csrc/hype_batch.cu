@@ -49,9 +49,10 @@ int kind_of(const hype_config &c)
     return (cons ? KIND_CONS0 : 0) + c.system * 4 + c.order;
 }
 
-// the persistent kernel family of a kind: -1 the primitive path's, else BATCH_PATH_*
+// the persistent kernel family of a kind: -1 the primitive path's and the mixed ones, else BATCH_PATH_*
 int path_of_kind(int id)
 {
+    if (kind_is_mixed(id)) return -1;
     if (id >= KIND_VISC_CONS0) return BATCH_PATH_VISC_CONS;
     if (id >= KIND_VISC0) return BATCH_PATH_VISC;
     if (id >= KIND_CONS0) return BATCH_PATH_CONS;
