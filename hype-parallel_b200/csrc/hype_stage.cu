@@ -4,14 +4,16 @@
 // host dispatch over (system, order, tile width).  The tile itself is
 // stage_tile in hype_stage_tile.cuh.
 //
-// Compiled once with HYPE_STAGE_SYS and HYPE_STAGE_ORDER for each system and order (the kernels, side
-// by side in as many compiler processes) and once without (the dispatch).  An object is one module,
-// which a process loads whole with its first kernel.
+// Compiled with HYPE_STAGE_SYS and HYPE_STAGE_ORDER for each system and order, once for the grid form and
+// once, with HYPE_STAGE_BATCH, for the persistent one (the kernels, side by side in as many compiler
+// processes), and once without (the dispatch).  An object is one module, which a process loads
+// whole with its first kernel.
 //
 // Built with --fmad=false: arithmetic rounds exactly as the reference's C does.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <initializer_list>
+#include <type_traits>
 #include "hype_stage_tile.cuh"
 
 namespace hype {
@@ -20,17 +22,23 @@ namespace hype {
 struct StageEntry {
     const void *single;
     const void *rhs;
-    const void *axpy, *mix;                // of the whole grid, by mode
-    const void *batch_axpy, *batch_mix, *batch_rk;   // batch_rk: N = 3's fifth stage, else null
+    const void *axpy, *mix;   // of the whole grid, by mode
     size_t smem;
     int threads;
     int aos_box;   // elements of one part of a cell-major row's box
     int mix_mode;
 };
+struct BatchEntry {
+    const void *axpy, *mix, *rk;   // by mode; rk: N = 3's fifth stage, else null
+    size_t smem;
+    int threads;
+    int mix_mode;
+};
 
 template <int SYS, int N> StageEntry stage_entry_of(int cells);
+template <int SYS, int N> BatchEntry batch_entry_of(int cells);
 
-#ifdef HYPE_STAGE_SYS
+#if defined(HYPE_STAGE_SYS) && !defined(HYPE_STAGE_BATCH)
 template <int SYS, int N, int CELLS>
 __global__ void __launch_bounds__(2 * CELLS, (StageKernel<SYS, N, CELLS>::MIN_BLOCKS))
 stage_kernel(const __grid_constant__ CUtensorMap tmap, const StageParams p)
@@ -57,6 +65,30 @@ stage_rhs_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant
     stage_tile<SYS, N, CELLS, false, false, false, true>(p, &tmap, blockIdx.x, p.run0 + (int)blockIdx.y, smem_raw);
 }
 
+template <int SYS, int N, int CELLS>
+static StageEntry entry_of()
+{
+    using K = StageKernel<SYS, N, CELLS>;
+    auto fn = [](auto *f) { return reinterpret_cast<const void *>(f); };
+    StageEntry e{};
+    e.single = fn(stage_kernel<SYS, N, CELLS>);
+    e.rhs = fn(stage_rhs_kernel<SYS, N, CELLS>);
+    e.axpy = fn(stage_mode_kernel<SYS, N, CELLS, OUT_AXPY>);
+    if constexpr (N > 0) e.mix = fn(stage_mode_kernel<SYS, N, CELLS, MIX_MODE<N>>);
+    e.smem = K::smem_bytes();
+    e.threads = 2 * CELLS;
+    e.aos_box = K::AOS_BOX;
+    e.mix_mode = MIX_MODE<N>;
+    return e;
+}
+
+template <int SYS, int N>
+StageEntry stage_entry_of(int cells)
+{
+    return cells == 64 ? entry_of<SYS, N, 64>() : entry_of<SYS, N, 128>();
+}
+template StageEntry stage_entry_of<HYPE_STAGE_SYS, HYPE_STAGE_ORDER>(int cells);
+#elif defined(HYPE_STAGE_SYS)
 // Persistent form: the block walks a list of (grid, tile) work items; every grid
 // has its own parameters, tensor map and device scalars.
 template <int SYS, int N, int CELLS, int MODE>
@@ -88,55 +120,56 @@ stage_batch_kernel(const StageParams *__restrict__ inst, const CUtensorMap *__re
 }
 
 template <int SYS, int N, int CELLS>
-static StageEntry entry_of()
+static BatchEntry entry_of()
 {
     using K = StageKernel<SYS, N, CELLS>;
     auto fn = [](auto *f) { return reinterpret_cast<const void *>(f); };
-    StageEntry e{};
-    e.single = fn(stage_kernel<SYS, N, CELLS>);
-    e.rhs = fn(stage_rhs_kernel<SYS, N, CELLS>);
-    e.axpy = fn(stage_mode_kernel<SYS, N, CELLS, OUT_AXPY>);
-    e.batch_axpy = fn(stage_batch_kernel<SYS, N, CELLS, OUT_AXPY>);
-    if constexpr (N > 0) {
-        e.mix = fn(stage_mode_kernel<SYS, N, CELLS, MIX_MODE<N>>);
-        e.batch_mix = fn(stage_batch_kernel<SYS, N, CELLS, MIX_MODE<N>>);
-    }
-    if constexpr (N == 3) e.batch_rk = fn(stage_batch_kernel<SYS, N, CELLS, OUT_RK104_5>);
+    BatchEntry e{};
+    e.axpy = fn(stage_batch_kernel<SYS, N, CELLS, OUT_AXPY>);
+    if constexpr (N > 0) e.mix = fn(stage_batch_kernel<SYS, N, CELLS, MIX_MODE<N>>);
+    if constexpr (N == 3) e.rk = fn(stage_batch_kernel<SYS, N, CELLS, OUT_RK104_5>);
     e.smem = K::smem_bytes();
     e.threads = 2 * CELLS;
-    e.aos_box = K::AOS_BOX;
     e.mix_mode = MIX_MODE<N>;
     return e;
 }
 
 template <int SYS, int N>
-StageEntry stage_entry_of(int cells)
+BatchEntry batch_entry_of(int cells)
 {
     return cells == 64 ? entry_of<SYS, N, 64>() : entry_of<SYS, N, 128>();
 }
-template StageEntry stage_entry_of<HYPE_STAGE_SYS, HYPE_STAGE_ORDER>(int cells);
+template BatchEntry batch_entry_of<HYPE_STAGE_SYS, HYPE_STAGE_ORDER>(int cells);
 #else
 // ---------------------------------------------------------------------------
 // host dispatch over (system, order, tile width)
 // ---------------------------------------------------------------------------
-template <int SYS>
-static StageEntry entry_sys(int order, int cells)
+template <int SYS, class Of>
+static auto entry_sys(int order, Of of)
 {
     switch (order) {
-    case 0: return stage_entry_of<SYS, 0>(cells);
-    case 1: return stage_entry_of<SYS, 1>(cells);
-    case 2: return stage_entry_of<SYS, 2>(cells);
-    default: return stage_entry_of<SYS, 3>(cells);
+    case 0: return of(std::integral_constant<int, SYS>{}, std::integral_constant<int, 0>{});
+    case 1: return of(std::integral_constant<int, SYS>{}, std::integral_constant<int, 1>{});
+    case 2: return of(std::integral_constant<int, SYS>{}, std::integral_constant<int, 2>{});
+    default: return of(std::integral_constant<int, SYS>{}, std::integral_constant<int, 3>{});
     }
 }
-
-static StageEntry stage_entry(int sys, int order, int cells)
+template <class Of>
+static auto entry(int sys, int order, Of of)
 {
     switch (sys) {
-    case SYS_EULER: return entry_sys<SYS_EULER>(order, cells);
-    case SYS_KAPILA: return entry_sys<SYS_KAPILA>(order, cells);
-    default: return entry_sys<SYS_BN>(order, cells);
+    case SYS_EULER: return entry_sys<SYS_EULER>(order, of);
+    case SYS_KAPILA: return entry_sys<SYS_KAPILA>(order, of);
+    default: return entry_sys<SYS_BN>(order, of);
     }
+}
+static StageEntry stage_entry(int sys, int order, int cells)
+{
+    return entry(sys, order, [cells](auto s, auto n) { return stage_entry_of<decltype(s)::value, decltype(n)::value>(cells); });
+}
+static BatchEntry batch_entry(int sys, int order, int cells)
+{
+    return entry(sys, order, [cells](auto s, auto n) { return batch_entry_of<decltype(s)::value, decltype(n)::value>(cells); });
 }
 
 size_t stage_smem_bytes(int sys, int order, int cells) { return stage_entry(sys, order, cells).smem; }
@@ -168,11 +201,11 @@ int stage_blocks_per_sm(int sys, int order, int cells)
 
 int stage_batch_blocks_per_sm(int sys, int order, int cells)
 {
-    const StageEntry e = stage_entry(sys, order, cells);
+    const BatchEntry e = batch_entry(sys, order, cells);
     int nb = 0;
-    // `single` gives the dt of an instance that joins
-    if (allow_smem({e.single, e.batch_axpy, e.batch_mix, e.batch_rk}, e.smem) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, e.batch_axpy, e.threads, e.smem) != cudaSuccess) return 0;
+    // the grid form's `single` gives the dt of an instance that joins
+    if (allow_smem({stage_entry(sys, order, cells).single, e.axpy, e.mix, e.rk}, e.smem) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, e.axpy, e.threads, e.smem) != cudaSuccess) return 0;
     return nb;
 }
 
@@ -204,9 +237,9 @@ cudaError_t launch_stage_rhs(int sys, int order, int cells, const CUtensorMap &t
 cudaError_t launch_stage_batch(int sys, int order, int cells, int mode, const StageParams *inst, const CUtensorMap *tmaps,
                                const int2 *work, int *sched, int blocks, cudaStream_t s)
 {
-    const StageEntry e = stage_entry(sys, order, cells);
+    const BatchEntry e = batch_entry(sys, order, cells);
     void *args[] = {&inst, &tmaps, &work, &sched};
-    const void *f = mode == OUT_AXPY ? e.batch_axpy : mode == OUT_RK104_5 ? e.batch_rk : mode == e.mix_mode ? e.batch_mix : nullptr;
+    const void *f = mode == OUT_AXPY ? e.axpy : mode == OUT_RK104_5 ? e.rk : mode == e.mix_mode ? e.mix : nullptr;
     if (!f) return cudaErrorInvalidValue;
     return cudaLaunchKernel(f, dim3((unsigned)blocks, 1, 1), dim3((unsigned)e.threads, 1, 1), args, e.smem, s);
 }
