@@ -462,7 +462,7 @@ __global__ void division_check_kernel(long long n, unsigned long long seed, unsi
             const double d = fmax(fabs(b), 1e-48);
             ck.divisor(d);
             if (!ck.special()) {
-                const double y = hype::rcp_near(d);
+                const double y = hype::rcp_rn(d);
                 if (__double_as_longlong(y) != __double_as_longlong(1.0 / d)) ++mism;
                 if (__double_as_longlong(hype::div_rn(100.0, d, y)) != __double_as_longlong(100.0 / d)) ++mism;
             }

@@ -17,39 +17,30 @@ namespace hype {
 
 __device__ __forceinline__ unsigned biased_exp(double x) { return (unsigned)((__double_as_longlong(x) >> 52) & 0x7ff); }
 
-// 1/b correctly rounded, for b normal with |binary exponent| <= 1000 and a significand
-// that is not all ones (rcp_ones):
-//   y0 ~ 1/b: the hardware approximation (PTX rcp.approx.ftz.f64, about 20 bits);
+// 1/b correctly rounded, for b normal with |binary exponent| <= 1000:
+//   y0 ~ 1/b: the hardware approximation (PTX rcp.approx.ftz.f64, about 20 bits, its low word zero)
+//        with 2^31 as its low word: about 2^-21 more than the approximation;
 //   y1 = y0 + e s, s = y0 + y0 e, e = 1 - b y0: Chebyshev's third-order iteration y0 (1 + e + e^2)
-//        by Horner's rule.  s rounds to 2^-53 of itself, 2^-73 of y1, and e^3 is about 2^-60, so y1
-//        is one of the two doubles around 1/b;
+//        by Horner's rule, (1/b)(1 - e^3).  s rounds to 2^-53 of itself, 2^-73 of y1, and e^3 is below
+//        2^-57, so y1 is one of the two doubles around 1/b;
 //   y2 = y1 + y1 (1 - b y1), both by fma: rounds (1/b)(1 - e1^2), |e1| <= 2^-53; no midpoint
 //        of two doubles lies between that and 1/b unless b is all ones (Markstein 2000, ch. 8).
-// Five fused multiply-adds, no branch.
-__device__ __forceinline__ double rcp_near(double b)
+// For b = 2^k (2 - 2^-52), all ones, 1/b = L (1 + 2^-53 + 2^-106 + ...), L = 2^-(k+1), lies just above
+// the midpoint of L and U = L (1 + 2^-52).  y0 = L (1 + 2^-21) is above it, so e < 0, y1 above the
+// midpoint by about 2^-63 L, which its rounding errors of 2^-74 L leave, and rounds to U; then
+// y2 = U (1 - 2^-53 + 2^-105) = L (1 + 2^-53 + 2^-157) rounds to U, which is right.  (From y0 = L, y1 is
+// the midpoint itself and both steps end on L.)
+// Five fused multiply-adds, no branch.  All-ones divisors are common: the density 1 - 2^-53 that
+// (alpha rho) / alpha gives in quiescent gas.
+__device__ __forceinline__ double rcp_rn(double b)
 {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = __hiloint2double(__double2hiint(y), (int)0x80000000u);
     const double e = fma(-b, y, 1.0);
     const double s = fma(y, e, y);
     y = fma(e, s, y);
     return fma(y, fma(-b, y, 1.0), y);
-}
-// the low word of b, all ones only if the whole significand is
-__device__ __forceinline__ unsigned rcp_low(double b) { return (unsigned)__double2loint(b) & ((unsigned)__double2hiint(b) | 0xfff00000u); }
-__device__ __forceinline__ bool rcp_ones(unsigned low) { return low == 0xffffffffu; }
-
-// 1/b correctly rounded whatever the significand.  For b = 2^k (2 - 2^-52) (all ones) 1/b =
-// 2^-(k+1) (1 + 2^-53 + 2^-106 + ...) rounds to 2^-(k+1) (1 + 2^-52), and rcp_near gives that or the
-// double below it, 2^-(k+1), whose last bit is 0: setting the last bit is right for both.  Such
-// divisors are common: the density 1 - 2^-53 that (alpha rho) / alpha gives in quiescent gas, which
-// a Kapila N = 0 step of 2048^2 took 0.94 ms for when they were left to the compiler's
-// division, and takes 0.77.  The weights' divisors (CrCheck) are not, and there the three
-// integer operations cost 1 to 2 % (N = 3 500^2 168 -> 171 us, 256^2 steps 2.45 -> 2.48 ms).
-__device__ __forceinline__ double rcp_rn(double b)
-{
-    const double y = rcp_near(b);
-    return __hiloint2double(__double2hiint(y), __double2loint(y) | (rcp_ones(rcp_low(b)) ? 1 : 0));
 }
 
 // a / b correctly rounded from y = rcp_rn(b): quotients by one divisor share y.  q1 = a y and one

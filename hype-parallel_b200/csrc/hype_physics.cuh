@@ -843,17 +843,16 @@ __device__ __forceinline__ void weno3_1d(double u_m2, double u_m1, double u_0, d
 // reconstruction.c:157-178 and :144-221 with the branch-free correctly rounded
 // reciprocals and quotients of hype_div.cuh: the bits of weno3_1d / Recon<2>.  Every weight
 // is gamma_k / d_k with d_k = (IS_k + 1e-12)^4 >= 1e-48 and is then divided by the weights'
-// sum.  With every d_k below 2^400 all operands and quotients lie in div_rn's range; that and
-// significands of all ones are tested on the integer pipe, once per cell and variable.  Where a
-// test fails (or for a NaN) `special` is set and the caller recomputes with Recon<2>.  The
+// sum.  With every d_k below 2^400 all operands and quotients lie in div_rn's range; that is
+// tested on the integer pipe, once per cell and variable.  Where the test fails (or for a NaN)
+// `special` is set and the caller recomputes with Recon<2>.  The
 // compiler's divisions each end in a branch, so a warp waits out one chain after the other;
 // these interleave: Kapila 2048^2 right-hand side 1.76 -> 1.59 ms, BN 1024^2 0.896 -> 0.780,
 // Euler 1531x897 0.380 -> 0.334.
 struct CrCheck {
-    unsigned hi = 0, lo = 0;
-    __device__ __forceinline__ void divisor(double d) { hi = max(hi, (unsigned)__double2hiint(d)); sum(d); }
-    __device__ __forceinline__ void sum(double t) { lo = max(lo, rcp_low(t)); }
-    __device__ __forceinline__ bool special() const { return hi >= ((1023u + 400u) << 20) || rcp_ones(lo); }
+    unsigned hi = 0;
+    __device__ __forceinline__ void divisor(double d) { hi = max(hi, (unsigned)__double2hiint(d)); }
+    __device__ __forceinline__ bool special() const { return hi >= ((1023u + 400u) << 20); }
 };
 
 __device__ __forceinline__ void weno3_1d_cr(double u_m2, double u_m1, double u_0, double u_p1, double u_p2, double &slope,
@@ -869,12 +868,11 @@ __device__ __forceinline__ void weno3_1d_cr(double u_m2, double u_m1, double u_0
     double IS1 = ux1 * ux1 + R13_3 * uxx1 * uxx1; const double d1 = pow4(IS1 + SMALL_NUM);
     double IS2 = ux2 * ux2 + R13_3 * uxx2 * uxx2; const double d2 = pow4(IS2 + SMALL_NUM);
     ck.divisor(d0); ck.divisor(d1); ck.divisor(d2);
-    double w0 = rcp_near(d0);
-    double w1 = div_rn(central_cell_wt, d1, rcp_near(d1));
-    double w2 = rcp_near(d2);
+    double w0 = rcp_rn(d0);
+    double w1 = div_rn(central_cell_wt, d1, rcp_rn(d1));
+    double w2 = rcp_rn(d2);
     const double total = w0 + w1 + w2;
-    ck.sum(total);
-    const double y = rcp_near(total);
+    const double y = rcp_rn(total);
     w0 = div_rn(w0, total, y);
     w1 = div_rn(w1, total, y);
     w2 = div_rn(w2, total, y);
@@ -899,10 +897,9 @@ struct Recon2Cr {
         double IS2 = temp + uxy2 * uxy2; const double d2 = pow4(IS2 + SMALL_NUM);
         double IS3 = temp + uxy3 * uxy3; const double d3 = pow4(IS3 + SMALL_NUM);
         ck.divisor(d0); ck.divisor(d1); ck.divisor(d2); ck.divisor(d3);
-        double w0 = rcp_near(d0), w1 = rcp_near(d1), w2 = rcp_near(d2), w3 = rcp_near(d3);
+        double w0 = rcp_rn(d0), w1 = rcp_rn(d1), w2 = rcp_rn(d2), w3 = rcp_rn(d3);
         const double total = w0 + w1 + w2 + w3;
-        ck.sum(total);
-        const double y = rcp_near(total);
+        const double y = rcp_rn(total);
         w0 = div_rn(w0, total, y); w1 = div_rn(w1, total, y); w2 = div_rn(w2, total, y); w3 = div_rn(w3, total, y);
         c[5] = w0 * uxy0 + w1 * uxy1 + w2 * uxy2 + w3 * uxy3;
         sp = ck.special();
@@ -952,7 +949,7 @@ struct Recon3 {
     __device__ __forceinline__ static void weights(const Stencil &s, double *coeffs, CrCheck &ck)
     {
         auto over_d = [&](double g, double d) {
-            if constexpr (CR) { ck.divisor(d); return div_rn(g, d, rcp_near(d)); }
+            if constexpr (CR) { ck.divisor(d); return div_rn(g, d, rcp_rn(d)); }
             else return g / d;
         };
         constexpr double gammaHi = 0.85, gammaLo = 0.85;
@@ -1013,8 +1010,7 @@ struct Recon3 {
         }
         double wt_ratio;
         if constexpr (CR) {
-            ck.sum(sum);
-            const double y = rcp_near(sum);
+            const double y = rcp_rn(sum);
             w_R4 = div_rn(w_R4, sum, y);
 #pragma unroll
             for (int i = 0; i < 5; ++i) w_R3[i] = div_rn(w_R3[i], sum, y);
