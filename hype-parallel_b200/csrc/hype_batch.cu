@@ -38,6 +38,7 @@ constexpr int KIND_CONS0 = 13, KIND_VISC0 = 25, KIND_VISC_CONS0 = 28;
 constexpr int KIND_MIXED_BN = 31, KIND_MIXED_EULER = 32;
 bool kind_is_mixed(int id) { return id == KIND_MIXED || id == KIND_MIXED_BN || id == KIND_MIXED_EULER; }
 constexpr int NBUF = 4;                // U, S0, S1, S2
+constexpr size_t FETCH_CHUNK = (size_t)4 << 20;
 constexpr int MAX_SUBSTEPS = 16;       // steps an instance may take per batch step
 
 int kind_of(const hype_config &c)
@@ -128,6 +129,8 @@ struct hype_batch {
     bool hold_dirty = false;
     cudaEvent_t hold_ev = nullptr;    // completion of the last hold upload
     double *dStage = nullptr;         // Vec-layout staging, max_cells * 9 doubles
+    char *hFetch = nullptr;           // pinned, two chunks of FETCH_CHUNK: fetches into pageable arrays (first use)
+    cudaEvent_t fetch_ev[2] = {};
     Kind kinds[NKIND];
     cudaGraphExec_t exec = nullptr;
     bool dirty = true;
@@ -691,6 +694,9 @@ int hype_batch_destroy(hype_batch *b)
     if (b->hHold) cudaFreeHost(b->hHold);
     if (b->hold_ev) cudaEventDestroy(b->hold_ev);
     if (b->dStage) cudaFree(b->dStage);
+    if (b->hFetch) cudaFreeHost(b->hFetch);
+    for (cudaEvent_t e : b->fetch_ev)
+        if (e) cudaEventDestroy(e);
     for (int k = 0; k < NKIND; ++k) {
         if (b->side[k]) cudaStreamDestroy(b->side[k]);
         if (b->join[k]) cudaEventDestroy(b->join[k]);
@@ -959,6 +965,43 @@ int hype_batch_hold(hype_batch *b, int id, int hold)
     return HYPE_OK;
 }
 
+// n bytes of dStage to a pageable array, chunk by chunk through pinned memory, each copied out by the
+// host copy pool while the next one arrives.  The array's pages are often fresh ones, and a copy by
+// one thread then waits for the kernel's page faults: 16 grids of sides 128..512 (84 MB) into new
+// arrays 25.9 -> 15.0 ms.
+static int fetch_pageable(hype_batch *b, char *to, size_t n)
+{
+    if (!b->hFetch) {
+        for (cudaEvent_t &e : b->fetch_ev)
+            if (!e) BCUDA(b, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        void *h = nullptr;
+        if (cudaHostAlloc(&h, 2 * FETCH_CHUNK, cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();   // without pinned memory the copy stays direct
+            BCUDA(b, cudaMemcpyAsync(to, b->dStage, n, cudaMemcpyDeviceToHost, b->stream));
+            BCUDA(b, cudaStreamSynchronize(b->stream));
+            return HYPE_OK;
+        }
+        b->hFetch = (char *)h;
+    }
+    const char *from = reinterpret_cast<const char *>(b->dStage);
+    const size_t chunks = (n + FETCH_CHUNK - 1) / FETCH_CHUNK;
+    auto size_of = [&](size_t k) { return std::min(FETCH_CHUNK, n - k * FETCH_CHUNK); };
+    auto enqueue = [&](size_t k) -> int {
+        BCUDA(b, cudaMemcpyAsync(b->hFetch + (k % 2) * FETCH_CHUNK, from + k * FETCH_CHUNK, size_of(k), cudaMemcpyDeviceToHost, b->stream));
+        BCUDA(b, cudaEventRecord(b->fetch_ev[k % 2], b->stream));
+        return HYPE_OK;
+    };
+    int rc;
+    for (size_t k = 0; k < chunks && k < 2; ++k)
+        if ((rc = enqueue(k))) return rc;
+    for (size_t k = 0; k < chunks; ++k) {
+        BCUDA(b, cudaEventSynchronize(b->fetch_ev[k % 2]));
+        host_copy(to + k * FETCH_CHUNK, b->hFetch + (k % 2) * FETCH_CHUNK, size_of(k));
+        if (k + 2 < chunks && (rc = enqueue(k + 2))) return rc;
+    }
+    return HYPE_OK;
+}
+
 int hype_batch_get_state(hype_batch *b, int id, double *U)
 {
     if (!b || !U || id < 0 || id >= (int)b->inst.size() || !b->inst[id].used) return bfail(b, HYPE_ERR_INVALID, "no instance %d", id);
@@ -967,7 +1010,9 @@ int hype_batch_get_state(hype_batch *b, int id, double *U)
     const hype_config &c = in.cfg;
     if (kind_is_mixed(in.kind)) BCUDA(b, launch_mixed_to_aos(c.system, in.mf[0], in.md[0], b->dStage, c.nx, c.ny, in.pitch, in.plane, b->stream));
     else BCUDA(b, launch_planes_to_aos(in.buf[B_U], b->dStage, c.nx, c.ny, in.nv, in.pitch, in.plane, b->stream));
-    BCUDA(b, cudaMemcpyAsync(U, b->dStage, sizeof(double) * (size_t)c.nx * c.ny * in.nv, cudaMemcpyDeviceToHost, b->stream));
+    const size_t bytes = sizeof(double) * (size_t)c.nx * c.ny * in.nv;
+    if (bytes >= ((size_t)1 << 20) && host_is_pageable(U)) return fetch_pageable(b, reinterpret_cast<char *>(U), bytes);
+    BCUDA(b, cudaMemcpyAsync(U, b->dStage, bytes, cudaMemcpyDeviceToHost, b->stream));
     BCUDA(b, cudaStreamSynchronize(b->stream));
     return HYPE_OK;
 }
