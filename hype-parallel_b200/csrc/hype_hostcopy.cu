@@ -17,6 +17,7 @@
 #include <condition_variable>
 #include <cstring>
 #include <mutex>
+#include <sys/mman.h>
 #include <thread>
 #include <unistd.h>
 
@@ -36,6 +37,7 @@ struct CopyPool {
         const char *src = nullptr;
         size_t dpitch = 0, spitch = 0, width = 0, rows = 0, rows_per_part = 0;
         int parts = 0;
+        bool populate = false;
     };
     std::mutex call_m;   // one copy at a time
     std::mutex m;
@@ -52,12 +54,27 @@ struct CopyPool {
         for (int k = 0; k < WORKERS; ++k) std::thread([this] { work(); }).detach();
     }
 
+    // the whole pages of n bytes at d, which are about to be written, in one call instead of a page
+    // fault each (a hint: kernels before Linux 5.14 refuse it)
+    static void populate_pages(char *d, size_t n)
+    {
+#ifdef MADV_POPULATE_WRITE
+        constexpr size_t PAGE = 4096;
+        char *a = reinterpret_cast<char *>((reinterpret_cast<size_t>(d) + PAGE - 1) & ~(PAGE - 1));
+        char *e = reinterpret_cast<char *>(reinterpret_cast<size_t>(d + n) & ~(PAGE - 1));
+        if (a < e) madvise(a, (size_t)(e - a), MADV_POPULATE_WRITE);
+#else
+        (void)d, (void)n;
+#endif
+    }
+
     void run_parts(const Task &t)
     {
         for (;;) {
             const int i = next.fetch_add(1);
             if (i >= t.parts) return;
             const size_t r0 = (size_t)i * t.rows_per_part, r1 = std::min(t.rows, r0 + t.rows_per_part);
+            if (t.populate) populate_pages(t.dst + r0 * t.width, (r1 - r0) * t.width);
             if (t.dpitch == t.width && t.spitch == t.width)
                 std::memcpy(t.dst + r0 * t.width, t.src + r0 * t.width, (r1 - r0) * t.width);
             else
@@ -88,7 +105,7 @@ struct CopyPool {
         }
     }
 
-    void copy(void *d, size_t dp, const void *s, size_t sp, size_t w, size_t nrows)
+    void copy(void *d, size_t dp, const void *s, size_t sp, size_t w, size_t nrows, bool populate)
     {
         if (!w || !nrows) return;
         std::lock_guard<std::mutex> call(call_m);
@@ -97,6 +114,7 @@ struct CopyPool {
         Task t;
         t.dst = (char *)d; t.src = (const char *)s;
         t.dpitch = dp; t.spitch = sp; t.width = w; t.rows = nrows;
+        t.populate = populate;
         t.rows_per_part = (nrows + want - 1) / want;
         t.parts = (int)((nrows + t.rows_per_part - 1) / t.rows_per_part);
         {
@@ -130,17 +148,20 @@ CopyPool *pool()
 
 void host_copy_2d(void *dst, size_t dpitch, const void *src, size_t spitch, size_t width, size_t rows)
 {
-    pool()->copy(dst, dpitch, src, spitch, width, rows);
+    pool()->copy(dst, dpitch, src, spitch, width, rows, false);
 }
 
-void host_copy(void *dst, const void *src, size_t bytes)
+static void copy_flat(void *dst, const void *src, size_t bytes, bool populate)
 {
     // as rows of 64 KiB (and one row for the rest), so that the parts split it
     constexpr size_t W = 64 << 10;
     const size_t rows = bytes / W, tail = bytes - rows * W;
-    if (rows) pool()->copy(dst, W, src, W, W, rows);
+    if (rows) pool()->copy(dst, W, src, W, W, rows, populate);
     if (tail) std::memcpy((char *)dst + rows * W, (const char *)src + rows * W, tail);
 }
+
+void host_copy(void *dst, const void *src, size_t bytes) { copy_flat(dst, src, bytes, false); }
+void host_copy_fresh(void *dst, const void *src, size_t bytes) { copy_flat(dst, src, bytes, true); }
 
 bool host_is_pageable(const void *p)
 {

@@ -294,6 +294,7 @@ cudaError_t launch_mixsys_batch(int sys, int cells, const MixedParams *inst, con
 // hype_hostcopy.cu: host copies split over a small thread pool (between a caller's
 // pageable arrays and pinned staging), and whether a host pointer is pageable
 void host_copy(void *dst, const void *src, size_t bytes);
+void host_copy_fresh(void *dst, const void *src, size_t bytes);   // dst's pages may be new ones
 void host_copy_2d(void *dst, size_t dpitch, const void *src, size_t spitch, size_t width, size_t rows);
 bool host_is_pageable(const void *p);
 
