@@ -37,8 +37,8 @@
 // Point values come from one pass, the admissibility divisions are left to the few cells
 // that need them, products that are zero take no sums or shuffles, and divisions are
 // branch-free chains that interleave (hype_div.cuh).  Right-hand sides from and to device
-// memory: Kapila N = 2 2048^2 1.48 ms, Euler 1531x897 0.288, BN 1024^2 0.652, Kapila N = 3 500^2
-// 0.167; with a pass per use of the point values, the compiler's divisions and a conversion
+// memory: Kapila N = 2 2048^2 1.46 ms, Euler 1531x897 0.287, BN 1024^2 0.642, Kapila N = 3 500^2
+// 0.166; with a pass per use of the point values, the compiler's divisions and a conversion
 // to planes 2.09, 0.414, 0.945 and 0.278.
 //
 // Two block barriers a row (where the fluxes share the coefficients' memory, also a count
